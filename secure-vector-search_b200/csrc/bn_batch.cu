@@ -616,18 +616,28 @@ __global__ void __launch_bounds__(128) zv_kernel(const uint64_t* __restrict__ z,
     if (threadIdx.x == 0) zv[(uint64_t)t * nq + q] = add_mod(add_mod(sh[0], sh[1]), add_mod(sh[2], sh[3]));
 }
 
-__global__ void ur_decide_kernel(const uint64_t* __restrict__ ur_part, uint32_t kpanels, uint32_t trials, uint32_t nq,
-                                 const uint64_t* __restrict__ zv, uint64_t* __restrict__ ur, int32_t* __restrict__ failed) {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= nq) return;
-    int32_t f = -1;
-    for (uint32_t t = 0; t < trials; ++t) {
+// One CTA per query, a warp per trial: the lanes sum the K panels' shares, and
+// the CTA keeps the first trial whose sides differ.  (A thread per query
+// walked trials x K panels dependent loads: 87 us at 8 queries, 64 panels.)
+__global__ void __launch_bounds__(1024)
+ur_decide_kernel(const uint64_t* __restrict__ ur_part, uint32_t kpanels, uint32_t trials, uint32_t nq,
+                 const uint64_t* __restrict__ zv, uint64_t* __restrict__ ur, int32_t* __restrict__ failed) {
+    const uint32_t q = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ int32_t first;
+    if (threadIdx.x == 0) first = 0x7fffffff;
+    __syncthreads();
+    for (uint32_t t = warp; t < trials; t += blockDim.x >> 5) {
         uint64_t acc = 0;
-        for (uint32_t kp = 0; kp < kpanels; ++kp) acc = add_mod(acc, ur_part[((uint64_t)kp * trials + t) * nq + q]);
-        if (ur) ur[(uint64_t)t * nq + q] = acc;
-        if (f < 0 && acc != zv[(uint64_t)t * nq + q]) f = (int32_t)t;
+        for (uint32_t kp = lane; kp < kpanels; kp += 32) acc = add_mod(acc, ur_part[((uint64_t)kp * trials + t) * nq + q]);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) acc = add_mod(acc, __shfl_xor_sync(0xffffffffu, acc, off));
+        if (lane == 0) {
+            if (ur) ur[(uint64_t)t * nq + q] = acc;
+            if (acc != zv[(uint64_t)t * nq + q]) atomicMin(&first, (int32_t)t);
+        }
     }
-    failed[q] = f;
+    __syncthreads();
+    if (threadIdx.x == 0) failed[q] = first == 0x7fffffff ? -1 : first;
 }
 
 unsigned grid_for(uint64_t work, unsigned threads, unsigned cap) {
@@ -718,7 +728,8 @@ void launch_zv(const uint64_t* d_z, const uint64_t* d_v, uint32_t trials, uint32
 void launch_ur_decide(const uint64_t* d_ur_part, uint32_t kpanels, uint32_t trials, uint32_t nq, const uint64_t* d_zv,
                       uint64_t* d_ur, int32_t* d_failed, cudaStream_t s) {
     if (!nq) return;
-    ur_decide_kernel<<<(nq + 127) / 128, 128, 0, s>>>(d_ur_part, kpanels, trials, nq, d_zv, d_ur, d_failed);
+    const uint32_t warps = trials < 1 ? 1 : trials < 32 ? trials : 32;
+    ur_decide_kernel<<<nq, 32 * warps, 0, s>>>(d_ur_part, kpanels, trials, nq, d_zv, d_ur, d_failed);
 }
 
 }  // namespace bn

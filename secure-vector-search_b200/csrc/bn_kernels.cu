@@ -821,19 +821,35 @@ __device__ __forceinline__ void warp_topk_offer(int64_t& ls, uint32_t& li, int k
     }
 }
 
-// Merges n (score, id) entries of shared memory into every warp's list
-// (entry e goes to warp e / 32 % warps), then the warps' lists into warp 0
-// through `xs`, `xi` (32 * warps entries).  Returns in warp 0's lanes.
+// Merges another sorted list (os, oi; same form) into this one: the better of
+// entry i and the other's entry 31 - i are the best 32 of both as a bitonic
+// sequence, which five exchanges sort; lanes >= k are emptied again.
+__device__ __forceinline__ void warp_topk_merge(int64_t& ls, uint32_t& li, int k, int64_t os, uint32_t oi, uint32_t lane) {
+    const int64_t rs = __shfl_sync(FULL, os, 31 - lane);
+    const uint32_t ri = __shfl_sync(FULL, oi, 31 - lane);
+    if (better(rs, ri, ls, li)) { ls = rs; li = ri; }
+#pragma unroll
+    for (int stride = 16; stride > 0; stride >>= 1) {
+        const int64_t ps = __shfl_xor_sync(FULL, ls, stride);
+        const uint32_t pi = __shfl_xor_sync(FULL, li, stride);
+        if (better(ps, pi, ls, li) == ((lane & stride) == 0)) { ls = ps; li = pi; }
+    }
+    if ((int)lane >= k) { ls = INT64_MIN; li = 0xffffffffu; }
+}
+
+// Merges the warps' lists into warp 0 by halves through `xs`, `xi` (32 *
+// warps entries).  Returns in warp 0's lanes.
 __device__ __forceinline__ void warp_topk_reduce(int64_t& ls, uint32_t& li, int k, int64_t* xs, uint32_t* xi,
                                                  uint32_t warp, uint32_t lane) {
-    xs[warp * 32 + lane] = ls;
-    xi[warp * 32 + lane] = li;
-    __syncthreads();
-    if (warp == 0) {
-        for (uint32_t w = 1; w < DT_THREADS / 32; ++w) {
-            const int64_t s = xs[w * 32 + lane];
-            const uint32_t id = xi[w * 32 + lane];
-            warp_topk_offer(ls, li, k, s != INT64_MIN, s, id, lane);
+    for (uint32_t half = DT_THREADS / 64; half > 0; half >>= 1) {
+        if (warp >= half && warp < 2 * half) {
+            xs[warp * 32 + lane] = ls;
+            xi[warp * 32 + lane] = li;
+        }
+        __syncthreads();
+        if (warp < half) {
+            const uint32_t o = (warp + half) * 32 + lane;
+            warp_topk_merge(ls, li, k, xs[o], xi[o], lane);
         }
     }
     __syncthreads();
@@ -1101,6 +1117,41 @@ topk_merge_kernel(const int64_t* __restrict__ cand_s, const uint32_t* __restrict
     if (threadIdx.x == 0) out_n[q] = (uint32_t)keep;
 }
 
+// The same for k <= 32 with the warps' own lists.
+__global__ void __launch_bounds__(DT_THREADS)
+topk_merge_warp_kernel(const int64_t* __restrict__ cand_s, const uint32_t* __restrict__ cand_i,
+                       const uint32_t* __restrict__ cand_n, uint32_t ctas, uint32_t k, uint32_t* __restrict__ out_ids,
+                       int64_t* __restrict__ out_scores, uint32_t* __restrict__ out_n) {
+    const uint32_t q = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ int64_t xs[DT_THREADS];
+    __shared__ uint32_t xi[DT_THREADS];
+    int64_t ls = INT64_MIN;
+    uint32_t li = 0xffffffffu;
+    const uint32_t total = ctas * k;
+    for (uint32_t t0 = warp * 32; t0 < total; t0 += DT_THREADS) {
+        const uint32_t e = t0 + lane;
+        bool v = false;
+        int64_t sc = 0;
+        uint32_t id = 0;
+        if (e < total) {
+            const uint64_t slot = (uint64_t)q * ctas + e / k;
+            sc = cand_s[slot * k + e % k];  // entries past the list's count are loaded and ignored
+            id = cand_i[slot * k + e % k];
+            v = e % k < cand_n[slot];
+        }
+        warp_topk_offer(ls, li, (int)k, v, sc, id, lane);
+    }
+    warp_topk_reduce(ls, li, (int)k, xs, xi, warp, lane);
+    if (warp == 0) {
+        const uint32_t keep = __popc(__ballot_sync(FULL, lane < k && ls != INT64_MIN));
+        if (lane < keep) {
+            out_ids[(uint64_t)q * k + lane] = li;
+            out_scores[(uint64_t)q * k + lane] = ls;
+        }
+        if (lane == 0) out_n[q] = keep;
+    }
+}
+
 // Top-k of residues combined on the fly: query q's row i scores
 // to_signed(a + b - c) (b, c nullable) with a = ra[q * ld + i] etc., ids[i]
 // (or i); mv_out (nullable) receives the combined residues at the same
@@ -1169,6 +1220,85 @@ topk_rows_kernel(const uint64_t* __restrict__ ra, const uint64_t* __restrict__ r
         cand_i[slot * k + i] = buf.id[i];
     }
     if (threadIdx.x == 0) cand_n[slot] = (uint32_t)keep;
+}
+
+// topk_rows_kernel for k <= 32: every warp keeps its own list, so the loop
+// holds no block barrier, and a thread has TR_UNROLL pairs of rows of all
+// three arrays in flight (the candidate buffer's two barriers per 512 rows
+// held the pass at 0.4 TB/s with 8 queries).
+constexpr uint32_t TR_UNROLL = 4;
+
+__global__ void __launch_bounds__(DT_THREADS)
+topk_rows_warp_kernel(const uint64_t* __restrict__ ra, const uint64_t* __restrict__ rb, const uint64_t* __restrict__ rc,
+                      uint64_t ld, uint64_t rows, const uint64_t* __restrict__ qoff, const uint32_t* __restrict__ ids,
+                      uint32_t k, int64_t* __restrict__ cand_s, uint32_t* __restrict__ cand_i,
+                      uint32_t* __restrict__ cand_n, uint64_t* __restrict__ mv_out) {
+    const uint32_t q = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ int64_t xs[DT_THREADS];
+    __shared__ uint32_t xi[DT_THREADS];
+    int64_t ls = INT64_MIN;
+    uint32_t li = 0xffffffffu;
+    const uint64_t base = qoff ? 0 : (uint64_t)q * ld;  // the same row ranges as topk_rows_kernel
+    const uint64_t first = qoff ? qoff[q] : 0, hi = qoff ? qoff[q + 1] : rows;
+    const uint64_t lo = first & ~1ull, span = hi > lo ? hi - lo : 0;
+    const uint64_t per = ((span + gridDim.x - 1) / gridDim.x + 1) & ~1ull;
+    const uint64_t v_begin = lo + min(span, (uint64_t)blockIdx.x * per);
+    const uint64_t v_end = min(hi, v_begin + per);
+    for (uint64_t tile = v_begin; tile < v_end; tile += 2 * DT_THREADS * TR_UNROLL) {
+        ulonglong2 x[TR_UNROLL], y[TR_UNROLL], z[TR_UNROLL];
+#pragma unroll
+        for (uint32_t u = 0; u < TR_UNROLL; ++u) {
+            const uint64_t i0 = tile + 2 * (u * DT_THREADS + threadIdx.x);
+            x[u] = y[u] = z[u] = make_ulonglong2(0, 0);
+            if (i0 < v_end) {  // 16-byte aligned and inside the row of ld, as in topk_rows_kernel
+                x[u] = *reinterpret_cast<const ulonglong2*>(ra + base + i0);
+                if (rb) y[u] = *reinterpret_cast<const ulonglong2*>(rb + base + i0);
+                if (rc) z[u] = *reinterpret_cast<const ulonglong2*>(rc + base + i0);
+            }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < TR_UNROLL; ++u) {
+            const uint64_t i0 = tile + 2 * (u * DT_THREADS + threadIdx.x);
+            const bool valid[2] = {i0 < v_end && i0 >= first, i0 + 1 < v_end};
+            const uint64_t mv[2] = {sub_mod(add_mod(x[u].x, y[u].x), z[u].x), sub_mod(add_mod(x[u].y, y[u].y), z[u].y)};
+            const int64_t ts = __shfl_sync(FULL, ls, k - 1);  // scores below the k-th best need no id
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (mv_out && valid[h]) mv_out[base + i0 + h] = mv[h];
+                const int64_t sc = to_signed(mv[h]);
+                const bool v = valid[h] && sc >= ts;
+                const uint32_t id = v ? (ids ? ids[i0 + h] : (uint32_t)(i0 + h)) : 0;
+                if (__any_sync(FULL, v)) warp_topk_offer(ls, li, (int)k, v, sc, id, lane);
+            }
+        }
+    }
+    warp_topk_reduce(ls, li, (int)k, xs, xi, warp, lane);
+    if (warp == 0) {
+        const uint64_t slot = (uint64_t)q * gridDim.x + blockIdx.x;
+        const uint32_t keep = __popc(__ballot_sync(FULL, lane < k && ls != INT64_MIN));
+        if (lane < keep) {
+            cand_s[slot * k + lane] = ls;
+            cand_i[slot * k + lane] = li;
+        }
+        if (lane == 0) cand_n[slot] = keep;
+    }
+}
+
+// k <= 32, what a warp's lanes hold: the warp-list kernels; larger k: the CTA
+// candidate buffers.
+void launch_topk(const uint64_t* d_a, const uint64_t* d_b, const uint64_t* d_c, uint64_t ld, uint64_t rows,
+                 const uint64_t* d_qoff, uint32_t nq, const uint32_t* d_ids, uint32_t k, int ctas_per_query,
+                 const TopkScratch& scratch, uint32_t* d_out_ids, int64_t* d_out_scores, uint32_t* d_out_n,
+                 uint64_t* d_mv_out, cudaStream_t s) {
+    if (!nq) return;
+    const bool warp_lists = k >= 1 && k <= (uint32_t)WARP_TOPK_MAX;
+    const dim3 grid(ctas_per_query, nq);
+    auto rows_fn = warp_lists ? topk_rows_warp_kernel : topk_rows_kernel;
+    auto merge_fn = warp_lists ? topk_merge_warp_kernel : topk_merge_kernel;
+    rows_fn<<<grid, DT_THREADS, 0, s>>>(d_a, d_b, d_c, ld, rows, d_qoff, d_ids, k, scratch.cand_s, scratch.cand_i,
+                                        scratch.cand_n, d_mv_out);
+    merge_fn<<<nq, DT_THREADS, 0, s>>>(scratch.cand_s, scratch.cand_i, scratch.cand_n, (uint32_t)ctas_per_query, k,
+                                       d_out_ids, d_out_scores, d_out_n);
 }
 
 // ------------------------------------------------------------------ keygen GEMM
@@ -1407,23 +1537,15 @@ void launch_topk_rows(const uint64_t* d_a, const uint64_t* d_b, const uint64_t* 
                       uint32_t nq, const uint32_t* d_ids, uint32_t k, int ctas_per_query, TopkScratch scratch,
                       uint32_t* d_out_ids, int64_t* d_out_scores, uint32_t* d_out_n, uint64_t* d_mv_out,
                       cudaStream_t s) {
-    if (!nq) return;
-    topk_rows_kernel<<<dim3(ctas_per_query, nq), DT_THREADS, 0, s>>>(d_a, d_b, d_c, ld, rows, nullptr, d_ids, k,
-                                                                   scratch.cand_s, scratch.cand_i, scratch.cand_n,
-                                                                   d_mv_out);
-    topk_merge_kernel<<<nq, DT_THREADS, 0, s>>>(scratch.cand_s, scratch.cand_i, scratch.cand_n, ctas_per_query, k,
-                                                d_out_ids, d_out_scores, d_out_n);
+    launch_topk(d_a, d_b, d_c, ld, rows, nullptr, nq, d_ids, k, ctas_per_query, scratch, d_out_ids, d_out_scores, d_out_n,
+                d_mv_out, s);
 }
 
 void launch_topk_segs(const uint64_t* d_a, const uint64_t* d_b, const uint64_t* d_c, const uint64_t* d_qoff,
                       uint32_t nq, const uint32_t* d_ids, uint32_t k, int ctas_per_query, TopkScratch scratch,
                       uint32_t* d_out_ids, int64_t* d_out_scores, uint32_t* d_out_n, cudaStream_t s) {
-    if (!nq) return;
-    topk_rows_kernel<<<dim3(ctas_per_query, nq), DT_THREADS, 0, s>>>(d_a, d_b, d_c, 0, 0, d_qoff, d_ids, k,
-                                                                   scratch.cand_s, scratch.cand_i, scratch.cand_n,
-                                                                   nullptr);
-    topk_merge_kernel<<<nq, DT_THREADS, 0, s>>>(scratch.cand_s, scratch.cand_i, scratch.cand_n, ctas_per_query, k,
-                                                d_out_ids, d_out_scores, d_out_n);
+    launch_topk(d_a, d_b, d_c, 0, 0, d_qoff, nq, d_ids, k, ctas_per_query, scratch, d_out_ids, d_out_scores, d_out_n,
+                nullptr, s);
 }
 
 void launch_gemm_abt(const uint64_t* d_A, const uint64_t* d_B, const uint64_t* d_D, uint64_t rows, uint32_t cols,
