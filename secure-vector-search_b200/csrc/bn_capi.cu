@@ -462,6 +462,10 @@ RunLayout make_layout(const Sizes& z, bool want_mv) {
     o.err = L.take<uint32_t>(1);
     o.flags = L.take<uint32_t>(1);  // DRAW_HIT_P when a Protocol 2 draw equalled p
     o.out_end = L.off;
+    // cleared with err and flags in one go (o.err .. o.zero_end)
+    o.cand_done = L.take<uint32_t>(z.B);
+    o.fin_done = L.take<uint32_t>(z.nvseg);
+    o.zero_end = L.off;
     o.limbs = L.take<QLimb>((uint64_t)z.B * N);
     o.x = L.take<uint64_t>((uint64_t)z.B * z.n1);
     o.r = L.take<uint64_t>(std::max<uint64_t>(z.total_out, 1));
@@ -475,7 +479,6 @@ RunLayout make_layout(const Sizes& z, bool want_mv) {
     o.cand_s = L.take<int64_t>(cand);
     o.cand_i = L.take<uint32_t>(cand);
     o.cand_n = L.take<uint32_t>(z.ctas);
-    o.cand_done = L.take<uint32_t>(z.B);
     o.u_buf = (tc && z.trials) ? L.take<uint8_t>(std::max<uint64_t>(z.nblocks, 1) * pass_rows(TC_MAX_TRIALS) * TC_ROWS) : 0;
     o.r_part = (tc && z.trials)
                    ? L.take<uint64_t>((uint64_t)tc_groups(pass_rows(std::min<uint32_t>(TC_MAX_TRIALS, z.trials))) *
@@ -506,12 +509,13 @@ int make_tc_maps(const Sizes& z, const uint8_t* d_u, const uint8_t* d_w, TcMaps&
 // Protocol 2 on the tensor engine, else the scan).
 int enqueue_pipeline(bn_ctx* ctx, const Corpus& c, const Sizes& z, const Meta& m, const Inputs& in, const Scratch& sc,
                      const Outputs& out, cudaStream_t s, cudaEvent_t prof0, cudaEvent_t prof1) {
-    CU(cudaMemsetAsync(sc.err, 0, 4, s));
-    CU(cudaMemsetAsync(sc.flags, 0, 4, s));
+    const bool tensor = z.trials && z.engine == BN_ENGINE_TENSOR;
+    launch_query_prep(c.L.at<uint64_t>(), c.n1, in.v, z.B, z.k ? sc.x : nullptr, tensor ? sc.wimg : nullptr, sc.err,
+                      sc.zero_words, s);
     if (z.trials && ctx->debug_draw_hit) launch_or_flag(sc.flags, DRAW_HIT_P, s);
-    launch_query_limbs(in.v, z.B, sc.limbs, s);
+    if (!tensor) launch_query_limbs(in.v, z.B, sc.limbs, s);
     const ChaChaKey* keys = reinterpret_cast<const ChaChaKey*>(in.seeds);
-    if (z.trials && z.engine == BN_ENGINE_TENSOR) {
+    if (tensor) {
         // One pass over m_enc yields r and the first <= 20 trials' z (tensor
         // cores); later passes of 20 trials reuse the now-known r.
         for (uint32_t t0 = 0, ps = 0; t0 < z.trials; t0 += TC_MAX_TRIALS, ++ps) {
@@ -519,7 +523,6 @@ int enqueue_pipeline(bn_ctx* ctx, const Corpus& c, const Sizes& z, const Meta& m
             if (ps == 0) {
                 launch_tc_ugen(m.vsegs, m.tc_blocks, m.nblocks, keys, nullptr, t0, tc, nr, sc.u_buf, sc.ur_part,
                                z.trials, sc.flags, s);
-                launch_query_wimg(in.v, z.B, sc.wimg, s);
                 if (prof0) CU(cudaEventRecord(prof0, s));
                 launch_tc_fused(c.tmap_m, m.maps->u[ps], m.maps->w, m.tc_panels, m.npanels, m.vsegs, tc, nr,
                                 z.trials, sc.z_part, sc.r_part, z.total_out, sc.err, ctx->num_sms, s,
@@ -535,7 +538,7 @@ int enqueue_pipeline(bn_ctx* ctx, const Corpus& c, const Sizes& z, const Meta& m
             }
         }
         launch_tc_finish(sc.z_part, sc.ur_part, m.seg_panel0, m.seg_block0, in.v, m.vsegs, m.nvseg, z.trials, sc.ur,
-                         sc.zv, sc.zv_chunks, out.vfailed, s);
+                         sc.zv, sc.zv_chunks, sc.fin_done, out.vfailed, s);
     } else {
         if (prof0) CU(cudaEventRecord(prof0, s));
         launch_scan(c.m_enc.at<uint64_t>(), sc.limbs, m.segs, m.seg_blk, m.nseg, m.total_blocks, sc.r, ctx->num_sms,
@@ -551,7 +554,6 @@ int enqueue_pipeline(bn_ctx* ctx, const Corpus& c, const Sizes& z, const Meta& m
         }
     }
     if (z.k) {
-        launch_lt_times_v(c.L.at<uint64_t>(), c.n1, in.v, z.B, sc.x, s);
         launch_decode_topk(sc.r, decode_corpus(c), m.segs, m.seg_unit, m.dq, z.B, in.v, in.g, sc.x, in.t, in.t_nnz, z.k,
                            z.ctas, sc.topk, out.mv, out.ids, out.scores, out.n, s);
     } else {
@@ -578,7 +580,8 @@ Scratch scratch_at(char* d, const RunLayout& o) {
                                reinterpret_cast<uint32_t*>(d + o.cand_n), reinterpret_cast<uint32_t*>(d + o.cand_done)},
                    reinterpret_cast<uint32_t*>(d + o.err), reinterpret_cast<uint8_t*>(d + o.u_buf),
                    reinterpret_cast<uint64_t*>(d + o.r_part), reinterpret_cast<uint64_t*>(d + o.zv_chunks),
-                   reinterpret_cast<uint8_t*>(d + o.wimg)};
+                   reinterpret_cast<uint8_t*>(d + o.wimg), reinterpret_cast<uint32_t*>(d + o.fin_done),
+                   (uint32_t)((o.zero_end - o.err) / 4)};
 }
 void pack_meta(char* h, const RunLayout& o, const HostMeta& hm) {
     memcpy(h + o.segs, hm.segs.data(), hm.segs.size() * sizeof(ScanSeg));
@@ -796,8 +799,7 @@ int run_verify(Engine& e, uint64_t row0, uint64_t rows, const uint64_t* r, const
     const ChaChaKey* keys = reinterpret_cast<const ChaChaKey*>(d + o.seeds);
     const uint64_t* dv = reinterpret_cast<uint64_t*>(d + o.v);
     int32_t* dfail = reinterpret_cast<int32_t*>(d + o.vfailed);
-    CU(cudaMemsetAsync(sc.flags, 0, 4, e.stream));
-    CU(cudaMemsetAsync(sc.err, 0, 4, e.stream));
+    CU(cudaMemsetAsync(sc.err, 0, sc.zero_words * 4ull, e.stream));  // status words and tickets
     if (e.ctx->debug_draw_hit) launch_or_flag(sc.flags, DRAW_HIT_P, e.stream);
     if (z.engine == BN_ENGINE_TENSOR) {
         for (uint32_t t0 = 0, ps = 0; t0 < trials; t0 += TC_MAX_TRIALS, ++ps) {
@@ -808,7 +810,7 @@ int run_verify(Engine& e, uint64_t row0, uint64_t rows, const uint64_t* r, const
                                 e.ctx->num_sms, e.stream, 0, e.ctx->debug_wait_cycles);
         }
         launch_tc_finish(sc.z_part, sc.ur_part, m.seg_panel0, m.seg_block0, dv, m.vsegs, 1, trials, sc.ur, sc.zv,
-                         sc.zv_chunks, dfail, e.stream);
+                         sc.zv_chunks, sc.fin_done, dfail, e.stream);
     } else {
         launch_freivalds(e.c.m_enc.at<uint64_t>(), sc.r, m.vsegs, 1, keys, trials, z.fp, sc.z_part, sc.ur_part, sc.flags,
                          e.stream);

@@ -252,6 +252,8 @@ struct Scratch {  // device pointers
     uint64_t* r_part;  // fused pass: per strip-group partial dots
     uint64_t* zv_chunks;
     uint8_t* wimg;     // fused pass: diagonal byte images of the queries
+    uint32_t* fin_done;   // tickets of the verdict kernel, one per verify segment
+    uint32_t zero_words;  // u32 from err on that a run clears first
 };
 struct Inputs {
     const uint64_t* v;
@@ -297,8 +299,8 @@ struct RunLayout {
     // outputs (contiguous -> one D2H)
     uint64_t ids, scores, n, vfailed, ur, zv, err, out_begin, out_end;
     // internal
-    uint64_t limbs, x, r, mv, z_part, ur_part, flags, cand_s, cand_i, cand_n, cand_done, u_buf, r_part, zv_chunks, wimg,
-        total;
+    uint64_t limbs, x, r, mv, z_part, ur_part, flags, cand_s, cand_i, cand_n, cand_done, fin_done, zero_end, u_buf,
+        r_part, zv_chunks, wimg, total;
 };
 
 // One run of the query pipeline over host inputs (bn_capi.cu): hm is the

@@ -16,12 +16,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <cooperative_groups.h>
 #include <type_traits>
 
 #include "bn_kernels.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace bn {
 
@@ -401,63 +398,107 @@ freivalds_finish_kernel(const uint64_t* __restrict__ z_part, const uint64_t* __r
 }
 
 // ------------------------------------------------------------------ L^T v
-// A cluster of 8 CTAs of 1024 threads per query (one CTA per query kept a
-// single SM busy for ~34 us): column k = tid % n1, rows j of the CTA's
-// range, slice, slice + slices, ... with v_j's limbs in shared memory, so
-// each term is six multiply-adds into three accumulators and the column
-// loads are independent (batches of 8 in flight).  Each thread sums at most
-// 64 terms below 2^53.2 (hi < 2^29), so the accumulators stay below 2^64.
-constexpr uint32_t LT_SPLIT = 8;  // CTAs per query (one cluster), N / LT_SPLIT terms each
+// A CTA takes 8 columns of L (64 of its bytes per row, whole sectors) for a
+// run of queries: thread (slice, column) holds its 32 elements of L, rows
+// slice, slice + 32, ..., in registers, all loads in flight at once, and every
+// query costs the limbs of its v in shared memory and six multiply-adds per
+// element.  Latency bound for one query (16 CTAs at n1 = 128, one round of
+// loads: 13 -> 4 us against a cluster of 8 CTAs with a distributed-shared-
+// memory sum); for many, L is read once per run of queries instead of once per
+// query (512 queries: 168 us before).  A thread adds 32 terms below 2^53.2, so
+// the accumulators stay below 2^64.
+constexpr uint32_t LT_THREADS = 256, LT_COLS = 8, LT_ROWS = N / (LT_THREADS / LT_COLS);
 
-__global__ void __cluster_dims__(1, LT_SPLIT, 1) __launch_bounds__(1024)
-lt_times_v_kernel(const uint64_t* __restrict__ L, uint32_t n1, const uint64_t* __restrict__ v, uint64_t* __restrict__ x) {
-    // CTA (q, s) of the query's cluster sums the terms j in [s N/8, (s+1) N/8)
-    // for every output k; CTA 0 adds the 8 partial rows through distributed
-    // shared memory.  A thread takes one k and every slices-th term of the range.
-    constexpr uint32_t TERMS = N / LT_SPLIT;
-    const uint32_t q = blockIdx.x, s = blockIdx.y;
-    const uint32_t k = threadIdx.x % n1, slices = blockDim.x / n1, sl = threadIdx.x / n1;
-    __shared__ uint4 vl[2 * TERMS];
-    __shared__ uint64_t part[1024];
-    __shared__ uint64_t row[512];  // this CTA's partial x (n1 <= 512)
-    for (uint32_t jj = threadIdx.x; jj < TERMS; jj += blockDim.x) {
-        const uint64_t w = v[(uint64_t)q * N + s * TERMS + jj];
-        const Limbs3 b = limbs(w), c = limbs_hi(w);
-        vl[2 * jj] = make_uint4(b.b0, b.b1, b.b2, c.b0);
-        vl[2 * jj + 1] = make_uint4(c.b1, c.b2, 0u, 0u);
-    }
-    __syncthreads();
-    uint64_t a0 = 0, a1 = 0, a2 = 0;
-    const uint32_t terms = TERMS / slices;  // n1 / 8: a multiple of 8 for n1 >= 64
-    for (uint32_t i0 = 0; i0 < terms; i0 += 8) {
-        uint64_t xs[8];
+struct LtShared {
+    uint4 lo[N];  // {b0, b1, b2, c0} of v_j
+    uint2 hi[N];  // {c1, c2}
+    uint64_t red[LT_THREADS / 32][LT_COLS];
+};
+
+__device__ __forceinline__ void lt_block(LtShared& sh, const uint64_t* __restrict__ L, uint32_t n1,
+                                         const uint64_t* __restrict__ v, uint32_t k0, uint32_t q0, uint32_t q1,
+                                         uint64_t* __restrict__ x) {
+    const uint32_t kk = threadIdx.x % LT_COLS, sl = threadIdx.x / LT_COLS;
+    constexpr uint32_t SLICES = LT_THREADS / LT_COLS;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint64_t l[LT_ROWS];
 #pragma unroll
-        for (int ii = 0; ii < 8; ++ii) xs[ii] = __ldg(L + (uint64_t)(s * TERMS + sl + (i0 + ii) * slices) * n1 + k);
+    for (uint32_t i = 0; i < LT_ROWS; ++i) l[i] = __ldg(L + (uint64_t)(sl + i * SLICES) * n1 + k0 + kk);
+    for (uint32_t q = q0; q < q1; ++q) {
+        for (uint32_t j = threadIdx.x; j < N; j += LT_THREADS) {
+            const uint64_t w = v[(uint64_t)q * N + j];
+            const Limbs3 b = limbs(w), c = limbs_hi(w);
+            sh.lo[j] = make_uint4(b.b0, b.b1, b.b2, c.b0);
+            sh.hi[j] = make_uint2(c.b1, c.b2);
+        }
+        __syncthreads();
+        uint64_t a0 = 0, a1 = 0, a2 = 0;
 #pragma unroll
-        for (int ii = 0; ii < 8; ++ii) {
-            const uint32_t jj = sl + (i0 + ii) * slices;
-            const uint4 l0 = vl[2 * jj], l1 = vl[2 * jj + 1];
-            const uint32_t xl = (uint32_t)xs[ii], xh = (uint32_t)(xs[ii] >> 32);
+        for (uint32_t i = 0; i < LT_ROWS; ++i) {
+            const uint4 l0 = sh.lo[sl + i * SLICES];
+            const uint2 l1 = sh.hi[sl + i * SLICES];
+            const uint32_t xl = (uint32_t)l[i], xh = (uint32_t)(l[i] >> 32);
             a0 = mac(mac(a0, xl, l0.x), xh, l0.w);
             a1 = mac(mac(a1, xl, l0.y), xh, l1.x);
             a2 = mac(mac(a2, xl, l0.z), xh, l1.y);
         }
+        uint64_t t = combine3(a0, a1, a2);
+        t = add_mod(t, __shfl_xor_sync(FULL, t, 8));
+        t = add_mod(t, __shfl_xor_sync(FULL, t, 16));
+        if (lane < LT_COLS) sh.red[warp][lane] = t;
+        __syncthreads();  // also: the limbs are no longer read
+        if (threadIdx.x < LT_COLS) {
+            uint64_t s = 0;
+#pragma unroll
+            for (uint32_t w = 0; w < LT_THREADS / 32; ++w) s = add_mod(s, sh.red[w][threadIdx.x]);
+            x[(uint64_t)q * n1 + k0 + threadIdx.x] = s;
+        }
     }
-    part[threadIdx.x] = combine3(a0, a1, a2);
-    __syncthreads();
-    if (threadIdx.x < n1) {
-        uint64_t t = 0;
-        for (uint32_t i = 0; i < slices; ++i) t = add_mod(t, part[i * n1 + threadIdx.x]);
-        row[threadIdx.x] = t;
+}
+
+// Queries per CTA: as many as leave two CTAs per SM, at most 16.
+uint32_t lt_run(uint32_t n1, uint32_t nq) {
+    const uint32_t run = (uint32_t)((uint64_t)nq * (n1 / LT_COLS) / (2 * 148));
+    return run < 1 ? 1 : run > 16 ? 16 : run;
+}
+
+__global__ void __launch_bounds__(LT_THREADS)
+lt_times_v_kernel(const uint64_t* __restrict__ L, uint32_t n1, const uint64_t* __restrict__ v, uint32_t nq,
+                  uint32_t run, uint64_t* __restrict__ x) {
+    __shared__ LtShared sh;
+    const uint32_t q0 = blockIdx.y * run;
+    lt_block(sh, L, n1, v, blockIdx.x * LT_COLS, q0, min(nq, q0 + run), x);
+}
+
+// Everything a query pipeline needs from v before its first pass, in one
+// launch: CTAs [0, lt_ctas) take L^T v (lt_cols column groups per run of
+// queries), the next wimg_ctas the diagonal byte images of the fused scan,
+//   w[((q * 64 + strip) * 16 + s) * 128 + 8 j + a] = byte (s - a) of
+//   v[q][strip * 16 + j] when 0 <= s - a <= 7, else 0,
+// and the last one clears the run's status words and tickets.
+__global__ void __launch_bounds__(LT_THREADS)
+query_prep_kernel(const uint64_t* __restrict__ L, uint32_t n1, const uint64_t* __restrict__ v, uint32_t nq,
+                  uint32_t run, uint32_t lt_ctas, uint64_t* __restrict__ x, uint32_t wimg_ctas, uint8_t* __restrict__ w,
+                  uint32_t* __restrict__ zero, uint32_t zero_words) {
+    __shared__ LtShared sh;
+    if (blockIdx.x < lt_ctas) {
+        const uint32_t cols = n1 / LT_COLS, q0 = blockIdx.x / cols * run;
+        lt_block(sh, L, n1, v, blockIdx.x % cols * LT_COLS, q0, min(nq, q0 + run), x);
+    } else if (blockIdx.x < lt_ctas + wimg_ctas) {
+        const uint64_t e = (uint64_t)(blockIdx.x - lt_ctas) * LT_THREADS + threadIdx.x;  // (query, strip, s, j)
+        const uint32_t j = (uint32_t)(e & 15), s = (uint32_t)((e >> 4) & 15);
+        const uint64_t qs = e >> 8;  // q * 64 + strip
+        const uint64_t y = v[(qs >> 6) * N + (qs & 63) * 16 + j];
+        uint64_t word = 0;
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+            const int b = (int)s - a;
+            if (b >= 0 && b <= 7) word |= ((y >> (8 * b)) & 0xffull) << (8 * a);
+        }
+        *reinterpret_cast<uint64_t*>(w + (qs * 16 + s) * 128 + 8 * j) = word;
+    } else {
+        for (uint32_t i = threadIdx.x; i < zero_words; i += LT_THREADS) zero[i] = 0;
     }
-    cg::cluster_group cluster = cg::this_cluster();
-    cluster.sync();  // every CTA's row is written
-    if (s == 0 && threadIdx.x < n1) {
-        uint64_t t = 0;
-        for (uint32_t r = 0; r < LT_SPLIT; ++r) t = add_mod(t, cluster.map_shared_rank(row, r)[threadIdx.x]);
-        x[(uint64_t)q * n1 + threadIdx.x] = t;
-    }
-    cluster.sync();  // no CTA leaves while CTA 0 still reads its row
 }
 
 // ------------------------------------------------------------------ decode
@@ -596,17 +637,17 @@ __device__ __forceinline__ void topk_offer(TopkBuf& b, bool valid, int64_t s, ui
 // folded lazily: every term is < 2^61, three terms fit below 2^63.
 __device__ __forceinline__ uint64_t signed_term(uint64_t x, bool neg) { return neg ? P - x : x; }
 
-// AL_i . g + H_i . x for corpus row gr from the 32-row-blocked alh_b: the
+// The columns [k_begin, k_end) of AL_i . g + H_i . x for corpus row gr from the 32-row-blocked alh_b: the
 // 2 n1 columns of the row's block are contiguous, so a warp's batch of 32
 // column loads is one 8 KB run.  lim[2k], lim[2k+1] hold the limbs of g_k
 // (k < n1) and of x_(k-n1) (k >= n1).  Every column adds lo*b + hi*c <
 // 2^53 + 2^50 (hi < 2^29: residues are < 2^61) to an accumulator, so the
 // 2 n1 <= 1024 columns stay below 2^64 with no fold.
 __device__ __forceinline__ uint64_t dense_terms_row(const uint64_t* __restrict__ alh_b, uint32_t n1, uint64_t gr,
-                                                    const uint4* __restrict__ lim) {
+                                                    const uint4* __restrict__ lim, uint32_t k_begin, uint32_t k_end) {
     const uint64_t* p = alh_b + (gr >> 5) * (2ull * n1) * 32 + (gr & 31);
     uint64_t a0 = 0, a1 = 0, a2 = 0;
-    for (uint32_t k0 = 0; k0 < 2 * n1; k0 += 32) {  // 2 n1 is a multiple of 32 (n1 >= 64)
+    for (uint32_t k0 = k_begin; k0 < k_end; k0 += 32) {  // ranges are multiples of 32 columns
         uint64_t xs[32];
 #pragma unroll
         for (int kk = 0; kk < 32; ++kk) xs[kk] = __ldg(p + (uint64_t)(k0 + kk) * 32);
@@ -707,25 +748,20 @@ __device__ __forceinline__ int32_t m_times_t_warp(const int8_t* __restrict__ m8_
     return acc - bias;
 }
 
-// M_i . T from the column-major residues (plaintext not int8-valued): one
-// row per lane, gathers lazily folded.
+// The T entries [c, c_end) of M_i . T from the column-major residues
+// (plaintext not int8-valued): one row per lane, gathers lazily folded.
 __device__ __forceinline__ uint64_t m_times_t_cm(const uint64_t* __restrict__ mp_cm, uint64_t rows, uint64_t gr,
-                                                 const uint32_t* __restrict__ tl, uint32_t tn) {
+                                                 const uint32_t* __restrict__ tl, uint32_t c, uint32_t c_end) {
     uint64_t m_t = 0;
-    uint32_t c = 0;
-    for (; c + 8 <= tn; c += 8) {  // 8 gathers in flight, folded two terms at a time
-        uint64_t x[8];
-        uint32_t e[8];
+    for (; c + 16 <= c_end; c += 16) {  // 16 gathers in flight, folded two terms at a time
+        uint64_t x[16];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            e[q] = tl[c + q];
-            x[q] = __ldg(mp_cm + (uint64_t)(e[q] & 0x3ffu) * rows + gr);
-        }
+        for (int q = 0; q < 16; ++q) x[q] = __ldg(mp_cm + (uint64_t)(tl[c + q] & 0x3ffu) * rows + gr);
 #pragma unroll
-        for (int q = 0; q < 8; q += 2)
-            m_t = fold(m_t) + signed_term(x[q], e[q] >> 31) + signed_term(x[q + 1], e[q + 1] >> 31);
+        for (int q = 0; q < 16; q += 2)
+            m_t = fold(m_t) + signed_term(x[q], tl[c + q] >> 31) + signed_term(x[q + 1], tl[c + q + 1] >> 31);
     }
-    for (; c < tn; ++c) {
+    for (; c < c_end; ++c) {
         const uint32_t e = tl[c];
         m_t = fold(m_t) + signed_term(__ldg(mp_cm + (uint64_t)(e & 0x3ffu) * rows + gr), e >> 31);
     }
@@ -740,19 +776,21 @@ __device__ __forceinline__ uint64_t m_times_t_cm(const uint64_t* __restrict__ mp
 // one row's sum per lane, and a shuffle hands row l to lane l.  Every entry
 // is an index into vt = [v_enc, 0, p - v_enc] (ELL_NEG, ELL_PAD), so a term
 // is one shared load and one add; the sums fold every 4 terms (4 terms
-// below 2^61 on top of a folded value stay below 2^64).
-__device__ __forceinline__ uint64_t s_times_v_warp(const DecodeCorpus& dc, uint64_t blk, const uint64_t* __restrict__ vt,
-                                                   uint32_t lane) {
+// below 2^61 on top of a folded value stay below 2^64).  Of PARTS warps that
+// share a slice, warp `part` takes every PARTS-th run of 32 chunks.
+template <uint32_t PARTS>
+__device__ __forceinline__ uint64_t s_times_v_part(const DecodeCorpus& dc, uint64_t blk, const uint64_t* __restrict__ vt,
+                                                   uint32_t part, uint32_t lane) {
     const uint32_t off = dc.s_off[blk], wdt = dc.s_w[blk];
     const uint4* base = reinterpret_cast<const uint4*>(dc.s_ell + off);  // slice data is 64 * wdt bytes
     const uint32_t chunks = wdt * 4;
     constexpr uint32_t PAD2 = ELL_PAD | (ELL_PAD << 16);
     uint64_t acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (uint32_t j0 = 0; j0 < chunks; j0 += 8 * 32) {
+    for (uint32_t j0 = 0; j0 < chunks; j0 += 8 * PARTS * 32) {
         uint4 ch[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            const uint32_t j = j0 + u * 32 + lane;
+            const uint32_t j = j0 + (u * PARTS + part) * 32 + lane;
             ch[u] = j < chunks ? __ldg(base + j) : make_uint4(PAD2, PAD2, PAD2, PAD2);
         }
 #pragma unroll
@@ -953,10 +991,10 @@ decode_topk_kernel(const uint64_t* __restrict__ r, DecodeCorpus dc, const ScanSe
                 const int32_t mt = m_times_t_warp(dc.m8_cm, (dc.rows + 31) & ~31ull, blk, tl, tn, lane);
                 m_t = mt >= 0 ? (uint64_t)mt : P - (uint64_t)(-(int64_t)mt);
             }
-            const uint64_t s_v = s_times_v_warp(dc, blk, vt, lane);
+            const uint64_t s_v = s_times_v_part<1>(dc, blk, vt, 0, lane);
             if (valid) {
-                if (!dc.m8_cm) m_t = m_times_t_cm(dc.mp_cm, dc.rows, gr, tl, tn);
-                const uint64_t dense = dense_terms_row(dc.alh_b, n1, gr, dyn_limbs);
+                if (!dc.m8_cm) m_t = m_times_t_cm(dc.mp_cm, dc.rows, gr, tl, 0, tn);
+                const uint64_t dense = dense_terms_row(dc.alh_b, n1, gr, dyn_limbs, 0, 2 * n1);
                 const uint64_t mv = sub_mod(sub_mod(rv, add_mod(dense, m_t)), s_v);
                 if (mv_out) mv_out[ridx] = mv;
                 score = to_signed(mv);
@@ -1497,7 +1535,18 @@ void launch_freivalds_finish(const uint64_t* d_z_part, const uint64_t* d_ur_part
 
 void launch_lt_times_v(const uint64_t* d_L, uint32_t n1, const uint64_t* d_v, uint32_t nq, uint64_t* d_x,
                        cudaStream_t s) {
-    lt_times_v_kernel<<<dim3(nq, LT_SPLIT), (1024 / n1) * n1, 0, s>>>(d_L, n1, d_v, d_x);
+    if (!nq) return;
+    const uint32_t run = lt_run(n1, nq);
+    lt_times_v_kernel<<<dim3(n1 / LT_COLS, (nq + run - 1) / run), LT_THREADS, 0, s>>>(d_L, n1, d_v, nq, run, d_x);
+}
+
+void launch_query_prep(const uint64_t* d_L, uint32_t n1, const uint64_t* d_v, uint32_t nq, uint64_t* d_x, uint8_t* d_w,
+                       uint32_t* d_zero, uint32_t zero_words, cudaStream_t s) {
+    const uint32_t run = lt_run(n1, nq);
+    const uint32_t lt_ctas = d_x ? (nq + run - 1) / run * (n1 / LT_COLS) : 0;
+    const uint32_t wimg_ctas = d_w ? nq * (64 * 16 * 16 / LT_THREADS) : 0;
+    query_prep_kernel<<<lt_ctas + wimg_ctas + 1, LT_THREADS, 0, s>>>(d_L, n1, d_v, nq, run, lt_ctas, d_x, wimg_ctas, d_w,
+                                                                      d_zero, zero_words);
 }
 
 void launch_dense_terms(const uint64_t* d_al_cm, const uint64_t* d_h_cm, uint64_t rows, uint32_t n1,
@@ -1518,7 +1567,6 @@ void launch_decode_topk(const uint64_t* d_r, const DecodeCorpus& dc, const ScanS
                         uint64_t* d_mv_out, uint32_t* d_out_ids, int64_t* d_out_scores, uint32_t* d_out_n,
                         cudaStream_t s) {
     if (!nq) return;
-    cudaMemsetAsync(scratch.done, 0, (uint64_t)nq * 4, s);
     const unsigned dyn = 2 * 2 * dc.n1 * 16;
     if (k >= 1 && k <= (uint32_t)WARP_TOPK_MAX) {  // every warp keeps its own list
         cudaFuncSetAttribute(decode_topk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 2 * 512 * 16);

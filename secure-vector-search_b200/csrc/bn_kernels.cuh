@@ -117,6 +117,13 @@ void launch_freivalds_finish(const uint64_t* d_z_part, const uint64_t* d_ur_part
 void launch_lt_times_v(const uint64_t* d_L, uint32_t n1, const uint64_t* d_v, uint32_t nq, uint64_t* d_x,
                        cudaStream_t s);
 
+// The per-query preparation of a pipeline run in one launch: x = L^T v (d_x
+// nullable: not wanted), the fused scan's diagonal byte images (bn_tc.cuh,
+// WIMG_BYTES_PER_QUERY bytes per query; d_w nullable) and zero_words u32 of
+// d_zero cleared (the run's status words and tickets).
+void launch_query_prep(const uint64_t* d_L, uint32_t n1, const uint64_t* d_v, uint32_t nq, uint64_t* d_x, uint8_t* d_w,
+                       uint32_t* d_zero, uint32_t zero_words, cudaStream_t s);
+
 // Dense decode terms only: out[i] = AL_i . g + H_i . x (FlatGpuState::
 // decode_dense_terms, gpu/mod.rs:390-408).
 void launch_dense_terms(const uint64_t* d_al_cm, const uint64_t* d_h_cm, uint64_t rows, uint32_t n1,
@@ -144,7 +151,7 @@ struct TopkScratch {
     int64_t* cand_s;    // [CTAs][k]
     uint32_t* cand_i;
     uint32_t* cand_n;   // [CTAs]
-    uint32_t* done;     // [nq] CTAs finished (decode_topk only; zeroed by its launcher)
+    uint32_t* done;     // [nq] CTAs finished (decode_topk only; zero before the launch)
 };
 
 // The corpus arrays the decode reads (layouts above).

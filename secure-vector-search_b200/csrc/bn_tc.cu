@@ -853,25 +853,6 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_constan
     }
 }
 
-// Diagonal byte image of each query for the fused scan MMA:
-// w[((q * 64 + strip) * 16 + s) * 128 + 8 j + a] = byte (s - a) of
-// v[q][strip * 16 + j] when 0 <= s - a <= 7, else 0.
-__global__ void query_wimg_kernel(const uint64_t* __restrict__ v, uint32_t nq, uint8_t* __restrict__ w) {
-    const uint64_t total = (uint64_t)nq * 64 * 16 * 16;  // (query, strip, s, j)
-    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t j = (uint32_t)(e & 15), s = (uint32_t)((e >> 4) & 15);
-        const uint64_t qs = e >> 8;  // q * 64 + strip
-        const uint64_t x = v[(qs >> 6) * N + (qs & 63) * 16 + j];
-        uint64_t word = 0;
-#pragma unroll
-        for (int a = 0; a < 8; ++a) {
-            const int b = (int)s - a;
-            if (b >= 0 && b <= 7) word |= ((x >> (8 * b)) & 0xffull) << (8 * a);
-        }
-        *reinterpret_cast<uint64_t*>(w + (qs * 16 + s) * 128 + 8 * j) = word;
-    }
-}
-
 // r[i] = sum over strip groups of r_part, then u_t . r for this pass's draws
 // rebuilt from their byte image (one CTA per 128-row block).  For the dot
 // products warp w takes trials w, w + 4, ... (at most 5) and lane l rows
@@ -933,15 +914,20 @@ tc_rreduce_kernel(const VerifySeg* __restrict__ vsegs, const TcBlock* __restrict
 // the splits add up); y == 8 sums every split-th row block's u_t . r
 // partial.  Splitting the panels over more CTAs keeps enough loads in flight
 // when a launch has few segments (one query: 245 panels at N = 1M).
+// The last CTA of a segment (a ticket taken after a device-scope fence, no
+// waiting) adds the shares up, a warp per trial, and keeps the first trial
+// whose sides differ (-1 if none).
 constexpr int FIN_CHUNKS = N / 128;
 
 __global__ void __launch_bounds__(128)
 tc_finish_kernel(const uint64_t* __restrict__ z_part, const uint64_t* __restrict__ ur_part,
                  const uint32_t* __restrict__ seg_panel0, const uint32_t* __restrict__ seg_block0,
                  const uint64_t* __restrict__ v_enc, const VerifySeg* __restrict__ vsegs, uint32_t trials,
-                 uint32_t split, uint64_t* __restrict__ chunks) {
+                 uint32_t split, uint64_t* chunks, uint32_t* __restrict__ done, uint64_t* __restrict__ ur,
+                 uint64_t* __restrict__ zv, int32_t* __restrict__ failed) {
     const uint32_t t = blockIdx.x, y = blockIdx.y, seg = blockIdx.z / split, sp = blockIdx.z % split;
     __shared__ uint64_t sh[4];
+    __shared__ int32_t last_s, first;
     uint64_t part = 0;
     if (y < FIN_CHUNKS) {
         const VerifySeg vs = vsegs[seg];
@@ -958,31 +944,26 @@ tc_finish_kernel(const uint64_t* __restrict__ z_part, const uint64_t* __restrict
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) part = add_mod(part, __shfl_xor_sync(FULLMASK, part, off));
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = part;
-    __syncthreads();
-    if (threadIdx.x == 0)
-        chunks[(((uint64_t)seg * trials + t) * (FIN_CHUNKS + 1) + y) * split + sp] =
-            add_mod(add_mod(sh[0], sh[1]), add_mod(sh[2], sh[3]));
-}
-
-// One CTA per segment, a warp per trial: ur_t and zv_t from the finish
-// kernel's shares, then the first trial whose sides differ (-1 if none).
-constexpr int DECIDE_WARPS = 8;
-
-__global__ void __launch_bounds__(DECIDE_WARPS * 32)
-tc_decide_kernel(const uint64_t* __restrict__ chunks, uint32_t trials, uint32_t split, uint64_t* __restrict__ ur,
-                 uint64_t* __restrict__ zv, int32_t* __restrict__ failed) {
-    const uint32_t seg = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __shared__ int32_t first;
-    if (threadIdx.x == 0) first = 0x7fffffff;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0) sh[warp] = part;
     __syncthreads();
     const uint32_t per = (FIN_CHUNKS + 1) * split;  // shares per trial; the last split of them are u . r
-    for (uint32_t t = warp; t < trials; t += DECIDE_WARPS) {
-        const uint64_t* c = chunks + ((uint64_t)seg * trials + t) * per;
+    if (threadIdx.x == 0) {
+        __stcg(chunks + ((uint64_t)seg * trials + t) * per + y * split + sp, add_mod(add_mod(sh[0], sh[1]), add_mod(sh[2], sh[3])));
+        __threadfence();  // the share is visible device-wide before its ticket
+        last_s = atomicAdd(&done[seg], 1u) == trials * per - 1;
+        first = 0x7fffffff;
+    }
+    __syncthreads();
+    if (!last_s) return;
+    __threadfence();
+    for (uint32_t tt = warp; tt < trials; tt += 4) {
+        const uint64_t* c = chunks + ((uint64_t)seg * trials + tt) * per;
         uint64_t a = 0, b = 0;
         for (uint32_t i = lane; i < per; i += 32) {
-            if (i < FIN_CHUNKS * split) b = add_mod(b, c[i]);
-            else a = add_mod(a, c[i]);
+            const uint64_t x = __ldcg(c + i);
+            if (i < FIN_CHUNKS * split) b = add_mod(b, x);
+            else a = add_mod(a, x);
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
@@ -990,13 +971,16 @@ tc_decide_kernel(const uint64_t* __restrict__ chunks, uint32_t trials, uint32_t 
             b = add_mod(b, __shfl_xor_sync(FULLMASK, b, off));
         }
         if (lane == 0) {
-            ur[(uint64_t)seg * trials + t] = a;
-            zv[(uint64_t)seg * trials + t] = b;
-            if (a != b) atomicMin(&first, (int32_t)t);
+            ur[(uint64_t)seg * trials + tt] = a;
+            zv[(uint64_t)seg * trials + tt] = b;
+            if (a != b) atomicMin(&first, (int32_t)tt);
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) failed[seg] = first == 0x7fffffff ? -1 : first;
+    if (threadIdx.x == 0) {
+        failed[seg] = first == 0x7fffffff ? -1 : first;
+        done[seg] = 0;
+    }
 }
 
 }  // namespace
@@ -1087,13 +1071,6 @@ void launch_tc_freivalds_small(const CUtensorMap& tmap_m, const CUtensorMap& tma
                                                              n_rows, trials_total, d_z_part, d_err, wl);
 }
 
-void launch_query_wimg(const uint64_t* d_v, uint32_t nq, uint8_t* d_w, cudaStream_t s) {
-    if (!nq) return;
-    const uint64_t total = (uint64_t)nq * 64 * 16 * 16;
-    const unsigned grid = (unsigned)std::min<uint64_t>((total + 255) / 256, 148 * 16);
-    query_wimg_kernel<<<grid, 256, 0, s>>>(d_v, nq, d_w);
-}
-
 void launch_tc_fused(const CUtensorMap& tmap_m, const CUtensorMap& tmap_u, const CUtensorMap& tmap_w,
                      const TcPanel* d_panels, uint32_t npanels, const VerifySeg* d_vsegs, uint32_t t_cnt,
                      uint32_t n_rows, uint32_t trials_total, uint64_t* d_z_part, uint64_t* d_r_part, uint64_t r_stride,
@@ -1123,8 +1100,8 @@ void launch_tc_rreduce(const VerifySeg* d_vsegs, const TcBlock* d_blocks, uint32
 
 void launch_tc_finish(const uint64_t* d_z_part, const uint64_t* d_ur_part, const uint32_t* d_seg_panel0,
                       const uint32_t* d_seg_block0, const uint64_t* d_v_enc, const VerifySeg* d_vsegs, uint32_t nseg,
-                      uint32_t trials, uint64_t* d_ur, uint64_t* d_zv, uint64_t* d_chunks, int32_t* d_failed,
-                      cudaStream_t s) {
+                      uint32_t trials, uint64_t* d_ur, uint64_t* d_zv, uint64_t* d_chunks, uint32_t* d_done,
+                      int32_t* d_failed, cudaStream_t s) {
     if (!nseg || !trials) return;
     const uint32_t split = tc_finish_split(nseg);
     const uint32_t per_launch = 65535u / split;  // grid.z limit
@@ -1132,9 +1109,9 @@ void launch_tc_finish(const uint64_t* d_z_part, const uint64_t* d_ur_part, const
         const uint32_t ns = nseg - s0 < per_launch ? nseg - s0 : per_launch;
         tc_finish_kernel<<<dim3(trials, FIN_CHUNKS + 1, ns * split), 128, 0, s>>>(
             d_z_part, d_ur_part, d_seg_panel0 + s0, d_seg_block0 + s0, d_v_enc, d_vsegs + s0, trials, split,
-            d_chunks + (uint64_t)s0 * trials * (FIN_CHUNKS + 1) * split);
+            d_chunks + (uint64_t)s0 * trials * (FIN_CHUNKS + 1) * split, d_done + s0, d_ur + (uint64_t)s0 * trials,
+            d_zv + (uint64_t)s0 * trials, d_failed + s0);
     }
-    tc_decide_kernel<<<nseg, DECIDE_WARPS * 32, 0, s>>>(d_chunks, trials, split, d_ur, d_zv, d_failed);
 }
 
 }  // namespace bn

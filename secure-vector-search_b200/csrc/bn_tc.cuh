@@ -88,7 +88,7 @@ void launch_tc_freivalds_small(const CUtensorMap& tmap_m, const CUtensorMap& tma
 // the tensor cores: z_part as above plus r_part[group][r index] (3-strip
 // group partial dots with the query, r_stride = total r entries, 22 groups),
 // summed by launch_tc_rreduce.  tmap_w: the queries' diagonal byte images
-// (launch_query_wimg) {128, nq * 1024}, box {128, 48}, swizzle 128B.
+// (launch_query_prep) {128, nq * 1024}, box {128, 48}, swizzle 128B.
 void launch_tc_fused(const CUtensorMap& tmap_m, const CUtensorMap& tmap_u, const CUtensorMap& tmap_w,
                      const TcPanel* d_panels, uint32_t npanels, const VerifySeg* d_vsegs, uint32_t t_cnt,
                      uint32_t n_rows, uint32_t trials_total, uint64_t* d_z_part, uint64_t* d_r_part, uint64_t r_stride,
@@ -96,9 +96,6 @@ void launch_tc_fused(const CUtensorMap& tmap_m, const CUtensorMap& tmap_u, const
 inline uint32_t tc_groups(uint32_t) { return 22u; }  // strip groups of the fused pass (3 strips each)
 constexpr uint32_t WIMG_BYTES_PER_QUERY = 64u * 16u * 128u;
 constexpr uint32_t WIMG_BOX_ROWS = 48;  // one strip group's diagonal rows
-// w[((q * 64 + strip) * 16 + s) * 128 + 8 j + a] = byte (s - a) of
-// v[q][strip * 16 + j] (0 <= s - a <= 7), else 0.
-void launch_query_wimg(const uint64_t* d_v, uint32_t nq, uint8_t* d_w, cudaStream_t s);
 // r = sum of the group partials, and u_t . r partials for the pass's trials
 // from the U byte image.
 void launch_tc_rreduce(const VerifySeg* d_vsegs, const TcBlock* d_blocks, uint32_t nblocks, const uint64_t* d_r_part,
@@ -110,13 +107,15 @@ void launch_tc_rreduce(const VerifySeg* d_vsegs, const TcBlock* d_blocks, uint32
 // d_chunks: scratch of tc_finish_words(nseg, trials) words (the shares of z . v
 // and u . r that the finish kernel's CTAs write and the decide kernel sums).
 // With few segments each one's panels are split over tc_finish_split CTAs.
+// d_done: nseg tickets, zero before the launch (the last CTA of a segment
+// decides it and leaves its ticket zero).
 inline uint32_t tc_finish_split(uint32_t nseg) { return nseg <= 4 ? 16u : 1u; }
 inline uint64_t tc_finish_words(uint32_t nseg, uint32_t trials) {
     return (uint64_t)nseg * trials * (N / 128 + 1) * tc_finish_split(nseg);
 }
 void launch_tc_finish(const uint64_t* d_z_part, const uint64_t* d_ur_part, const uint32_t* d_seg_panel0,
                       const uint32_t* d_seg_block0, const uint64_t* d_v_enc, const VerifySeg* d_vsegs, uint32_t nseg,
-                      uint32_t trials, uint64_t* d_ur, uint64_t* d_zv, uint64_t* d_chunks, int32_t* d_failed,
-                      cudaStream_t s);
+                      uint32_t trials, uint64_t* d_ur, uint64_t* d_zv, uint64_t* d_chunks, uint32_t* d_done,
+                      int32_t* d_failed, cudaStream_t s);
 
 }  // namespace bn
