@@ -35,7 +35,8 @@ struct BlockPlan {
     bool verify_only = false;  // Protocol 2 over claimed responses only
     uint64_t rows = 0, nld = 0, npad = 0;
     uint32_t t_pass = 0, n_rows = 0;   // trials per Freivalds pass, U rows (8 * even trials)
-    uint32_t nblocks = 0, npanels = 0;  // U row blocks, z panels (4096 rows)
+    uint32_t panel_rows = TC_PANEL_ROWS;
+    uint32_t nblocks = 0, npanels = 0;  // U row blocks, z panels
     // tuned GEMM configuration
     uint32_t w_tile = 256, stages = 4, order = 0, a_res = 0, k_panel4 = 16384;
     uint32_t ks2 = 1;  // two K steps per pipeline stage in G1-G3
@@ -370,7 +371,8 @@ int block_plan_create(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k, uint3
     b->t_pass = std::min<uint32_t>(std::max<uint32_t>(trials, 1), TC_MAX_TRIALS);
     b->n_rows = 8 * ((b->t_pass + 1) & ~1u);
     b->nblocks = (uint32_t)((c.rows + TC_ROWS - 1) / TC_ROWS);
-    b->npanels = (uint32_t)((c.rows + TC_PANEL_ROWS - 1) / TC_PANEL_ROWS);
+    b->panel_rows = tc_panel_rows(b->nblocks, 1);
+    b->npanels = (uint32_t)((c.rows + b->panel_rows - 1) / b->panel_rows);
     b->w_tile = (uint32_t)std::min<uint64_t>(256, align_up(8ull * B, 16));
     b->a_res = 8ull * B > b->w_tile ? 1u : 0u;  // A tiles reused across several W tiles
     if (!c.block_ready) b->a_res = 0;
@@ -405,8 +407,8 @@ int block_plan_create(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k, uint3
         for (uint32_t i = 0; i < b->nblocks; ++i) blocks[i] = TcBlock{0, i * (uint32_t)TC_ROWS};
         auto* panels = reinterpret_cast<TcPanel*>(hm.data() + (b->o_panels - b->o_vseg));
         for (uint32_t p = 0; p < b->npanels; ++p) {
-            const uint64_t r0 = (uint64_t)p * TC_PANEL_ROWS;
-            panels[p] = TcPanel{r0, (uint32_t)std::min<uint64_t>(TC_PANEL_ROWS, c.rows - r0),
+            const uint64_t r0 = (uint64_t)p * b->panel_rows;
+            panels[p] = TcPanel{r0, (uint32_t)std::min<uint64_t>(b->panel_rows, c.rows - r0),
                                 (uint32_t)(r0 / TC_ROWS), 0, 0};
         }
         if (cudaMemsetAsync(b->ws.p, 0, b->o_vseg, s) != cudaSuccess ||
@@ -447,7 +449,8 @@ uint64_t block_plan_estimate(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k
     b.t_pass = std::min<uint32_t>(std::max<uint32_t>(trials, 1), TC_MAX_TRIALS);
     b.n_rows = 8 * ((b.t_pass + 1) & ~1u);
     b.nblocks = (uint32_t)((c.rows + TC_ROWS - 1) / TC_ROWS);
-    b.npanels = (uint32_t)((c.rows + TC_PANEL_ROWS - 1) / TC_PANEL_ROWS);
+    b.panel_rows = tc_panel_rows(b.nblocks, 1);
+    b.npanels = (uint32_t)((c.rows + b.panel_rows - 1) / b.panel_rows);
     b.topk_ctas = (int)std::max<uint64_t>(1, std::min<uint64_t>((c.rows + 511) / 512, (uint64_t)f->e.ctx->num_sms * 4 / B));
     return block_layout(b, c.n1, (uint32_t)align_up(2ull * c.n1, 128), false);
 }

@@ -403,14 +403,17 @@ void finish_meta(HostMeta& hm) {
     hm.panels.clear();
     hm.seg_block0.assign(hm.vsegs.size() + 1, 0);
     hm.seg_panel0.assign(hm.vsegs.size() + 1, 0);
+    uint64_t max_blocks = 0;
+    for (const VerifySeg& v : hm.vsegs) max_blocks = std::max<uint64_t>(max_blocks, (v.rows + TC_ROWS - 1) / TC_ROWS);
+    const uint32_t panel_rows = tc_panel_rows(max_blocks, hm.vsegs.size());
     for (uint32_t s = 0; s < hm.vsegs.size(); ++s) {
         const VerifySeg& v = hm.vsegs[s];
         hm.seg_block0[s] = (uint32_t)hm.blocks.size();
         hm.seg_panel0[s] = (uint32_t)hm.panels.size();
         for (uint32_t i0 = 0; i0 < v.rows; i0 += TC_ROWS) hm.blocks.push_back(TcBlock{s, i0});
-        for (uint32_t p0 = 0; p0 < v.rows; p0 += TC_PANEL_ROWS)
-            hm.panels.push_back(TcPanel{v.row0 + p0, std::min<uint32_t>(TC_PANEL_ROWS, v.rows - p0),
-                                        hm.seg_block0[s] + p0 / TC_ROWS, s, 0});
+        for (uint64_t p0 = 0; p0 < v.rows; p0 += panel_rows)
+            hm.panels.push_back(TcPanel{v.row0 + p0, (uint32_t)std::min<uint64_t>(panel_rows, v.rows - p0),
+                                        hm.seg_block0[s] + (uint32_t)(p0 / TC_ROWS), s, 0});
     }
     hm.seg_block0.back() = (uint32_t)hm.blocks.size();
     hm.seg_panel0.back() = (uint32_t)hm.panels.size();

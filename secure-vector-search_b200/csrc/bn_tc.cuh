@@ -20,8 +20,33 @@
 namespace bn {
 
 constexpr int TC_ROWS = 128;         // rows (K) per stage
-constexpr int TC_PANEL_ROWS = 4096;  // rows accumulated in TMEM before a drain (4096 * 255^2 < 2^31)
+constexpr int TC_PANEL_ROWS = 4096;  // rows accumulated in TMEM before a drain (twice as many * 255^2 < 2^31)
 constexpr int TC_MAX_TRIALS = 20;    // per pass: N = 8 * trials_padded <= 160
+
+// Rows per panel for `nseg` segments of at most `blocks` 128-row blocks each: a
+// multiple of 128 up to 2 * TC_PANEL_ROWS.  A launch deals panels x 22 strip
+// groups out to the SMs in rounds, and a round takes as long as a panel's
+// blocks plus its drain (about TC_DRAIN_BLOCKS blocks' time), so the size is
+// the one with the shortest whole schedule: the fixed 4096 rows left a 5,000-
+// row corpus on 44 SMs with panels of 32 and 8 blocks, and cost a 200,000-row
+// one 8 rounds of 32 blocks where 7 of 34 do.  Many segments (inverted lists)
+// keep 4096: most are a single shorter panel.
+constexpr uint32_t TC_DRAIN_BLOCKS = 4, TC_SMS = 148;
+inline uint32_t tc_panel_rows(uint64_t blocks, uint64_t nseg) {
+    if (nseg > 8 || !blocks) return TC_PANEL_ROWS;
+    uint32_t best = TC_PANEL_ROWS / 128;
+    uint64_t best_cost = ~0ull;
+    for (uint32_t pb = 2 * TC_PANEL_ROWS / 128; pb >= 2; --pb) {
+        const uint64_t panels = (blocks + pb - 1) / pb * nseg;
+        const uint64_t rounds = (panels * 22 + TC_SMS - 1) / TC_SMS;
+        const uint64_t cost = rounds * ((pb < blocks ? pb : blocks) + TC_DRAIN_BLOCKS);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = pb;
+        }
+    }
+    return best * 128;
+}
 
 // One panel of a verify segment: rows [row0, row0 + rows) of m_enc, whose U
 // tiles start at row block `rb0` of the U buffer.
