@@ -57,12 +57,19 @@ __device__ __forceinline__ uint32_t find_seg(const uint64_t* __restrict__ seg_bl
 // ------------------------------------------------------------------ scan, TMA pipeline
 // One producer warp streams each 4-row block (up to 32 KiB, contiguous in
 // m_enc) into a ring of shared-memory stages with a single cp.async.bulk;
-// four consumer groups of four warps take the stages round-robin.  Every
+// three consumer groups of four warps take the stages round-robin.  A stage
+// must always fall to the same group: a barrier wait names a phase by its parity,
+// so a group that met a stage on every second round only would take the round
+// before last for the one it waits for whenever the round between them, another
+// group's, is late (copies finish out of order, most of all on cold pages), read
+// the stage early and release it twice.  With four groups on six stages that
+// happened: wrong r and launch failures at 50,001 rows.  Every
 // mbarrier wait is bounded: on timeout the CTA records an error in *err
 // and stops, so a lost completion cannot hang the GPU.
 constexpr int TS_STAGES = 6;
-constexpr int TS_GROUPS = 4;
-constexpr int TS_CONSUMERS = 32 * 4 * TS_GROUPS;   // 512
+constexpr int TS_GROUPS = 3;
+static_assert(TS_STAGES % TS_GROUPS == 0, "a stage must always fall to the same group");
+constexpr int TS_CONSUMERS = 32 * 4 * TS_GROUPS;   // 384
 constexpr int TS_THREADS = TS_CONSUMERS + 32;      // + producer warp
 constexpr uint32_t TS_STAGE_BYTES = SCAN_ROWS * N * 8;  // 32 KiB
 constexpr long long WAIT_CYCLES = 2000000000ll;    // ~1 s at 1.9 GHz
