@@ -15,26 +15,101 @@
 namespace bn {
 namespace {
 
-constexpr uint32_t RT_THREADS = 256;
+constexpr uint32_t RT_THREADS = 64;
+constexpr uint32_t RT_BATCH = 32, RT_DEPTH = 6;  // centroid values per copy group, groups in flight
 constexpr uint32_t RT_SORT_THREADS = 1024;
 
-// dist[q][c] for centroid c = blockIdx.x * 256 + threadIdx.x; centroids are
-// stored dimension-major (cent_t[i][c]) so a warp's loads are coalesced.
+// One of a thread's own centroid values into its own column of the ring (only
+// this thread reads it, so the copy groups need no barrier).
+__device__ __forceinline__ void copy4(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// dist[q][c] for centroid c = blockIdx.x * 64 + threadIdx.x and QPT queries
+// from blockIdx.y * QPT on; centroids are stored dimension-major (cent_t[i][c])
+// so a warp's loads are coalesced.  The sum over the dimensions is a serial
+// chain by definition, so the kernel is bound by the latency of its loads: a
+// thread keeps RT_DEPTH groups of RT_BATCH of them in flight through a ring of
+// its own in shared memory (one load after the other: 54 us for 640 lists of 768
+// dimensions), and each serves QPT queries, whose chains overlap.  Dimensions past
+// d are zero on both sides and add +0 to a sum that is never -0.
+template <int QPT>
 __global__ void __launch_bounds__(RT_THREADS)
 route_dist_kernel(const float* __restrict__ cent_t, uint32_t nlist, uint32_t d, const float* __restrict__ queries,
-                  float* __restrict__ dist) {
-    extern __shared__ float qs[];
-    const uint32_t q = blockIdx.y;
-    for (uint32_t i = threadIdx.x; i < d; i += blockDim.x) qs[i] = queries[(uint64_t)q * d + i];
-    __syncthreads();
+                  uint32_t nq, float* __restrict__ dist) {
+    extern __shared__ float ring[];  // [RT_DEPTH][RT_BATCH][RT_THREADS], then qs [d rounded up to RT_BATCH][QPT]
+    float* qs = ring + RT_DEPTH * RT_BATCH * RT_THREADS;
+    const uint32_t q0 = blockIdx.y * QPT;
+    const uint32_t groups = (d + RT_BATCH - 1) / RT_BATCH;
     const uint32_t c = blockIdx.x * RT_THREADS + threadIdx.x;
-    if (c >= nlist) return;
-    float s = 0.0f;
-    for (uint32_t i = 0; i < d; ++i) {
-        const float t = __fsub_rn(qs[i], cent_t[(uint64_t)i * nlist + c]);
-        s = __fadd_rn(s, __fmul_rn(t, t));
+    const bool on = c < nlist;
+    auto fetch = [&](uint32_t g) {
+        float* dst = ring + (g % RT_DEPTH) * RT_BATCH * RT_THREADS + threadIdx.x;
+#pragma unroll 8
+        for (uint32_t k = 0; k < RT_BATCH; ++k) {
+            const uint32_t i = g * RT_BATCH + k;
+            if (on && i < d) copy4(dst + k * RT_THREADS, cent_t + (uint64_t)i * nlist + c);
+            else dst[k * RT_THREADS] = 0.0f;
+        }
+    };
+    for (uint32_t g = 0; g < RT_DEPTH - 1; ++g) {
+        if (g < groups) fetch(g);
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    dist[(uint64_t)q * nlist + c] = __fsqrt_rn(s);
+#pragma unroll
+    for (int u = 0; u < QPT; ++u)
+        for (uint32_t i = threadIdx.x; i < groups * RT_BATCH; i += RT_THREADS)
+            qs[i * QPT + u] = i < d && q0 + u < nq ? queries[(uint64_t)(q0 + u) * d + i] : 0.0f;
+    __syncthreads();
+    float s[QPT];
+#pragma unroll
+    for (int u = 0; u < QPT; ++u) s[u] = 0.0f;
+    for (uint32_t g = 0; g < groups; ++g) {
+        if (g + RT_DEPTH - 1 < groups) fetch(g + RT_DEPTH - 1);  // the slot read in the last round
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(RT_DEPTH - 1) : "memory");
+        const float* src = ring + (g % RT_DEPTH) * RT_BATCH * RT_THREADS + threadIdx.x;
+        const float* qg = qs + g * RT_BATCH * QPT;
+#pragma unroll
+        for (uint32_t k = 0; k < RT_BATCH; ++k) {
+            const float x = src[k * RT_THREADS];
+#pragma unroll
+            for (int u = 0; u < QPT; ++u) {
+                const float t = __fsub_rn(qg[k * QPT + u], x);
+                s[u] = __fadd_rn(s[u], __fmul_rn(t, t));
+            }
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < QPT; ++u)
+        if (on && q0 + u < nq) dist[(uint64_t)(q0 + u) * nlist + c] = __fsqrt_rn(s[u]);
+}
+
+// At most 1024 lists: one key per thread.  Exchanges over fewer than 32
+// threads are shuffles; the 15 wider ones (of 55 at 1024 keys) go through
+// shared memory, two buffers in turn so that each costs one barrier.
+__global__ void __launch_bounds__(RT_SORT_THREADS)
+route_select_small_kernel(const float* __restrict__ dist, uint32_t nlist, uint32_t np, uint32_t* __restrict__ probes) {
+    __shared__ uint64_t xch[2][RT_SORT_THREADS];
+    const uint32_t q = blockIdx.x, i = threadIdx.x;  // blockDim.x: a power of two, at least 32
+    uint64_t key = i < nlist ? ((uint64_t)__float_as_uint(dist[(uint64_t)q * nlist + i]) << 32) | i : ~0ull;
+    uint32_t buf = 0;
+    for (uint32_t size = 2; size <= blockDim.x; size <<= 1)
+        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+            uint64_t other;
+            if (stride >= 32) {
+                xch[buf][i] = key;
+                __syncthreads();
+                other = xch[buf][i ^ stride];
+                buf ^= 1;
+            } else {
+                other = __shfl_xor_sync(0xffffffffu, key, stride);
+            }
+            const bool low = (i & stride) == 0, up = (i & size) == 0;
+            key = (low == up) == (key < other) ? key : other;
+        }
+    if (i < np) probes[(uint64_t)q * np + i] = (uint32_t)key;
 }
 
 // One CTA per query: keys (distance bits << 32 | index) -- the bits of a
@@ -111,14 +186,28 @@ int bn_ivf_route(bn_ivf* v, uint32_t B, const float* queries, uint32_t nprobe, u
     char* dv = v->e.ws.at<char>();
     cudaStream_t s = v->e.stream;
     CU(cudaMemcpyAsync(dv + o_q, queries, (uint64_t)B * d * 4, cudaMemcpyHostToDevice, s));
-    route_dist_kernel<<<dim3((nlist + RT_THREADS - 1) / RT_THREADS, B), RT_THREADS, d * 4, s>>>(
-        v->cent_t.at<float>(), nlist, d, reinterpret_cast<const float*>(dv + o_q), reinterpret_cast<float*>(dv + o_d));
-    uint32_t pow2 = 1;
+    // Queries per thread: each centroid value loaded serves QPT queries, as long
+    // as the grid still covers the chip (two warps per CTA) and the query rows fit
+    // beside the ring.
+    const float* dc = v->cent_t.at<float>();
+    const float* dq = reinterpret_cast<const float*>(dv + o_q);
+    float* dd = reinterpret_cast<float*>(dv + o_d);
+    const uint32_t gx = (nlist + RT_THREADS - 1) / RT_THREADS;
+    const uint32_t ring = RT_DEPTH * RT_BATCH * RT_THREADS * 4, qrow = (d + RT_BATCH - 1) / RT_BATCH * RT_BATCH * 4;
+    const uint32_t qpt = (uint64_t)gx * ((B + 3) / 4) >= (uint32_t)v->e.ctx->num_sms && qrow <= 16 * 1024 ? 4 : 1;
+    auto dist_fn = qpt == 4 ? route_dist_kernel<4> : route_dist_kernel<1>;
+    const int dist_smem = (int)(ring + qpt * qrow);
+    CU(cudaFuncSetAttribute(dist_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dist_smem));
+    dist_fn<<<dim3(gx, (B + qpt - 1) / qpt), RT_THREADS, dist_smem, s>>>(dc, nlist, d, dq, B, dd);
+    uint32_t pow2 = 32;
     while (pow2 < nlist) pow2 <<= 1;
-    const int smem = (int)(pow2 * 8);
-    CU(cudaFuncSetAttribute(route_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_MAX_NLIST * 8));
-    route_select_kernel<<<B, RT_SORT_THREADS, smem, s>>>(reinterpret_cast<const float*>(dv + o_d), nlist, np, pow2,
-                                                         reinterpret_cast<uint32_t*>(dv + o_p));
+    uint32_t* dp = reinterpret_cast<uint32_t*>(dv + o_p);
+    if (pow2 <= RT_SORT_THREADS) {
+        route_select_small_kernel<<<B, pow2, 0, s>>>(dd, nlist, np, dp);
+    } else {
+        CU(cudaFuncSetAttribute(route_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_MAX_NLIST * 8));
+        route_select_kernel<<<B, RT_SORT_THREADS, (int)(pow2 * 8), s>>>(dd, nlist, np, pow2, dp);
+    }
     CU(cudaGetLastError());
     CU(cudaMemcpyAsync(probes, dv + o_p, (uint64_t)B * np * 4, cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
