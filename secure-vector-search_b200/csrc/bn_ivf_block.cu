@@ -58,7 +58,7 @@ struct IvChunk {
     uint32_t ublk;  // first 128-row block of the list's U image
     uint32_t rows;
 };
-constexpr uint32_t IV_CHUNK_ROWS = 2048;
+constexpr uint32_t IV_CHUNK_ROWS = 512;
 
 // u . r work of one CTA: chunk c of a list (its U blocks from ublk0 on) for
 // up to UR_SLAB of the list's pairs (list-major positions lp0 ...).
@@ -69,7 +69,7 @@ struct IvUrTask {
 };
 constexpr uint32_t UR_SLAB = 8;
 constexpr uint32_t UR_WARPS = 8;
-constexpr uint32_t UR_PER_WARP = (UR_SLAB * TC_MAX_TRIALS + UR_WARPS - 1) / UR_WARPS;
+constexpr uint32_t UR_PER_WARP = (TC_MAX_TRIALS + UR_WARPS - 1) / UR_WARPS;  // trials
 
 // One distinct list of a batch: a group of the grouped GEMMs.
 struct IvGroup {
@@ -138,17 +138,21 @@ __device__ __forceinline__ void mac128(uint64_t& lo, uint64_t& hi, uint64_t a, u
 
 // u_t . r for the pairs of one list chunk, trials [t_base, t_base + t_cnt):
 // the chunk's U blocks (launch_tc_ugen, per-block images: byte a of u_t[i] at
-// row 8t + a, column i) are read once each into shared memory and serve every
-// pair of the slab.  Warp w owns the (pair, trial) combos w, w + 8, ... for
-// the whole chunk; lane l takes rows 4l .. 4l + 3 of each block, reads one
-// 32-bit word from each of the 8 byte rows of trial t and transposes them
-// into the four u_t values.  16 blocks x 4 rows = 64 products (< 2^122 each)
-// per lane and combo are summed in 128 bits.
+// row 8t + a, column i) and the slab's r are read once each into shared memory.
+// Warp w owns trials w, w + 8, ... for the whole chunk; lane l takes rows 4l ..
+// 4l + 3 of each block, reads one 32-bit word from each of the 8 byte rows of
+// trial t, transposes them into the four u_t values and multiplies them with
+// every pair's r.  4 blocks x 4 rows = 16 products (< 2^122 each) per lane,
+// trial and pair are summed in 128 bits.  Latency bound: chunks of 2048 rows,
+// with r read from memory once per trial, left a batch of 512 pairs on 175 CTAs
+// (115 us) and one of 4,096 at 230 us.
 __global__ void __launch_bounds__(UR_WARPS * 32)
 ur_lists_kernel(const IvUrTask* __restrict__ tasks, const IvPair* __restrict__ pairs, const uint32_t* __restrict__ lmi,
                 const uint8_t* __restrict__ ub, uint32_t n_rows, uint32_t t_base, uint32_t t_cnt,
                 uint32_t trials_total, const uint64_t* __restrict__ r, uint64_t* __restrict__ ur_part) {
     extern __shared__ uint4 u_img[];  // one U block: 8 t_cnt rows x 128 bytes
+    // r of a block per pair: rows 4l, 4l + 1 of lane l, then its rows 4l + 2, 4l + 3
+    __shared__ ulonglong2 r_s[UR_SLAB][2][TC_ROWS / 4];
     __shared__ uint64_t rbase_s[UR_SLAB];
     __shared__ uint32_t out_s[UR_SLAB];
     const IvUrTask tk = tasks[blockIdx.x];
@@ -158,54 +162,62 @@ ur_lists_kernel(const IvUrTask* __restrict__ tasks, const IvPair* __restrict__ p
         rbase_s[threadIdx.x] = pr.out0 + (uint64_t)tk.c * IV_CHUNK_ROWS;
         out_s[threadIdx.x] = pr.ch0 + tk.c;
     }
-    const uint32_t combos = tk.npairs * t_cnt;
-    uint64_t lo[UR_PER_WARP], hi[UR_PER_WARP];
+    uint64_t lo[UR_PER_WARP][UR_SLAB], hi[UR_PER_WARP][UR_SLAB];
 #pragma unroll
-    for (uint32_t ii = 0; ii < UR_PER_WARP; ++ii) lo[ii] = hi[ii] = 0;
+    for (uint32_t ii = 0; ii < UR_PER_WARP; ++ii)
+#pragma unroll
+        for (uint32_t p = 0; p < UR_SLAB; ++p) lo[ii][p] = hi[ii][p] = 0;
     const uint32_t nblk = (tk.rows + TC_ROWS - 1) / TC_ROWS;
     const uint32_t img_words = 8 * t_cnt * TC_ROWS / 16;
     const uint8_t* img = reinterpret_cast<const uint8_t*>(u_img) + 4 * lane;
     for (uint32_t b = 0; b < nblk; ++b) {
-        __syncthreads();  // the previous block's image is no longer read (and rbase_s is set)
+        __syncthreads();  // the previous block is no longer read (and rbase_s is set)
         const uint4* src = reinterpret_cast<const uint4*>(ub + (uint64_t)(tk.ublk0 + b) * n_rows * TC_ROWS);
         for (uint32_t x = threadIdx.x; x < img_words; x += blockDim.x) u_img[x] = src[x];
+        for (uint32_t x = threadIdx.x; x < tk.npairs * TC_ROWS; x += blockDim.x) {
+            const uint32_t p = x / TC_ROWS, i = x % TC_ROWS, row = b * TC_ROWS + i;
+            reinterpret_cast<uint64_t*>(r_s[p][(i >> 1) & 1])[2 * (i >> 2) + (i & 1)] =
+                row < tk.rows ? r[rbase_s[p] + row] : 0;
+        }
         __syncthreads();
-        const uint32_t i0 = b * TC_ROWS + 4 * lane;
 #pragma unroll
         for (uint32_t ii = 0; ii < UR_PER_WARP; ++ii) {
-            const uint32_t k = warp + UR_WARPS * ii;
-            if (k < combos) {
-                const uint32_t pk = k / t_cnt, t = k % t_cnt;
-                const uint64_t rb = rbase_s[pk];
-                uint64_t rv[4];
+            const uint32_t t = warp + UR_WARPS * ii;
+            if (t >= t_cnt) break;  // warp-uniform
+            uint32_t w[8];
 #pragma unroll
-                for (int h = 0; h < 4; ++h) rv[h] = i0 + h < tk.rows ? r[rb + i0 + h] : 0;
-                uint32_t w[8];
+            for (int a = 0; a < 8; ++a) w[a] = *reinterpret_cast<const uint32_t*>(img + (8 * t + a) * TC_ROWS);
+            // 8 x 4 byte transpose: byte a of u[h] = byte h of w[a]
+            const uint32_t l01 = __byte_perm(w[0], w[1], 0x5140), h01 = __byte_perm(w[0], w[1], 0x7362);
+            const uint32_t l23 = __byte_perm(w[2], w[3], 0x5140), h23 = __byte_perm(w[2], w[3], 0x7362);
+            const uint32_t l45 = __byte_perm(w[4], w[5], 0x5140), h45 = __byte_perm(w[4], w[5], 0x7362);
+            const uint32_t l67 = __byte_perm(w[6], w[7], 0x5140), h67 = __byte_perm(w[6], w[7], 0x7362);
+            uint64_t u[4];
+            u[0] = __byte_perm(l01, l23, 0x5410) | ((uint64_t)__byte_perm(l45, l67, 0x5410) << 32);
+            u[1] = __byte_perm(l01, l23, 0x7632) | ((uint64_t)__byte_perm(l45, l67, 0x7632) << 32);
+            u[2] = __byte_perm(h01, h23, 0x5410) | ((uint64_t)__byte_perm(h45, h67, 0x5410) << 32);
+            u[3] = __byte_perm(h01, h23, 0x7632) | ((uint64_t)__byte_perm(h45, h67, 0x7632) << 32);
 #pragma unroll
-                for (int a = 0; a < 8; ++a) w[a] = *reinterpret_cast<const uint32_t*>(img + (8 * t + a) * TC_ROWS);
-                // 8 x 4 byte transpose: byte a of u[h] = byte h of w[a]
-                const uint32_t l01 = __byte_perm(w[0], w[1], 0x5140), h01 = __byte_perm(w[0], w[1], 0x7362);
-                const uint32_t l23 = __byte_perm(w[2], w[3], 0x5140), h23 = __byte_perm(w[2], w[3], 0x7362);
-                const uint32_t l45 = __byte_perm(w[4], w[5], 0x5140), h45 = __byte_perm(w[4], w[5], 0x7362);
-                const uint32_t l67 = __byte_perm(w[6], w[7], 0x5140), h67 = __byte_perm(w[6], w[7], 0x7362);
-                uint64_t u[4];
-                u[0] = __byte_perm(l01, l23, 0x5410) | ((uint64_t)__byte_perm(l45, l67, 0x5410) << 32);
-                u[1] = __byte_perm(l01, l23, 0x7632) | ((uint64_t)__byte_perm(l45, l67, 0x7632) << 32);
-                u[2] = __byte_perm(h01, h23, 0x5410) | ((uint64_t)__byte_perm(h45, h67, 0x5410) << 32);
-                u[3] = __byte_perm(h01, h23, 0x7632) | ((uint64_t)__byte_perm(h45, h67, 0x7632) << 32);
-#pragma unroll
-                for (int h = 0; h < 4; ++h) mac128(lo[ii], hi[ii], u[h], rv[h]);
+            for (uint32_t p = 0; p < UR_SLAB; ++p) {
+                if (p >= tk.npairs) break;  // CTA-uniform
+                const ulonglong2 ra = r_s[p][0][lane], rb = r_s[p][1][lane];
+                mac128(lo[ii][p], hi[ii][p], u[0], ra.x);
+                mac128(lo[ii][p], hi[ii][p], u[1], ra.y);
+                mac128(lo[ii][p], hi[ii][p], u[2], rb.x);
+                mac128(lo[ii][p], hi[ii][p], u[3], rb.y);
             }
         }
     }
 #pragma unroll
     for (uint32_t ii = 0; ii < UR_PER_WARP; ++ii) {
-        const uint32_t k = warp + UR_WARPS * ii;
-        if (k < combos) {  // warp-uniform
-            uint64_t x = reduce128(lo[ii], hi[ii]);
+        const uint32_t t = warp + UR_WARPS * ii;
+#pragma unroll
+        for (uint32_t p = 0; p < UR_SLAB; ++p) {
+            if (t >= t_cnt || p >= tk.npairs) continue;  // warp-uniform
+            uint64_t x = reduce128(lo[ii][p], hi[ii][p]);
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) x = add_mod(x, __shfl_xor_sync(0xffffffffu, x, off));
-            if (lane == 0) ur_part[(uint64_t)out_s[k / t_cnt] * trials_total + t_base + k % t_cnt] = x;
+            if (lane == 0) ur_part[(uint64_t)out_s[p] * trials_total + t_base + t] = x;
         }
     }
 }
@@ -223,11 +235,11 @@ __global__ void zsum_lists_kernel(const uint64_t* __restrict__ z_part, const IvZ
 
 // zv[i][t] = z_t^u . v_{q(i)} for pairs ZV_PAIRS * blockIdx.z, ... of list
 // u = blockIdx.x and trials [ZV_TRIALS * blockIdx.y, + ZV_TRIALS): list u's z
-// (at zbase + zoff[u]: its single panel's z_part, or its panel sum) is read
-// into registers (thread x holds elements x + 128 e) and serves up to
-// ZV_PAIRS of the list's pairs, whose v rows come from L2 (a list probed by
-// many queries of the batch spreads over several CTAs).  8 products (< 2^122
-// each) per thread and trial are summed in 128 bits.
+// (at zbase + zoff[u]: its single panel's z_part, or its panel sum) is read into
+// shared memory and serves up to ZV_PAIRS of the list's pairs, whose v rows come
+// from L2, a warp per pair: a lane takes columns lane, lane + 32, ... and sums its
+// 32 products (< 2^122 each) per trial in 128 bits.  (A pair at a time by the
+// whole CTA, with a cross-warp sum and two barriers each: 135 us for 4,096 pairs.)
 constexpr uint32_t ZV_TRIALS = 4;
 constexpr uint32_t ZV_PAIRS = 8;
 __global__ void __launch_bounds__(128) zv_lists_kernel(const uint64_t* __restrict__ zbase,
@@ -244,33 +256,33 @@ __global__ void __launch_bounds__(128) zv_lists_kernel(const uint64_t* __restric
     if (k0 >= g.n) return;  // CTA-uniform: this list has fewer pairs
     const uint32_t k1 = min(g.n, k0 + ZV_PAIRS);
     const uint64_t* zr = zbase + zoff[u] + (uint64_t)t0 * N;
-    uint64_t z[ZV_TRIALS][N / 128];
+    __shared__ uint64_t z[ZV_TRIALS][N];
 #pragma unroll
     for (uint32_t tt = 0; tt < ZV_TRIALS; ++tt)
 #pragma unroll
-        for (uint32_t e = 0; e < N / 128; ++e) z[tt][e] = tt < tn ? zr[(uint64_t)tt * N + threadIdx.x + 128 * e] : 0;
-    __shared__ uint64_t sh[4][ZV_TRIALS];
-    for (uint32_t k = k0; k < k1; ++k) {
+        for (uint32_t e = 0; e < N / 128; ++e)
+            z[tt][threadIdx.x + 128 * e] = tt < tn ? zr[(uint64_t)tt * N + threadIdx.x + 128 * e] : 0;
+    __syncthreads();
+    for (uint32_t k = k0 + warp; k < k1; k += 4) {
         const uint32_t i = lmi[g.lp0 + k];
-        const uint64_t* vr = v + (uint64_t)pairs[i].q * N;
-        uint64_t vv[N / 128];
+        const uint64_t* vr = v + (uint64_t)pairs[i].q * N + lane;
+        uint64_t lo[ZV_TRIALS] = {}, hi[ZV_TRIALS] = {};
+        for (uint32_t e0 = 0; e0 < N / 32; e0 += 8) {
+            uint64_t vv[8];
 #pragma unroll
-        for (uint32_t e = 0; e < N / 128; ++e) vv[e] = vr[threadIdx.x + 128 * e];
+            for (uint32_t e = 0; e < 8; ++e) vv[e] = vr[32 * (e0 + e)];
+#pragma unroll
+            for (uint32_t e = 0; e < 8; ++e)
+#pragma unroll
+                for (uint32_t tt = 0; tt < ZV_TRIALS; ++tt) mac128(lo[tt], hi[tt], z[tt][32 * (e0 + e) + lane], vv[e]);
+        }
 #pragma unroll
         for (uint32_t tt = 0; tt < ZV_TRIALS; ++tt) {
-            uint64_t lo = 0, hi = 0;
-#pragma unroll
-            for (uint32_t e = 0; e < N / 128; ++e) mac128(lo, hi, z[tt][e], vv[e]);
-            uint64_t x = reduce128(lo, hi);
+            uint64_t x = reduce128(lo[tt], hi[tt]);
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) x = add_mod(x, __shfl_xor_sync(0xffffffffu, x, off));
-            if (lane == 0) sh[warp][tt] = x;
+            if (lane == 0 && tt < tn) zv[(uint64_t)i * trials + t0 + tt] = x;
         }
-        __syncthreads();
-        if (threadIdx.x < tn)
-            zv[(uint64_t)i * trials + t0 + threadIdx.x] =
-                add_mod(add_mod(sh[0][threadIdx.x], sh[1][threadIdx.x]), add_mod(sh[2][threadIdx.x], sh[3][threadIdx.x]));
-        __syncthreads();  // sh is rewritten by the next pair
     }
 }
 
