@@ -392,10 +392,10 @@ tc_freivalds_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_con
 
 // ------------------------------------------------------------------ small panels
 // tc_freivalds_kernel for panels of at most TC_SMALL_RB row blocks (the short
-// inverted lists of an IVF batch, most of them a single 128-row block).  A
-// CTA takes whole panels: the panel's U tiles are loaded once into one of two
-// shared-memory regions (the next panel's load overlaps this one's MMAs) and
-// stay there while the panel's 64 strips of m_enc stream through the stage
+// inverted lists of an IVF batch).  A CTA takes a panel, or one of `split` equal
+// runs of its 64 strips: the panel's U tiles are loaded once into one of two
+// shared-memory regions (the next item's load overlaps this one's MMAs) and
+// stay there while the strips of m_enc stream through the stage
 // ring, one strip per item, into three rotating TMEM accumulators (3 x n_rows
 // <= 480 columns): the drain of a strip overlaps the MMAs of the next two.
 // Roles: warp 0 TMA, warp 1 MMA issuer, warps 2-21 drain (5 per lane
@@ -410,7 +410,7 @@ constexpr int SM_THREADS = 64 + 32 * SM_EPI_WARPS;
 
 __global__ void __launch_bounds__(SM_THREADS, 1)
 tc_freivalds_small_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_constant__ CUtensorMap tmap_u,
-                          const TcPanel* __restrict__ panels, uint32_t p_first, uint32_t npanels,
+                          const TcPanel* __restrict__ panels, uint32_t p_first, uint32_t npanels, uint32_t split,
                           uint32_t t_base, uint32_t t_cnt, uint32_t n_rows, uint32_t trials_total,
                           uint64_t* __restrict__ z_part, uint32_t* __restrict__ err, long long wait_limit) {
     extern __shared__ uint8_t tc_dyn[];
@@ -425,6 +425,7 @@ tc_freivalds_small_kernel(const __grid_constant__ CUtensorMap tmap_m, const __gr
     const uint32_t u_region = TC_SMALL_RB * u_tile;
     const uint32_t ring_off = 2 * u_region;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t items = npanels * split, run = 64 / split;  // strips per item
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < SM_STAGES; ++s) {
@@ -460,8 +461,8 @@ tc_freivalds_small_kernel(const __grid_constant__ CUtensorMap tmap_m, const __gr
             uint64_t it = 0;
             uint32_t pc = 0;
             bool stop = false;
-            for (uint32_t w = blockIdx.x; w < npanels && !stop; w += gridDim.x, ++pc) {
-                const TcPanel pn = panels[p_first + w];
+            for (uint32_t w = blockIdx.x; w < items && !stop; w += gridDim.x, ++pc) {
+                const TcPanel pn = panels[p_first + w / split];
                 const uint32_t nrb = min((pn.rows + TC_ROWS - 1) / TC_ROWS, TC_SMALL_RB);
                 const uint32_t ub = pc & 1;
                 // U region ub is free once the MMAs of panel pc - 2 have read it
@@ -474,7 +475,7 @@ tc_freivalds_small_kernel(const __grid_constant__ CUtensorMap tmap_m, const __gr
                 bar_expect_tx(&ufull_b[ub], nrb * u_tile);
                 for (uint32_t rb = 0; rb < nrb; ++rb)
                     tma_2d(sm + ub * u_region + rb * u_tile, &tmap_u, 0, (int)((pn.rb0 + rb) * n_rows), &ufull_b[ub]);
-                for (uint32_t s = 0; s < 64 && !stop; ++s)
+                for (uint32_t s = w % split * run, s1 = s + run; s < s1 && !stop; ++s)
                     for (uint32_t rb = 0; rb < nrb; ++rb, ++it) {
                         const uint32_t st = (uint32_t)(it % SM_STAGES);
                         if (it >= SM_STAGES && !bar_wait(&empty_b[st], (uint32_t)(((it / SM_STAGES) - 1) & 1), wait_limit)) {
@@ -502,8 +503,8 @@ tc_freivalds_small_kernel(const __grid_constant__ CUtensorMap tmap_m, const __gr
             uint64_t it = 0, sc = 0;
             uint32_t pc = 0;
             bool stop = false;
-            for (uint32_t w = blockIdx.x; w < npanels && !stop; w += gridDim.x, ++pc) {
-                const TcPanel pn = panels[p_first + w];
+            for (uint32_t w = blockIdx.x; w < items && !stop; w += gridDim.x, ++pc) {
+                const TcPanel pn = panels[p_first + w / split];
                 const uint32_t nrb = min((pn.rows + TC_ROWS - 1) / TC_ROWS, TC_SMALL_RB);
                 const uint32_t ub = pc & 1;
                 if (!bar_wait(&ufull_b[ub], (pc >> 1) & 1, wait_limit) || abort_s) {
@@ -512,7 +513,7 @@ tc_freivalds_small_kernel(const __grid_constant__ CUtensorMap tmap_m, const __gr
                     break;
                 }
                 tc_after();
-                for (uint32_t s = 0; s < 64 && !stop; ++s, ++sc) {
+                for (uint32_t s = 0; s < run && !stop; ++s, ++sc) {
                     const uint32_t b = (uint32_t)(sc % 3), use = (uint32_t)(sc / 3);
                     if (use > 0 && !bar_wait(&acce_b[b], (use - 1) & 1, wait_limit)) {
                         abort_s = 1;
@@ -556,10 +557,10 @@ tc_freivalds_small_kernel(const __grid_constant__ CUtensorMap tmap_m, const __gr
         const uint32_t tasks = (n_rows + 31) / 32;            // 32-column chunks (the last may be 16)
         uint64_t sc = 0;
         bool stop = false;
-        for (uint32_t w = blockIdx.x; w < npanels && !stop; w += gridDim.x) {
-            const uint32_t p = p_first + w;
+        for (uint32_t w = blockIdx.x; w < items && !stop; w += gridDim.x) {
+            const uint32_t p = p_first + w / split;
             uint64_t* z_out = z_part + ((uint64_t)p * trials_total + t_base) * N;
-            for (uint32_t s = 0; s < 64; ++s, ++sc) {
+            for (uint32_t s = w % split * run, s1 = s + run; s < s1; ++s, ++sc) {
                 const uint32_t b = (uint32_t)(sc % 3), use = (uint32_t)(sc / 3);
                 const bool ok = __all_sync(FULLMASK, bar_wait(&accf_b[b], use & 1, wait_limit));  // warp-uniform
                 if (!ok && lane == 0) { abort_s = 1; atomicOr(err, 16u); }
@@ -1066,9 +1067,23 @@ void launch_tc_freivalds_small(const CUtensorMap& tmap_m, const CUtensorMap& tma
     const long long wl = wait_cycles > 0 ? wait_cycles : TC_WAIT_CYCLES;
     const int smem = (int)(2 * TC_SMALL_RB * n_rows * TC_ROWS + SM_STAGES * STRIP_BYTES + 1024);
     cudaFuncSetAttribute(tc_freivalds_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    const unsigned grid = npanels < (uint32_t)num_sms ? npanels : (unsigned)num_sms;
-    tc_freivalds_small_kernel<<<grid, SM_THREADS, smem, s>>>(tmap_m, tmap_u, d_panels, p_first, npanels, t_base, t_cnt,
-                                                             n_rows, trials_total, d_z_part, d_err, wl);
+    // Strip runs per panel: the count whose rounds over the SMs are shortest, an
+    // item costing its strips and about three more to fill and empty the
+    // pipeline.  (Whole panels only: a batch with 67 short lists kept 67 SMs busy
+    // for 124 us.)
+    uint32_t split = 1;
+    uint64_t best = ~0ull;
+    for (uint32_t sp = 1; sp <= 8; sp *= 2) {
+        const uint64_t rounds = ((uint64_t)npanels * sp + num_sms - 1) / num_sms, cost = rounds * (64 / sp + 3);
+        if (cost < best) {
+            best = cost;
+            split = sp;
+        }
+    }
+    const uint32_t items = npanels * split;
+    const unsigned grid = items < (uint32_t)num_sms ? items : (unsigned)num_sms;
+    tc_freivalds_small_kernel<<<grid, SM_THREADS, smem, s>>>(tmap_m, tmap_u, d_panels, p_first, npanels, split, t_base,
+                                                             t_cnt, n_rows, trials_total, d_z_part, d_err, wl);
 }
 
 void launch_tc_fused(const CUtensorMap& tmap_m, const CUtensorMap& tmap_u, const CUtensorMap& tmap_w,
