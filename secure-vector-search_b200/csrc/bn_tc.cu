@@ -914,7 +914,10 @@ tc_rreduce_kernel(const VerifySeg* __restrict__ vsegs, const TcBlock* __restrict
 // and writes that share of z_t . v (z . v is linear in z, so the shares of
 // the splits add up); y == 8 sums every split-th row block's u_t . r
 // partial.  Splitting the panels over more CTAs keeps enough loads in flight
-// when a launch has few segments (one query: 245 panels at N = 1M).
+// when a launch has few segments (one query: 127 panels at N = 1M).  With many
+// segments (the lists of an IVF batch, a panel each) a CTA takes all 1024
+// columns of its trial: 128 segments were 23,040 CTAs of one load per thread,
+// 38 us.
 // The last CTA of a segment (a ticket taken after a device-scope fence, no
 // waiting) adds the shares up, a warp per trial, and keeps the first trial
 // whose sides differ (-1 if none).
@@ -926,18 +929,32 @@ tc_finish_kernel(const uint64_t* __restrict__ z_part, const uint64_t* __restrict
                  const uint64_t* __restrict__ v_enc, const VerifySeg* __restrict__ vsegs, uint32_t trials,
                  uint32_t split, uint64_t* chunks, uint32_t* __restrict__ done, uint64_t* __restrict__ ur,
                  uint64_t* __restrict__ zv, int32_t* __restrict__ failed) {
+    // split > 1: grid.y = 8 column chunks, then u . r; split == 1: one CTA takes
+    // all of z . v (grid.y 0), another u . r
     const uint32_t t = blockIdx.x, y = blockIdx.y, seg = blockIdx.z / split, sp = blockIdx.z % split;
+    const uint32_t z_ctas = split > 1 ? FIN_CHUNKS : 1;
     __shared__ uint64_t sh[4];
     __shared__ int32_t last_s, first;
     uint64_t part = 0;
-    if (y < FIN_CHUNKS) {
+    if (y < z_ctas) {
         const VerifySeg vs = vsegs[seg];
-        const uint32_t j = y * 128 + threadIdx.x;
         const uint32_t p0 = seg_panel0[seg], p1 = seg_panel0[seg + 1];
-        uint64_t z = 0;
+        const uint64_t* v = v_enc + (uint64_t)vs.query * N;
+        if (split > 1) {
+            const uint32_t j = y * 128 + threadIdx.x;
+            uint64_t z = 0;
 #pragma unroll 4
-        for (uint32_t p = p0 + sp; p < p1; p += split) z = add_mod(z, z_part[((uint64_t)p * trials + t) * N + j]);
-        part = mul_mod(z, v_enc[(uint64_t)vs.query * N + j]);
+            for (uint32_t p = p0 + sp; p < p1; p += split) z = add_mod(z, z_part[((uint64_t)p * trials + t) * N + j]);
+            part = mul_mod(z, v[j]);
+        } else {
+            uint64_t z[FIN_CHUNKS] = {};
+            for (uint32_t p = p0; p < p1; ++p)
+#pragma unroll
+                for (int c = 0; c < FIN_CHUNKS; ++c)
+                    z[c] = add_mod(z[c], z_part[((uint64_t)p * trials + t) * N + c * 128 + threadIdx.x]);
+#pragma unroll
+            for (int c = 0; c < FIN_CHUNKS; ++c) part = add_mod(part, mul_mod(z[c], v[c * 128 + threadIdx.x]));
+        }
     } else {
         const uint32_t b0 = seg_block0[seg], b1 = seg_block0[seg + 1];
         for (uint32_t b = b0 + sp + split * threadIdx.x; b < b1; b += split * blockDim.x)
@@ -948,7 +965,7 @@ tc_finish_kernel(const uint64_t* __restrict__ z_part, const uint64_t* __restrict
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0) sh[warp] = part;
     __syncthreads();
-    const uint32_t per = (FIN_CHUNKS + 1) * split;  // shares per trial; the last split of them are u . r
+    const uint32_t per = (z_ctas + 1) * split;  // shares per trial; the last split of them are u . r
     if (threadIdx.x == 0) {
         __stcg(chunks + ((uint64_t)seg * trials + t) * per + y * split + sp, add_mod(add_mod(sh[0], sh[1]), add_mod(sh[2], sh[3])));
         __threadfence();  // the share is visible device-wide before its ticket
@@ -963,7 +980,7 @@ tc_finish_kernel(const uint64_t* __restrict__ z_part, const uint64_t* __restrict
         uint64_t a = 0, b = 0;
         for (uint32_t i = lane; i < per; i += 32) {
             const uint64_t x = __ldcg(c + i);
-            if (i < FIN_CHUNKS * split) b = add_mod(b, x);
+            if (i < z_ctas * split) b = add_mod(b, x);
             else a = add_mod(a, x);
         }
 #pragma unroll
@@ -1122,7 +1139,7 @@ void launch_tc_finish(const uint64_t* d_z_part, const uint64_t* d_ur_part, const
     const uint32_t per_launch = 65535u / split;  // grid.z limit
     for (uint32_t s0 = 0; s0 < nseg; s0 += per_launch) {
         const uint32_t ns = nseg - s0 < per_launch ? nseg - s0 : per_launch;
-        tc_finish_kernel<<<dim3(trials, FIN_CHUNKS + 1, ns * split), 128, 0, s>>>(
+        tc_finish_kernel<<<dim3(trials, split > 1 ? FIN_CHUNKS + 1 : 2, ns * split), 128, 0, s>>>(
             d_z_part, d_ur_part, d_seg_panel0 + s0, d_seg_block0 + s0, d_v_enc, d_vsegs + s0, trials, split,
             d_chunks + (uint64_t)s0 * trials * (FIN_CHUNKS + 1) * split, d_done + s0, d_ur + (uint64_t)s0 * trials,
             d_zv + (uint64_t)s0 * trials, d_failed + s0);
