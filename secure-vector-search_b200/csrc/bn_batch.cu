@@ -8,7 +8,7 @@
 //   warp 1    MMA issuer: 4 x tcgen05.mma (M=128, N=w_tile, K=32) per stage
 //             into one of two TMEM accumulators (double-buffered across
 //             items), tcgen05.commit frees the stage / hands over the item
-//   warps 2-9 epilogue: tcgen05.ld, byte-weight recombination mod p, stores
+//   warps 2-17 epilogue: tcgen05.ld, byte-weight recombination mod p, stores
 // Every mbarrier wait is bounded; on timeout the CTA sets *err and winds down
 // (waits for its own copies and MMAs, frees TMEM) instead of hanging.
 #include <cudaTypedefs.h>
@@ -25,8 +25,24 @@ namespace {
 
 using namespace tcg;
 
-constexpr int BG_EPI_WARPS = 8;
+// Four epilogue warps per TMEM lane quarter: at K = 256 bytes an item's MMAs
+// take a fifth of its recombination, and two warps per scheduler left that
+// waiting on its own 64-bit chains.
+constexpr int BG_EPI_WARPS = 16;
+constexpr uint32_t BG_EPI_PARTS = BG_EPI_WARPS / 4;
 constexpr int BG_THREADS = 64 + 32 * BG_EPI_WARPS;  // TMA warp, MMA warp, epilogue warps
+
+// sum of v[b] 2^(8b), b < 8, times 2^w mod p (v: accumulators >= 0): below 2^61 + 8,
+// so 8 of them add up below 2^64.
+__device__ __forceinline__ uint64_t byte_part(const uint32_t* v, uint32_t w) {
+    uint64_t lo = 0, hi = 0;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        lo += (uint64_t)v[b] << (8 * b);
+        hi += (uint64_t)v[4 + b] << (8 * b);
+    }
+    return fold(rotl61(lo + rotl61(hi, 32), w));
+}
 
 // A work item: K panel, TMA rows of the A and W tiles, and the output range.
 struct ItemIdx {
@@ -37,52 +53,85 @@ __device__ __forceinline__ ItemIdx grid_item(const BgParams& p, uint32_t kp, uin
     const uint32_t x0 = p.mode == BG_S8 ? ta * BG_AROWS : ta * (BG_AROWS / 8);
     return ItemIdx{kp, tw, p.a_blocked ? ta : ta * BG_AROWS, tw * p.w_tile, x0, p.x_count, tw * p.w_tile / 8, p.y_count};
 }
-__device__ __forceinline__ ItemIdx item_idx(const BgParams& p, uint32_t item) {
-    const uint32_t per = p.a_tiles * p.w_tiles;
-    const uint32_t kp = item / per, rem = item % per;
-    if (p.order_a_fast) return grid_item(p, kp, rem % p.a_tiles, rem / p.a_tiles);
-    return grid_item(p, kp, rem / p.w_tiles, rem % p.w_tiles);
-}
-
-// The j-th work item of this CTA.  Streaming mode: global items blockIdx.x +
-// j * gridDim.x.  A-resident mode: this CTA owns A tiles blockIdx.x + t *
-// gridDim.x and visits every W tile of each (j = t * w_tiles + tw).
-__device__ __forceinline__ bool item_at(const BgParams& p, uint32_t items, uint32_t j, ItemIdx& ix) {
-    if (p.item_tab) {
-        const uint32_t item = blockIdx.x + j * gridDim.x;
-        if (item >= p.n_items) return false;
-        const BgItem t = p.item_tab[item];
-        ix = ItemIdx{0, 1, t.a_y, t.w_y, t.x0, t.x_lim, t.y0, t.y_lim};
-        return true;
-    }
-    if (p.a_resident) {
-        const uint32_t ta = blockIdx.x + (j / p.w_tiles) * gridDim.x;
-        if (ta >= p.a_tiles) return false;
-        ix = grid_item(p, 0, ta, j % p.w_tiles);
-        return true;
-    }
-    const uint32_t item = blockIdx.x + j * gridDim.x;
-    if (item >= items) return false;
-    ix = item_idx(p, item);
-    return true;
-}
-
-// This CTA's items in order, the next item's entry fetched one item ahead (in
-// grouped mode an item-table load, whose latency then overlaps the current item).
+// This CTA's work items in order.  Streaming mode: global items blockIdx.x + j *
+// gridDim.x of the (K panel, A tile, W tile) grid, W tile or A tile fastest;
+// the step is taken as a carry through the three indices, no division per item.
+// A-resident mode: A tiles blockIdx.x + t * gridDim.x, every W tile of each.
+// Grouped mode: entries of the item table, the next one fetched one item ahead
+// (its load then overlaps the current item).
 struct ItemCursor {
     const BgParams& p;
-    uint32_t items, j = 0;
-    ItemIdx cur, nxt;
-    bool have_cur, have_nxt;
-    __device__ __forceinline__ ItemCursor(const BgParams& p_, uint32_t items_) : p(p_), items(items_) {
-        have_cur = item_at(p, items, 0, cur);
-        have_nxt = have_cur && item_at(p, items, 1, nxt);
+    uint32_t kpanels, j = 0;
+    uint32_t kp = 0, ta = 0, tw = 0;  // streaming and A-resident
+    uint32_t s_fast = 0, s_slow = 0;  // gridDim.x in units of the fastest index and the next
+    ItemIdx cur;
+    BgItem nxt;
+    bool have_cur, have_nxt = false;
+    __device__ __forceinline__ ItemCursor(const BgParams& p_, uint32_t kpanels_) : p(p_), kpanels(kpanels_) {
+        if (p.item_tab) {
+            have_cur = blockIdx.x < p.n_items;
+            if (have_cur) from_table(p.item_tab[blockIdx.x]);
+            fetch();
+            return;
+        }
+        if (p.a_resident) {
+            ta = blockIdx.x;
+            have_cur = ta < p.a_tiles;
+        } else {
+            const uint32_t nf = p.order_a_fast ? p.a_tiles : p.w_tiles, ns = p.order_a_fast ? p.w_tiles : p.a_tiles;
+            s_fast = gridDim.x % nf;
+            s_slow = gridDim.x / nf;
+            const uint32_t fast = blockIdx.x % nf;
+            uint32_t slow = blockIdx.x / nf;
+            kp = slow / ns;
+            slow %= ns;
+            ta = p.order_a_fast ? fast : slow;
+            tw = p.order_a_fast ? slow : fast;
+            have_cur = kp < kpanels;
+        }
+        if (have_cur) cur = grid_item(p, kp, ta, tw);
+    }
+    __device__ __forceinline__ void from_table(const BgItem& t) {
+        cur = ItemIdx{0, 1, t.a_y, t.w_y, t.x0, t.x_lim, t.y0, t.y_lim};
+    }
+    __device__ __forceinline__ void fetch() {
+        const uint32_t item = blockIdx.x + (j + 1) * gridDim.x;
+        have_nxt = item < p.n_items;
+        if (have_nxt) nxt = p.item_tab[item];
     }
     __device__ __forceinline__ void advance() {
         ++j;
-        cur = nxt;
-        have_cur = have_nxt;
-        if (have_cur) have_nxt = item_at(p, items, j + 1, nxt);
+        if (p.item_tab) {
+            have_cur = have_nxt;
+            if (have_cur) {
+                from_table(nxt);
+                fetch();
+            }
+            return;
+        }
+        if (p.a_resident) {
+            if (++tw == p.w_tiles) {
+                tw = 0;
+                ta += gridDim.x;
+            }
+            have_cur = ta < p.a_tiles;
+        } else {
+            uint32_t& fast = p.order_a_fast ? ta : tw;
+            uint32_t& slow = p.order_a_fast ? tw : ta;
+            const uint32_t nf = p.order_a_fast ? p.a_tiles : p.w_tiles, ns = p.order_a_fast ? p.w_tiles : p.a_tiles;
+            fast += s_fast;
+            slow += s_slow;
+            if (fast >= nf) {
+                fast -= nf;
+                ++slow;
+            }
+            while (slow >= ns) {
+                slow -= ns;
+                ++kp;
+            }
+            have_cur = kp < kpanels;
+        }
+        if (have_cur) cur = grid_item(p, kp, ta, tw);
     }
 };
 
@@ -105,13 +154,16 @@ bgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     const uint32_t w_bytes = p.w_tile * BG_KSTEP;
     const uint32_t ksub = p.ksteps2 ? 2u : 1u, kstage = ksub * BG_KSTEP;  // K steps / bytes per stage
     const uint32_t kpanels = (p.k_bytes + p.k_panel - 1) / p.k_panel;
-    const uint32_t items = p.item_tab ? p.n_items : kpanels * p.a_tiles * p.w_tiles;
     const uint32_t a_slots = p.a_resident ? p.k_bytes / BG_KSTEP : 0;
     const uint32_t base = sbase + a_slots * A_BYTES;  // stage ring
     uint8_t* ring = sptr + a_slots * A_BYTES;
     // TMA coordinates of A's K step at byte k: row-major (x = k, y = row), or
     // K-blocked (x = 0, y = (tile * K steps + k / 128) * 128)
     const uint32_t a_ksteps = p.k_bytes / BG_KSTEP;
+    // at most two 32-column chunks per item: half the epilogue warps take the
+    // items of one TMEM buffer, half those of the other, so two items are
+    // recombined at a time (8 queries: see the figures at BG_EPI_WARPS)
+    const bool narrow = p.w_tile <= 64;
     auto a_x = [&](uint32_t k) -> int { return p.a_blocked ? 0 : (int)k; };
     auto a_row = [&](const ItemIdx& ix, uint32_t k) -> int {
         return p.a_blocked ? (int)((ix.a_y * a_ksteps + k / BG_KSTEP) * BG_AROWS) : (int)ix.a_y;
@@ -124,7 +176,7 @@ bgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         }
         for (int b = 0; b < 2; ++b) {
             bar_init(&accf_b[b], 1);
-            bar_init(&acce_b[b], BG_EPI_WARPS);
+            bar_init(&acce_b[b], narrow ? BG_EPI_WARPS / 2 : BG_EPI_WARPS);
         }
         for (uint32_t k = 0; k < a_slots; ++k) {
             bar_init(&afull_b[k], 1);
@@ -155,7 +207,7 @@ bgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
             // A loads issued last: slots [0, a_n) for tile a_t, the rest for a_t - 1
             uint32_t a_t = 0xffffffffu, a_n = 0;
             bool stop = false;
-            for (ItemCursor cs(p, items); !stop && cs.have_cur; cs.advance()) {
+            for (ItemCursor cs(p, kpanels); !stop && cs.have_cur; cs.advance()) {
                 const ItemIdx& ix = cs.cur;
                 const uint32_t j = cs.j;
                 const uint32_t t = a_slots ? j / p.w_tiles : 0;
@@ -221,7 +273,7 @@ bgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
                                    ((uint32_t)(BG_AROWS >> 4) << 24);
             uint64_t it = 0;
             bool stop = false;
-            for (ItemCursor cs(p, items); !stop && cs.have_cur; cs.advance()) {
+            for (ItemCursor cs(p, kpanels); !stop && cs.have_cur; cs.advance()) {
                 const ItemIdx& ix = cs.cur;
                 const uint32_t j = cs.j;
                 const uint64_t n = j;
@@ -271,75 +323,69 @@ bgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         }
     } else {
         // -------------------------------------------------------------- epilogue
-        // 8 warps: warp w reads TMEM lane quarter w % 4 and every other
-        // 64-column chunk (half = (w - 2) / 4) of each item.
+        // 16 warps: warp w reads TMEM lane quarter w % 4 and every fourth
+        // 32-column chunk (part = (w - 2) / 4) of each item; a last 16-column
+        // chunk, when w_tile is not a multiple of 32, counts as one more.
         const uint32_t q = (uint32_t)(warp & 3);
-        const uint32_t half = (uint32_t)(warp - 2) >> 2;
-        const uint32_t wide = p.w_tile & ~63u;  // columns handled in 64-column chunks
-        for (ItemCursor cs(p, items); cs.have_cur; cs.advance()) {
+        const uint32_t parts = narrow ? BG_EPI_PARTS / 2 : BG_EPI_PARTS;
+        const uint32_t part = ((uint32_t)(warp - 2) >> 2) % parts, group = ((uint32_t)(warp - 2) >> 2) / parts;
+        const uint32_t wide = p.w_tile & ~31u;  // columns handled in 32-column chunks
+        for (ItemCursor cs(p, kpanels); cs.have_cur; cs.advance()) {
             const ItemIdx& ix = cs.cur;
             const uint64_t n = cs.j;
             const uint32_t buf = (uint32_t)(n & 1), use = (uint32_t)(n >> 1);
+            if (narrow && buf != group) continue;  // the other half's item
             // output bases of the y this lane stores, loaded before the wait:
-            // PLANAR lane (xi, a) stores y = chunk + a (wide chunks) and
-            // chunk + {0, 1} (16-column chunks); S8 lanes share every y, so
-            // lane l holds chunk + (l & 7) and the stores shuffle it out
+            // PLANAR lane (xi, a) stores y = chunk + a / 2 (wide chunks) and
+            // chunk + {0, 1} (the 16-column chunk); S8 lanes share every y, so
+            // lane l holds chunk + (l & 3) and the stores shuffle it out
             const uint32_t ybase = ix.y0;
             auto obase = [&](uint32_t y) -> uint64_t {
                 return y < ix.y_lim ? (p.pair_base ? p.pair_base[y] : (uint64_t)y * p.out_ld) : 0;
             };
-            const uint32_t ysel = lane & 7;  // PLANAR: a; S8: the y this lane holds for the shuffles
-            uint64_t ob_w[2], ob_r[2][2];
+            const uint32_t ysel = p.mode == BG_PLANAR ? (lane & 7) >> 1 : lane & 3;
+            uint64_t ob_w[2], ob_r[2];
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                const uint32_t cw = 64 * half + 128 * k, cr = wide + 16 * half + 32 * k;
+                const uint32_t cw = 32 * (part + parts * k);
                 ob_w[k] = cw < wide ? obase(ybase + cw / 8 + ysel) : 0;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) ob_r[k][h] = cr < p.w_tile ? obase(ybase + cr / 8 + h) : 0;
+                ob_r[k] = wide < p.w_tile ? obase(ybase + wide / 8 + k) : 0;
             }
             const bool ok = __all_sync(FULLMASK, bar_wait(&accf_b[buf], use & 1, wait_limit));  // warp-uniform
             if (!ok && lane == 0) { abort_s = 1; atomicOr(err, 16u); }
             if (__any_sync(FULLMASK, !ok || abort_s)) break;
             tc_after();
             const uint32_t taddr = tmem + ((q * 32u) << 16) + buf * 256u;
+            const bool mine_r = wide < p.w_tile && (wide / 32) % parts == part;  // the 16-column chunk
             if (p.mode == BG_PLANAR) {
                 const uint32_t a = lane & 7, xi = lane >> 3;
                 const uint32_t x4 = ix.x0 + q * 4;  // first x of this warp
                 const uint32_t x = x4 + xi;
                 const uint32_t w1 = 8 * a;
+                const bool b2 = (a & 4) != 0, b1 = (a & 2) != 0;
                 uint64_t* out = p.out + (uint64_t)ix.kp * p.out_pstride;
-                for (uint32_t c0 = 64 * half, k = 0; c0 < wide; c0 += 128, ++k) {
-                    uint32_t v[64];
-                    tmem_ld64(taddr + c0, v);
-                    uint64_t part[8];  // (lo + hi 2^32) 2^(8a) mod p for the chunk's 8 y
+                for (uint32_t c0 = 32 * part, k = 0; c0 < wide; c0 += 32 * parts, ++k) {
+                    uint32_t v[32];
+                    tmem_ld32(taddr + c0, v);
+                    uint64_t pt[4];  // the byte products times 2^(8a) mod p for the chunk's 4 y
 #pragma unroll
-                    for (int yy = 0; yy < 8; ++yy) {
-                        uint64_t lo = 0, hi = 0;
-#pragma unroll
-                        for (int b = 0; b < 4; ++b) {
-                            lo += (uint64_t)v[8 * yy + b] << (8 * b);
-                            hi += (uint64_t)v[8 * yy + 4 + b] << (8 * b);
-                        }
-                        part[yy] = fold(rotl61(lo + rotl61(hi, 32), w1));  // < 2^61 + 8: 8 sum below 2^64
-                    }
-                    // butterfly over the 8 lanes of one x: each level halves the
-                    // y values a lane carries; lane a ends with y = a
-                    const bool b2 = (a & 4) != 0, b1 = (a & 2) != 0, b0 = (a & 1) != 0;
-                    uint64_t k4[4], k2[2];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        k4[i] = (b2 ? part[i + 4] : part[i]) + __shfl_xor_sync(FULLMASK, b2 ? part[i] : part[i + 4], 4);
+                    for (int yy = 0; yy < 4; ++yy) pt[yy] = byte_part(v + 8 * yy, w1);
+                    // butterfly over the 8 lanes of one x: two levels halve the
+                    // y values a lane carries, the third adds the pair up; lanes
+                    // a and a ^ 1 end with y = a / 2
+                    uint64_t k2[2];
 #pragma unroll
                     for (int i = 0; i < 2; ++i)
-                        k2[i] = (b1 ? k4[i + 2] : k4[i]) + __shfl_xor_sync(FULLMASK, b1 ? k4[i] : k4[i + 2], 2);
-                    const uint64_t f =
-                        canon((b0 ? k2[1] : k2[0]) + __shfl_xor_sync(FULLMASK, b0 ? k2[0] : k2[1], 1));  // < 8p
-                    const uint32_t y = ybase + c0 / 8 + a;
-                    if (y < ix.y_lim && x < ix.x_lim) out[(k ? ob_w[1] : ob_w[0]) + x] = f;
+                        k2[i] = (b2 ? pt[i + 2] : pt[i]) + __shfl_xor_sync(FULLMASK, b2 ? pt[i] : pt[i + 2], 4);
+                    uint64_t f = (b1 ? k2[1] : k2[0]) + __shfl_xor_sync(FULLMASK, b1 ? k2[0] : k2[1], 2);
+                    f = canon(f + __shfl_xor_sync(FULLMASK, f, 1));  // < 8p
+                    const uint32_t y = ybase + c0 / 8 + (a >> 1);
+                    if ((a & 1) == 0 && y < ix.y_lim && x < ix.x_lim) out[(k ? ob_w[1] : ob_w[0]) + x] = f;
                     if (p.planar_out) {
                         // 4 x 8 byte transpose across the lanes of one y: lane
                         // (xi, a) ends with planes 4(xi&1) + 2(xi>>1) + {0, 1}
-                        // of f(x4..x4+3, y) as two 32-bit words
+                        // of f(x4..x4+3, y) as two 32-bit words, of which the
+                        // lane pair (a, a ^ 1) stores one each
                         const bool e0 = (xi & 1) != 0, e1 = (xi & 2) != 0;
                         const uint32_t flo = (uint32_t)f, fhi = (uint32_t)(f >> 32);
                         const uint32_t keep1 = e0 ? fhi : flo;
@@ -350,28 +396,19 @@ bgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
                         const uint32_t recv2 = __shfl_xor_sync(FULLMASK, e1 ? pa : pb, 16);
                         const uint32_t p0 = e1 ? recv2 : keep2, p1 = e1 ? keep2 : recv2;
                         if (y < ix.y_lim && x4 < ix.x_lim) {
-                            const uint32_t plane = 4 * (xi & 1) + 2 * (xi >> 1);
-                            uint8_t* dst = p.planar_out + ((uint64_t)y * 8 + plane) * p.planar_ld + x4;
-                            *reinterpret_cast<uint32_t*>(dst) = __byte_perm(p0, p1, 0x5410);
-                            *reinterpret_cast<uint32_t*>(dst + p.planar_ld) = __byte_perm(p0, p1, 0x7632);
+                            const uint32_t plane = 4 * (xi & 1) + 2 * (xi >> 1) + (a & 1);
+                            *reinterpret_cast<uint32_t*>(p.planar_out + ((uint64_t)y * 8 + plane) * p.planar_ld + x4) =
+                                __byte_perm(p0, p1, (a & 1) ? 0x7632 : 0x5410);
                         }
                     }
                 }
-                // remaining columns (w_tile not a multiple of 64): 16 at a time
-                for (uint32_t c0 = wide + 16 * half, k = 0; c0 < p.w_tile; c0 += 32, ++k) {
+                if (mine_r) {
                     uint32_t v[16];
-                    tmem_ld16(taddr + c0, v);
+                    tmem_ld16(taddr + wide, v);
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const uint32_t y = ybase + c0 / 8 + h;
-                        const uint64_t ob = k ? ob_r[1][h] : ob_r[0][h];
-                        uint64_t lo = 0, hi = 0;
-#pragma unroll
-                        for (int b = 0; b < 4; ++b) {
-                            lo += (uint64_t)v[8 * h + b] << (8 * b);
-                            hi += (uint64_t)v[8 * h + 4 + b] << (8 * b);
-                        }
-                        uint64_t f = fold(rotl61(lo + rotl61(hi, 32), w1));
+                        const uint32_t y = ybase + wide / 8 + h;
+                        uint64_t f = byte_part(v + 8 * h, w1);
                         f += __shfl_xor_sync(FULLMASK, f, 1);
                         f += __shfl_xor_sync(FULLMASK, f, 2);
                         f += __shfl_xor_sync(FULLMASK, f, 4);
@@ -380,7 +417,7 @@ bgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
                         packed |= __shfl_xor_sync(FULLMASK, packed, 8);
                         packed |= __shfl_xor_sync(FULLMASK, packed, 16);
                         if (y < ix.y_lim) {
-                            if (a == 0 && x < ix.x_lim) out[ob + x] = f;
+                            if (a == 0 && x < ix.x_lim) out[ob_r[h] + x] = f;
                             if (p.planar_out && lane < 8 && x4 < ix.x_lim)
                                 *reinterpret_cast<uint32_t*>(p.planar_out + ((uint64_t)y * 8 + lane) * p.planar_ld +
                                                              x4) = packed;
@@ -391,42 +428,30 @@ bgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
                 const uint32_t x = ix.x0 + q * 32 + lane;
                 const bool xv = x < ix.x_lim;
                 const uint64_t corr = xv ? p.corr[x] : 0;
-                for (uint32_t c0 = 64 * half, k = 0; c0 < wide; c0 += 128, ++k) {
-                    uint32_t v[64];
-                    tmem_ld64(taddr + c0, v);
+                auto store = [&](const uint32_t* v, uint32_t y, uint64_t ob) {
+                    int64_t lo = 0, hi = 0;
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        lo += (int64_t)(int32_t)v[b] * (int64_t)(1ll << (8 * b));
+                        hi += (int64_t)(int32_t)v[4 + b] * (int64_t)(1ll << (8 * b));
+                    }
+                    const uint64_t lr = lo < 0 ? (uint64_t)(lo + (int64_t)P) : (uint64_t)lo;
+                    const uint64_t hr = hi < 0 ? (uint64_t)(hi + (int64_t)P) : (uint64_t)hi;
+                    if (xv && y < ix.y_lim) p.out[ob + x] = add_mod(canon(lr + rotl61(hr, 32)), corr);
+                };
+                for (uint32_t c0 = 32 * part, k = 0; c0 < wide; c0 += 32 * parts, ++k) {
+                    uint32_t v[32];
+                    tmem_ld32(taddr + c0, v);
                     const uint64_t obk = k ? ob_w[1] : ob_w[0];
 #pragma unroll
-                    for (int yy = 0; yy < 8; ++yy) {
-                        const uint64_t ob = __shfl_sync(FULLMASK, obk, yy);
-                        int64_t lo = 0, hi = 0;
-#pragma unroll
-                        for (int b = 0; b < 4; ++b) {
-                            lo += (int64_t)(int32_t)v[8 * yy + b] * (int64_t)(1ll << (8 * b));
-                            hi += (int64_t)(int32_t)v[8 * yy + 4 + b] * (int64_t)(1ll << (8 * b));
-                        }
-                        const uint64_t lr = lo < 0 ? (uint64_t)(lo + (int64_t)P) : (uint64_t)lo;
-                        const uint64_t hr = hi < 0 ? (uint64_t)(hi + (int64_t)P) : (uint64_t)hi;
-                        const uint32_t y = ybase + c0 / 8 + yy;
-                        if (xv && y < ix.y_lim) p.out[ob + x] = add_mod(canon(lr + rotl61(hr, 32)), corr);
-                    }
+                    for (int yy = 0; yy < 4; ++yy)
+                        store(v + 8 * yy, ybase + c0 / 8 + yy, __shfl_sync(FULLMASK, obk, yy));
                 }
-                for (uint32_t c0 = wide + 16 * half, k = 0; c0 < p.w_tile; c0 += 32, ++k) {
+                if (mine_r) {
                     uint32_t v[16];
-                    tmem_ld16(taddr + c0, v);
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const uint64_t ob = k ? ob_r[1][h] : ob_r[0][h];
-                        int64_t lo = 0, hi = 0;
-#pragma unroll
-                        for (int b = 0; b < 4; ++b) {
-                            lo += (int64_t)(int32_t)v[8 * h + b] * (int64_t)(1ll << (8 * b));
-                            hi += (int64_t)(int32_t)v[8 * h + 4 + b] * (int64_t)(1ll << (8 * b));
-                        }
-                        const uint64_t lr = lo < 0 ? (uint64_t)(lo + (int64_t)P) : (uint64_t)lo;
-                        const uint64_t hr = hi < 0 ? (uint64_t)(hi + (int64_t)P) : (uint64_t)hi;
-                        const uint32_t y = ybase + c0 / 8 + h;
-                        if (xv && y < ix.y_lim) p.out[ob + x] = add_mod(canon(lr + rotl61(hr, 32)), corr);
-                    }
+                    tmem_ld16(taddr + wide, v);
+                    store(v, ybase + wide / 8, ob_r[0]);
+                    store(v + 8, ybase + wide / 8 + 1, ob_r[1]);
                 }
             }
             tc_before();
