@@ -577,44 +577,71 @@ __global__ void ms8_s_kernel(const uint16_t* __restrict__ s_ell, const uint32_t*
     }
 }
 
-__global__ void w_tv_kernel(const uint64_t* __restrict__ v, uint32_t nq, int8_t* __restrict__ dst) {
-    const uint32_t chunks = N / 16;
-    const uint64_t total = (uint64_t)nq * 8 * chunks;
-    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t qb = e / chunks;
-        const uint32_t jc = (uint32_t)(e % chunks);
-        const uint32_t q = (uint32_t)(qb >> 3), b = (uint32_t)(qb & 7);
-        int8_t* row = dst + qb * (2 * N);
-        reinterpret_cast<uint4*>(row)[jc] = make_uint4(0, 0, 0, 0);  // T part (b = 0 filled below)
-        uint32_t w[4] = {0, 0, 0, 0};
+// All three W operand images of one query, a CTA each: byte planes of v, of
+// -[g | x], and [T | bytes(v) - 128].  T's column sums of +-1 entries are counted
+// in shared memory (repeated columns add up).
+constexpr uint32_t WI_THREADS = 128;
+
+__device__ __forceinline__ void planes16(const uint64_t (&x)[16], int a, uint32_t (&w)[4]) {
+    w[0] = w[1] = w[2] = w[3] = 0;
 #pragma unroll
-        for (int t = 0; t < 16; ++t) {
-            const int byte = (int)((v[(uint64_t)q * N + jc * 16 + t] >> (8 * b)) & 0xffu) - 128;
-            w[t >> 2] |= (uint32_t)((uint8_t)(int8_t)byte) << (8 * (t & 3));
-        }
-        reinterpret_cast<uint4*>(row + N)[jc] = make_uint4(w[0], w[1], w[2], w[3]);
-    }
+    for (int t = 0; t < 16; ++t) w[t >> 2] |= (uint32_t)((x[t] >> (8 * a)) & 0xffu) << (8 * (t & 3));
 }
 
-// T part of row (q, b = 0): column sums of query q's +-1 entries, one CTA per
-// query (shared-memory counters, so repeated columns add up).
-__global__ void __launch_bounds__(256) w_t_kernel(const uint32_t* __restrict__ t_ent, const uint32_t* __restrict__ t_nnz,
-                                                  int8_t* __restrict__ dst, uint32_t* __restrict__ bad) {
-    const uint32_t q = blockIdx.x;
+__global__ void __launch_bounds__(WI_THREADS)
+w_images_kernel(const uint64_t* __restrict__ v, const uint64_t* __restrict__ g, const uint64_t* __restrict__ x,
+                const uint32_t* __restrict__ t_ent, const uint32_t* __restrict__ t_nnz, const uint32_t* __restrict__ map,
+                uint32_t n1, uint8_t* __restrict__ wv, uint8_t* __restrict__ wgx, uint8_t* __restrict__ wtv,
+                uint32_t* __restrict__ bad) {
+    const uint32_t q = map ? map[blockIdx.x] : blockIdx.x;
+    const uint64_t row0 = (uint64_t)blockIdx.x * 8;
     __shared__ int acc[N];
-    for (uint32_t i = threadIdx.x; i < N; i += blockDim.x) acc[i] = 0;
+    for (uint32_t i = threadIdx.x; i < N; i += WI_THREADS) acc[i] = 0;
     __syncthreads();
     const uint32_t tn = min(t_nnz[q], (uint32_t)N);
-    for (uint32_t c = threadIdx.x; c < tn; c += blockDim.x) {
+    for (uint32_t c = threadIdx.x; c < tn; c += WI_THREADS) {
         const uint32_t e = t_ent[(uint64_t)q * N + c];
         atomicAdd(&acc[e & 0x3ffu], (e >> 31) ? -1 : 1);
     }
+    // threads 0..63: 16 elements of v each; 64..127: 16 of [g | x] (2 n1 <= 1024)
+    const uint32_t jc = threadIdx.x & 63;
+    const bool of_v = threadIdx.x < 64;
+    if (of_v || jc < 2 * n1 / 16) {
+        const uint64_t* src = of_v ? v + (uint64_t)q * N + jc * 16
+                                   : jc * 16 < n1 ? g + (uint64_t)q * n1 + jc * 16 : x + (uint64_t)q * n1 + jc * 16 - n1;
+        uint64_t e[16];
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+            const uint64_t y = src[t];
+            e[t] = of_v || y == 0 ? y : P - y;
+        }
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+            uint32_t w[4];
+            planes16(e, a, w);
+            if (of_v) {
+                reinterpret_cast<uint4*>(wv + (row0 + a) * N)[jc] = make_uint4(w[0], w[1], w[2], w[3]);
+                reinterpret_cast<uint4*>(wtv + (row0 + a) * (2 * N) + N)[jc] =  // byte - 128
+                    make_uint4(w[0] ^ 0x80808080u, w[1] ^ 0x80808080u, w[2] ^ 0x80808080u, w[3] ^ 0x80808080u);
+            } else {
+                reinterpret_cast<uint4*>(wgx + (row0 + a) * (2 * n1))[jc] = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+        }
+    }
     __syncthreads();
-    int8_t* row = dst + (uint64_t)q * 8 * (2 * N);  // row (q, b = 0)
-    for (uint32_t i = threadIdx.x; i < N; i += blockDim.x) {
-        const int v = acc[i];
-        if (v < -128 || v > 127) atomicOr(bad, 2u);
-        row[i] = (int8_t)v;
+    for (uint32_t c = threadIdx.x; c < 8 * (N / 16); c += WI_THREADS) {  // T part: row b = 0 holds T, the others 0
+        uint32_t w[4] = {0, 0, 0, 0};
+        if (c < N / 16) {
+            bool out_of_range = false;
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                const int y = acc[c * 16 + t];
+                out_of_range |= y < -128 || y > 127;
+                w[t >> 2] |= (uint32_t)((uint8_t)(int8_t)y) << (8 * (t & 3));
+            }
+            if (out_of_range) atomicOr(bad, 2u);
+        }
+        reinterpret_cast<uint4*>(wtv + (row0 + c / (N / 16)) * (2 * N))[c % (N / 16)] = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
@@ -732,11 +759,11 @@ void launch_ms8(const uint64_t* d_mp_cm, const uint16_t* d_s_ell, const uint32_t
                                                                d_prow);
 }
 
-void launch_w_tv(const uint64_t* d_v, const uint32_t* d_t, const uint32_t* d_t_nnz, uint32_t nq, int8_t* d_dst,
-                 uint32_t* d_bad, cudaStream_t s) {
-    if (!nq) return;
-    w_tv_kernel<<<grid_for((uint64_t)nq * 8 * (N / 16), 256, 148 * 8), 256, 0, s>>>(d_v, nq, d_dst);
-    w_t_kernel<<<nq, 256, 0, s>>>(d_t, d_t_nnz, d_dst, d_bad);
+void launch_w_images(const uint64_t* d_v, const uint64_t* d_g, const uint64_t* d_x, const uint32_t* d_t,
+                     const uint32_t* d_t_nnz, const uint32_t* d_map, uint32_t count, uint32_t n1, uint8_t* d_wv,
+                     uint8_t* d_wgx, uint8_t* d_wtv, uint32_t* d_bad, cudaStream_t s) {
+    if (!count) return;
+    w_images_kernel<<<count, WI_THREADS, 0, s>>>(d_v, d_g, d_x, d_t, d_t_nnz, d_map, n1, d_wv, d_wgx, d_wtv, d_bad);
 }
 
 void launch_zsum(const uint64_t* d_z_part, uint32_t npanels, uint32_t t_base, uint32_t t_cnt, uint32_t trials_total,

@@ -110,12 +110,14 @@ void launch_planar_cm(const uint64_t* d_src_cm, uint64_t rows, uint32_t k, uint8
 void launch_ms8(const uint64_t* d_mp_cm, const uint16_t* d_s_ell, const uint32_t* d_s_off, const uint16_t* d_s_w,
                 uint64_t rows, int8_t* d_dst, uint64_t* d_corr, uint32_t* d_bad, cudaStream_t s,
                 const uint32_t* d_prow = nullptr);
-// W operand of the signed decode GEMM for nq queries: rows (q, b) of 2n
-// bytes: [T_q if b == 0 else 0 | byte b of v_q - 128].  T entries as in
-// DecodeQuery (col | 0x80000000 for -1); *bad |= 2 when a column sum leaves
-// [-128, 127].
-void launch_w_tv(const uint64_t* d_v, const uint32_t* d_t, const uint32_t* d_t_nnz, uint32_t nq, int8_t* d_dst,
-                 uint32_t* d_bad, cudaStream_t s);
+// The W operands of the three scoring GEMMs for `count` images of 8 rows, image
+// i of query d_map[i] (or i): d_wv rows (i, b) of n bytes, byte b of v; d_wgx of
+// 2 n1 bytes, byte b of p - [g | x]; d_wtv of 2n bytes, [T if b == 0 else 0 | byte
+// b of v - 128].  T entries as in DecodeQuery (col | 0x80000000 for -1); *bad |= 2
+// when a column sum leaves [-128, 127].
+void launch_w_images(const uint64_t* d_v, const uint64_t* d_g, const uint64_t* d_x, const uint32_t* d_t,
+                     const uint32_t* d_t_nnz, const uint32_t* d_map, uint32_t count, uint32_t n1, uint8_t* d_wv,
+                     uint8_t* d_wgx, uint8_t* d_wtv, uint32_t* d_bad, cudaStream_t s);
 // z_t = sum over panels of z_part[panel][t_base + t][j] -> z[t_base + t][j].
 void launch_zsum(const uint64_t* d_z_part, uint32_t npanels, uint32_t t_base, uint32_t t_cnt, uint32_t trials_total,
                  uint64_t* d_z, cudaStream_t s);

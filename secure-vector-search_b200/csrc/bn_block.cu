@@ -527,17 +527,14 @@ int block_enqueue(BlockPlan& b, const uint64_t* d_v, const uint64_t* d_g, const 
     CU(cudaMemsetAsync(err, 0, 8, s));  // pipeline + operand flags
     uint8_t* vp = reinterpret_cast<uint8_t*>(d + b.o_vp);
     uint8_t* gx = reinterpret_cast<uint8_t*>(d + b.o_gx);
-    int8_t* tv = reinterpret_cast<int8_t*>(d + b.o_tv);
+    uint8_t* tv = reinterpret_cast<uint8_t*>(d + b.o_tv);
     uint64_t* x = reinterpret_cast<uint64_t*>(d + b.o_x);
     uint64_t* r = reinterpret_cast<uint64_t*>(d + b.o_r);
     uint8_t* rp = reinterpret_cast<uint8_t*>(d + b.o_rp);
     if (b.k == 0 && !d_ids) d_ids = reinterpret_cast<uint32_t*>(d + b.o_out_ids);  // unused when k = 0
     // operands of this block
-    launch_planar_rows(d_v, b.B, N, N, 0, vp, N, 0, s);
     launch_lt_times_v(c.L.at<uint64_t>(), c.n1, d_v, b.B, x, s);
-    launch_planar_rows(d_g, b.B, c.n1, c.n1, 1, gx, c.k_alh, 0, s);
-    launch_planar_rows(x, b.B, c.n1, c.n1, 1, gx, c.k_alh, c.n1, s);
-    launch_w_tv(d_v, d_t, d_tn, b.B, tv, reinterpret_cast<uint32_t*>(d + b.o_bad), s);
+    launch_w_images(d_v, d_g, x, d_t, d_tn, nullptr, b.B, c.n1, vp, gx, tv, reinterpret_cast<uint32_t*>(d + b.o_bad), s);
     // G1: r = M_enc v (and its byte planes for Protocol 2)
     BgParams p = g1_params(b, c);
     p.out = r;

@@ -86,23 +86,21 @@ struct IvZsum {
 };
 
 // ------------------------------------------------------------------ kernels
-// dst block lp (8 rows of row_bytes) = src block map[lp]
-__global__ void gather8_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, const uint32_t* __restrict__ map,
-                               uint32_t n, uint32_t row_bytes) {
-    const uint32_t per = 8 * row_bytes / 16;
-    const uint64_t total = (uint64_t)n * per;
-    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t lp = (uint32_t)(e / per), c = (uint32_t)(e % per);
-        dst[(uint64_t)lp * per + c] = src[(uint64_t)map[lp] * per + c];
-    }
-}
-
 // The grouped GEMMs' item tables: group u owns PLANAR items [it_pl(u),
 // it_pl(u + 1)), W tiles outer x 16-row A tiles inner, and S8 items likewise
 // with 128-row A tiles (every group has at least one item of each).
-__global__ void expand_items_kernel(const IvGroup* __restrict__ groups, uint32_t U, uint32_t n_pl, uint32_t n_s8,
-                                    uint32_t wy, BgItem* __restrict__ items_pl, BgItem* __restrict__ items_s8) {
-    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+// The first n_chunks CTAs fill idmap[r-space entry] = corpus id of its row, a
+// chunk each.
+__global__ void tables_kernel(const IvGroup* __restrict__ groups, uint32_t U, uint32_t n_pl, uint32_t n_s8, uint32_t wy,
+                              BgItem* __restrict__ items_pl, BgItem* __restrict__ items_s8,
+                              const IvChunk* __restrict__ chunks, uint32_t n_chunks, const uint32_t* __restrict__ ids,
+                              uint32_t* __restrict__ idmap) {
+    if (blockIdx.x < n_chunks) {
+        const IvChunk c = chunks[blockIdx.x];
+        for (uint32_t i = threadIdx.x; i < c.rows; i += blockDim.x) idmap[c.r0 + i] = ids[c.row0 + i];
+        return;
+    }
+    const uint32_t e = (blockIdx.x - n_chunks) * blockDim.x + threadIdx.x;
     if (e >= n_pl + n_s8) return;
     const bool s8 = e >= n_pl;
     const uint32_t it = s8 ? e - n_pl : e;
@@ -120,13 +118,6 @@ __global__ void expand_items_kernel(const IvGroup* __restrict__ groups, uint32_t
     const BgItem item{(s8 ? g.t128 : g.t16) + xi, 8 * y0, x0, g.row0 + g.m, y0, g.lp0 + g.n};
     if (s8) items_s8[it] = item;
     else items_pl[it] = item;
-}
-
-// idmap[r-space entry] = corpus id of its row
-__global__ void idmap_kernel(const IvChunk* __restrict__ chunks, const uint32_t* __restrict__ ids,
-                             uint32_t* __restrict__ idmap) {
-    const IvChunk c = chunks[blockIdx.x];
-    for (uint32_t i = threadIdx.x; i < c.rows; i += blockDim.x) idmap[c.r0 + i] = ids[c.row0 + i];
 }
 
 // 128-bit accumulation of a 61 x 61-bit product.
@@ -364,7 +355,7 @@ struct IvfBlockJob {
     // outputs (one D2H)
     uint64_t o_ids, o_sc, o_n, o_fc, o_ft, o_err, out_end;
     // scratch
-    uint64_t o_items_pl, o_items_s8, o_vp, o_gx, o_tv, o_x, o_wv, o_wgx, o_wtv, o_r, o_f2, o_f3, o_idmap, o_ub, o_zpart,
+    uint64_t o_items_pl, o_items_s8, o_x, o_wv, o_wgx, o_wtv, o_r, o_f2, o_f3, o_idmap, o_ub, o_zpart,
         o_z, o_urpart, o_zv, o_pfail, o_urout, o_cs, o_ci, o_cn, total;
     CUtensorMap tm_wv, tm_wgx, tm_wtv, tm_u;
     CUtensorMap tm_wv2, tm_wgx2, tm_wtv2;  // 3-D views: two K steps per box
@@ -555,9 +546,6 @@ int ivf_block_plan(const bn_ivf& v, IvfBlockJob& j, uint32_t B, const uint32_t* 
     j.out_end = L.take<uint8_t>(0);
     j.o_items_pl = L.take<BgItem>(j.n_pl);
     j.o_items_s8 = L.take<BgItem>(j.n_s8);
-    j.o_vp = L.take<uint8_t>(8 * qb * N);
-    j.o_gx = L.take<uint8_t>(8 * qb * c.k_alh);
-    j.o_tv = L.take<uint8_t>(8 * qb * 2 * N);
     j.o_x = L.take<uint64_t>(qb * n1);
     j.o_wv = L.take<uint8_t>(8 * pb * N);
     j.o_wgx = L.take<uint8_t>(8 * pb * c.k_alh);
@@ -718,27 +706,14 @@ int ivf_block_launch(Engine& e, IvfBlockJob& j, DevMem& ws, PinnedMem& host, cud
     const IvChunk* dchunks = reinterpret_cast<const IvChunk*>(d + j.o_chunks);
     if (!j.verify_only) {
         if (j.P) {
-            // per-query operand images, then one image per (list, query) pair, grouped by list
-            if (c.k_alh != 2 * n1) CU(cudaMemsetAsync(d + j.o_gx, 0, 8ull * B * c.k_alh, s));
-            launch_planar_rows(dv, B, N, N, 0, U8(j.o_vp), N, 0, s);
+            // one operand image per (list, query) pair, grouped by list
             launch_lt_times_v(c.L.at<uint64_t>(), n1, dv, B, U64(j.o_x), s);
-            launch_planar_rows(U64(j.o_g), B, n1, n1, 1, U8(j.o_gx), c.k_alh, 0, s);
-            launch_planar_rows(U64(j.o_x), B, n1, n1, 1, U8(j.o_gx), c.k_alh, n1, s);
-            launch_w_tv(dv, U32(j.o_t), U32(j.o_tn), B, reinterpret_cast<int8_t*>(d + j.o_tv), err + 1, s);
-            const uint32_t* lmq = U32(j.o_lmq);
-            struct Img {
-                uint64_t src, dst;
-                uint32_t row_bytes;
-            };
-            const Img imgs[3] = {{j.o_vp, j.o_wv, N}, {j.o_gx, j.o_wgx, c.k_alh}, {j.o_tv, j.o_wtv, 2 * N}};
-            for (const Img& im : imgs)
-                gather8_kernel<<<grid_cap((uint64_t)j.P * im.row_bytes / 2, 256, (unsigned)sms * 8), 256, 0, s>>>(
-                    reinterpret_cast<const uint4*>(d + im.src), reinterpret_cast<uint4*>(d + im.dst), lmq, j.P,
-                    im.row_bytes);
-            idmap_kernel<<<j.NCH, 256, 0, s>>>(dchunks, c.ids.at<uint32_t>(), U32(j.o_idmap));
-            expand_items_kernel<<<(j.n_pl + j.n_s8 + 255) / 256, 256, 0, s>>>(
+            launch_w_images(dv, U64(j.o_g), U64(j.o_x), U32(j.o_t), U32(j.o_tn), U32(j.o_lmq), j.P, n1, U8(j.o_wv),
+                            U8(j.o_wgx), U8(j.o_wtv), err + 1, s);
+            tables_kernel<<<j.NCH + (j.n_pl + j.n_s8 + 255) / 256, 256, 0, s>>>(
                 reinterpret_cast<const IvGroup*>(d + j.o_groups), j.U, j.n_pl, j.n_s8, j.w_tile / 8,
-                reinterpret_cast<BgItem*>(d + j.o_items_pl), reinterpret_cast<BgItem*>(d + j.o_items_s8));
+                reinterpret_cast<BgItem*>(d + j.o_items_pl), reinterpret_cast<BgItem*>(d + j.o_items_s8), dchunks, j.NCH,
+                c.ids.at<uint32_t>(), U32(j.o_idmap));
             mark(1);
             // G1 r = M_c v_q, G2 f2 = -(AL_c g_q + H_c x_q), G3 f3 = M_c T_q + S_c v_q
             BgParams p{};
