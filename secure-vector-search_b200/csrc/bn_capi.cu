@@ -68,7 +68,7 @@ int upload_colmajor(bn_ctx* ctx, const uint64_t* host, uint64_t rows, uint32_t c
     TRY(tmp.alloc(ctx, chunk * cols * 8));
     for (uint64_t r0 = 0; r0 < rows; r0 += chunk) {
         uint64_t cr = std::min(chunk, rows - r0);
-        CU(cudaMemcpyAsync(tmp.p, host + r0 * cols, cr * cols * 8, cudaMemcpyHostToDevice, s));
+        TRY(stage_h2d(ctx, tmp.p, host + r0 * cols, cr * cols * 8, s));
         launch_transpose_u64(tmp.at<uint64_t>(), cr, cols, dst.at<uint64_t>() + r0, rows, s);
         CU(cudaStreamSynchronize(s));
     }
@@ -132,9 +132,8 @@ int upload_sparse_ell(bn_ctx* ctx, bn_sparse_csr S, uint64_t rows, Corpus& c, cu
         if (total > 0xffffffffull) return fail(BN_EINVAL, "s_mat too large for the sliced-ELL layout");
     }
     const uint64_t nnz = rows ? S.rowptr[rows] : 0;
-    for (uint64_t e = 0; e < nnz; ++e)
-        if (S.idx[e] >= N || (S.sign[e] != 1 && S.sign[e] != -1))
-            return fail(BN_EINVAL, "s_mat entry %llu is not (col < n, sign +-1)", (unsigned long long)e);
+    const uint64_t bad = first_bad_entry(S, nnz);
+    if (bad < nnz) return fail(BN_EINVAL, "s_mat entry %llu is not (col < n, sign +-1)", (unsigned long long)bad);
     TRY(c.s_ell.alloc(ctx, std::max<uint64_t>(total, 1) * 2));
     TRY(c.s_off.alloc(ctx, off.size() * 4));
     TRY(c.s_w.alloc(ctx, w.size() * 2));
@@ -145,23 +144,16 @@ int upload_sparse_ell(bn_ctx* ctx, bn_sparse_csr S, uint64_t rows, Corpus& c, cu
         TRY(rp.alloc(ctx, (rows + 1) * 8));
         TRY(ix.alloc(ctx, std::max<uint64_t>(nnz, 1) * 4));
         TRY(sg.alloc(ctx, std::max<uint64_t>(nnz, 1)));
-        CU(cudaMemcpyAsync(rp.p, S.rowptr, (rows + 1) * 8, cudaMemcpyHostToDevice, s));
+        TRY(stage_h2d(ctx, rp.p, S.rowptr, (rows + 1) * 8, s));
         if (nnz) {
-            CU(cudaMemcpyAsync(ix.p, S.idx, nnz * 4, cudaMemcpyHostToDevice, s));
-            CU(cudaMemcpyAsync(sg.p, S.sign, nnz, cudaMemcpyHostToDevice, s));
+            TRY(stage_h2d(ctx, ix.p, S.idx, nnz * 4, s));
+            TRY(stage_h2d(ctx, sg.p, S.sign, nnz, s));
         }
         launch_csr_to_ell(rp.at<uint64_t>(), ix.at<uint32_t>(), sg.at<int8_t>(), rows, c.s_off.at<uint32_t>(),
                           c.s_w.at<uint16_t>(), c.s_ell.at<uint16_t>(), s);
         CU(cudaGetLastError());
         CU(cudaStreamSynchronize(s));
     }
-    return BN_OK;
-}
-
-int validate_residues(const uint64_t* a, uint64_t count, const char* what) {
-    for (uint64_t i = 0; i < count; ++i)
-        if (a[i] >= P) return fail(BN_EINVAL, "%s[%llu] = %llu is not a canonical residue mod 2^61-1", what,
-                                   (unsigned long long)i, (unsigned long long)a[i]);
     return BN_OK;
 }
 
@@ -236,10 +228,10 @@ int device_encrypt(bn_ctx* ctx, const uint64_t* d_mq, uint64_t rows, uint32_t n1
         TRY(rp.alloc(ctx, (rows + 1) * 8));
         TRY(ix.alloc(ctx, std::max<uint64_t>(nnz, 1) * 4));
         TRY(sg.alloc(ctx, std::max<uint64_t>(nnz, 1)));
-        CU(cudaMemcpyAsync(rp.p, S.rowptr, (rows + 1) * 8, cudaMemcpyHostToDevice, s));
+        TRY(stage_h2d(ctx, rp.p, S.rowptr, (rows + 1) * 8, s));
         if (nnz) {
-            CU(cudaMemcpyAsync(ix.p, S.idx, nnz * 4, cudaMemcpyHostToDevice, s));
-            CU(cudaMemcpyAsync(sg.p, S.sign, nnz, cudaMemcpyHostToDevice, s));
+            TRY(stage_h2d(ctx, ix.p, S.idx, nnz * 4, s));
+            TRY(stage_h2d(ctx, sg.p, S.sign, nnz, s));
         }
         launch_apply_sparse(rp.at<uint64_t>(), ix.at<uint32_t>(), sg.at<int8_t>(), rows, N, m_enc.at<uint64_t>(), s);
         CU(cudaGetLastError());
@@ -262,8 +254,8 @@ int check_plain_inputs(const uint64_t* m_q, uint64_t rows, const uint64_t* L, co
     TRY(validate_residues(L, (uint64_t)N * n1, "l_subspace"));
     TRY(validate_residues(H, rows * n1, "h"));
     if (rows && S.rowptr[rows] && (!S.idx || !S.sign)) return fail(BN_EINVAL, "s_mat arrays are null");
-    for (uint64_t e = 0; rows && e < S.rowptr[rows]; ++e)
-        if (S.idx[e] >= N || (S.sign[e] != 1 && S.sign[e] != -1)) return fail(BN_EINVAL, "bad s_mat entry %llu", (unsigned long long)e);
+    const uint64_t nnz = rows ? S.rowptr[rows] : 0, bad = first_bad_entry(S, nnz);
+    if (bad < nnz) return fail(BN_EINVAL, "bad s_mat entry %llu", (unsigned long long)bad);
     return BN_OK;
 }
 
@@ -277,8 +269,8 @@ int build_corpus_from_plain(bn_ctx* ctx, Corpus& c, const uint64_t* m_q, uint64_
     TRY(d_L.alloc(ctx, (uint64_t)N * n1 * 8));
     TRY(d_H.alloc(ctx, rows * n1 * 8));
     if (rows) {
-        CU(cudaMemcpyAsync(d_mq.p, m_q, rows * N * 8, cudaMemcpyHostToDevice, s));
-        CU(cudaMemcpyAsync(d_H.p, H, rows * n1 * 8, cudaMemcpyHostToDevice, s));
+        TRY(stage_h2d(ctx, d_mq.p, m_q, rows * N * 8, s));
+        TRY(stage_h2d(ctx, d_H.p, H, rows * n1 * 8, s));
     }
     CU(cudaMemcpyAsync(d_L.p, L, (uint64_t)N * n1 * 8, cudaMemcpyHostToDevice, s));
     TRY(device_encrypt(ctx, d_mq.at<uint64_t>(), rows, n1, d_L.at<uint64_t>(), d_H.at<uint64_t>(), S, c.m_enc, al_rm, s));
@@ -341,7 +333,7 @@ int build_corpus_device_keys(bn_ctx* ctx, Corpus& c, const uint64_t* m_q, uint64
     DevMem d_mq, d_L, al_rm;
     TRY(d_mq.alloc(ctx, rows * N * 8));
     TRY(d_L.alloc(ctx, (uint64_t)N * n1 * 8));
-    if (rows) CU(cudaMemcpyAsync(d_mq.p, m_q, rows * N * 8, cudaMemcpyHostToDevice, s));
+    if (rows) TRY(stage_h2d(ctx, d_mq.p, m_q, rows * N * 8, s));
     CU(cudaMemcpyAsync(d_L.p, L, (uint64_t)N * n1 * 8, cudaMemcpyHostToDevice, s));
     TRY(device_encrypt_dev(ctx, d_mq.at<uint64_t>(), rows, n1, d_L.at<uint64_t>(), d_H.at<uint64_t>(),
                            d_rowptr.at<uint64_t>(), d_idx.at<uint32_t>(), d_sign.at<int8_t>(), c.m_enc, al_rm, s));
@@ -796,7 +788,7 @@ int run_verify(Engine& e, uint64_t row0, uint64_t rows, const uint64_t* r, const
     pack_meta(h, o, hm);
     CU(cudaSetDevice(e.ctx->device));
     CU(cudaMemcpyAsync(d, h, o.in_end, cudaMemcpyHostToDevice, e.stream));
-    CU(cudaMemcpyAsync(d + o.r, r, rows * 8, cudaMemcpyHostToDevice, e.stream));
+    TRY(stage_h2d(e.ctx, d + o.r, r, rows * 8, e.stream));
     const Meta m = meta_at(d, o, hm, &maps);
     const Scratch sc = scratch_at(d, o);
     const ChaChaKey* keys = reinterpret_cast<const ChaChaKey*>(d + o.seeds);
@@ -860,7 +852,7 @@ int run_scan(Engine& e, uint64_t row0, uint64_t rows, const uint64_t* v_encs, ui
                 reinterpret_cast<uint64_t*>(d + o_b), B, hm.seg_blk.back(), reinterpret_cast<uint64_t*>(d + o_r),
                 e.ctx->num_sms, reinterpret_cast<uint32_t*>(d + o_e), e.stream, e.ctx->debug_wait_cycles);
     CU(cudaGetLastError());
-    CU(cudaMemcpyAsync(r, d + o_r, (uint64_t)B * rows * 8, cudaMemcpyDeviceToHost, e.stream));
+    TRY(stage_d2h(e.ctx, r, d + o_r, (uint64_t)B * rows * 8, e.stream));
     uint32_t ev = 0;
     CU(cudaMemcpyAsync(&ev, d + o_e, 4, cudaMemcpyDeviceToHost, e.stream));
     CU(cudaStreamSynchronize(e.stream));
@@ -888,9 +880,7 @@ int run_dense_terms(Engine& e, uint64_t row0, uint64_t rows, const uint64_t* g, 
                        reinterpret_cast<uint64_t*>(d + o_g), reinterpret_cast<uint64_t*>(d + o_x),
                        reinterpret_cast<uint64_t*>(d + o_o), e.stream);
     CU(cudaGetLastError());
-    CU(cudaMemcpyAsync(out, d + o_o, rows * 8, cudaMemcpyDeviceToHost, e.stream));
-    CU(cudaStreamSynchronize(e.stream));
-    return BN_OK;
+    return stage_d2h(e.ctx, out, d + o_o, rows * 8, e.stream);
 }
 
 }  // namespace api
@@ -1021,8 +1011,7 @@ int bn_flat_build(bn_ctx* ctx, const uint64_t* m_enc, const uint64_t* a_l, const
         f->m = m;
         rc = c.m_enc.alloc(ctx, m * N * 8);
         if (rc == BN_OK && m) {
-            cudaError_t er = cudaMemcpyAsync(c.m_enc.p, m_enc, m * N * 8, cudaMemcpyHostToDevice, f->e.stream);
-            if (er != cudaSuccess) rc = fail(BN_ECUDA, "upload m_enc: %s", cudaGetErrorString(er));
+            rc = stage_h2d(ctx, c.m_enc.p, m_enc, m * N * 8, f->e.stream);
         }
         if (rc == BN_OK) rc = corpus_tmap(c);
         if (rc == BN_OK) rc = upload_colmajor(ctx, a_l, m, n1, c.al_cm, f->e.stream);
@@ -1412,8 +1401,7 @@ int bn_ivf_build(bn_ctx* ctx, uint32_t nlist, const uint64_t* off, const uint32_
     c.rows = rows;
     c.n1 = n1;
     if (rc == BN_OK) rc = c.m_enc.alloc(ctx, rows * N * 8);
-    if (rc == BN_OK && rows && cudaMemcpy(c.m_enc.p, m_enc, rows * N * 8, cudaMemcpyHostToDevice) != cudaSuccess)
-        rc = fail(BN_ECUDA, "upload m_enc failed");
+    if (rc == BN_OK) rc = stage_h2d(ctx, c.m_enc.p, m_enc, rows * N * 8, v->e.stream);
     if (rc == BN_OK) rc = corpus_tmap(c);
     if (rc == BN_OK) rc = c.ids.alloc(ctx, std::max<uint64_t>(rows, 1) * 4);
     if (rc == BN_OK && rows && cudaMemcpy(c.ids.p, ids, rows * 4, cudaMemcpyHostToDevice) != cudaSuccess)
@@ -1606,11 +1594,9 @@ int bn_keygen_h_s(bn_ctx* ctx, const uint8_t* h_seed, uint64_t m, uint32_t n1, u
                           (unsigned long long)s_cap);
             } else {
                 memcpy(s_rowptr, hrp.data(), (m + 1) * 8);
-                cudaError_t e = cudaMemcpyAsync(H, dH.p, m * n1 * 8, cudaMemcpyDeviceToHost, s);
-                if (e == cudaSuccess && hrp[m]) e = cudaMemcpyAsync(s_idx, ix.p, hrp[m] * 4, cudaMemcpyDeviceToHost, s);
-                if (e == cudaSuccess && hrp[m]) e = cudaMemcpyAsync(s_sign, sg.p, hrp[m], cudaMemcpyDeviceToHost, s);
-                if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-                if (e != cudaSuccess) rc = fail(BN_ECUDA, "keygen copy-back: %s", cudaGetErrorString(e));
+                rc = stage_d2h(ctx, H, dH.p, m * n1 * 8, s);
+                if (rc == BN_OK) rc = stage_d2h(ctx, s_idx, ix.p, hrp[m] * 4, s);
+                if (rc == BN_OK) rc = stage_d2h(ctx, s_sign, sg.p, hrp[m], s);
             }
         }
     }
@@ -1712,16 +1698,16 @@ int bn_encrypt_cluster(bn_ctx* ctx, const uint64_t* m_q, uint64_t m, uint32_t n,
         if (rc == BN_OK) rc = d_L.alloc(ctx, (uint64_t)N * n1 * 8);
         if (rc == BN_OK) rc = d_H.alloc(ctx, m * n1 * 8);
         if (rc == BN_OK) {
-            cudaMemcpyAsync(d_mq.p, m_q, m * N * 8, cudaMemcpyHostToDevice, s);
-            cudaMemcpyAsync(d_L.p, L, (uint64_t)N * n1 * 8, cudaMemcpyHostToDevice, s);
-            cudaMemcpyAsync(d_H.p, H, m * n1 * 8, cudaMemcpyHostToDevice, s);
+            rc = stage_h2d(ctx, d_mq.p, m_q, m * N * 8, s);
+            if (rc == BN_OK) rc = stage_h2d(ctx, d_L.p, L, (uint64_t)N * n1 * 8, s);
+            if (rc == BN_OK) rc = stage_h2d(ctx, d_H.p, H, m * n1 * 8, s);
+        }
+        if (rc == BN_OK) {
             rc = device_encrypt(ctx, d_mq.at<uint64_t>(), m, n1, d_L.at<uint64_t>(), d_H.at<uint64_t>(), S, enc, al, s);
         }
         if (rc == BN_OK) {
-            cudaMemcpyAsync(m_enc, enc.p, m * N * 8, cudaMemcpyDeviceToHost, s);
-            cudaMemcpyAsync(a_l, al.p, m * n1 * 8, cudaMemcpyDeviceToHost, s);
-            cudaError_t e = cudaStreamSynchronize(s);
-            if (e != cudaSuccess) rc = fail(BN_ECUDA, "encrypt: %s", cudaGetErrorString(e));
+            rc = stage_d2h(ctx, m_enc, enc.p, m * N * 8, s);
+            if (rc == BN_OK) rc = stage_d2h(ctx, a_l, al.p, m * n1 * 8, s);
         }
     }
     cudaStreamDestroy(s);

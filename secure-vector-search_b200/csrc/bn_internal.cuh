@@ -15,6 +15,22 @@
 #include "bn_kernels.cuh"
 #include "bn_tc.cuh"
 
+namespace bn {
+namespace api {
+// Pinned slots for copies of pageable host memory (bn_xfer.cu): one set per
+// context, made on first use, given back with it; one copy at a time uses them
+// (a copy that finds them taken goes to the driver directly).
+struct HostStage {
+    static constexpr int SLOTS = 3;
+    static constexpr uint64_t SLOT_BYTES = 2u << 20, MIN_BYTES = 128u << 10;
+    std::mutex mu;
+    void* p = nullptr;
+    cudaEvent_t ev[SLOTS] = {};
+    ~HostStage();
+};
+}  // namespace api
+}  // namespace bn
+
 // ------------------------------------------------------------------ context
 struct bn_ctx {
     int device = 0;
@@ -24,6 +40,7 @@ struct bn_ctx {
     long long debug_wait_cycles = 0;  // bn_debug_set_wait_limit (0 = the kernels' ~1 s default)
     uint64_t budget = 0, used = 0, peak = 0;
     std::mutex mu;
+    bn::api::HostStage stage;
 };
 
 namespace bn {
@@ -413,6 +430,13 @@ uint64_t block_plan_estimate(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k
 int block_prepare_engine(Engine& e, const std::vector<uint64_t>* offsets);
 int pick_ctas(uint64_t max_rows_per_query, uint32_t B, int sms);
 int validate_residues(const uint64_t* a, uint64_t count, const char* what);
+// First entry of S below nnz that is not (col < n, sign +-1), or nnz.
+uint64_t first_bad_entry(bn_sparse_csr S, uint64_t nnz);
+// Copies of pageable host memory in s's order (bn_xfer.cu).  stage_h2d: src may
+// be reused on return, the copy may still be under way on s; stage_d2h: dst is
+// written on return.
+int stage_h2d(bn_ctx* ctx, void* dst, const void* src, uint64_t bytes, cudaStream_t s);
+int stage_d2h(bn_ctx* ctx, void* dst, const void* src, uint64_t bytes, cudaStream_t s);
 // bn_ivf_build_keygen over lists whose global indices start at list0 (the
 // keys of list c are drawn from derive_h_seed(upload_seed, list0 + c)).
 int ivf_build_keygen_from(bn_ctx* ctx, uint32_t nlist, const uint64_t* off, const uint32_t* ids, const uint64_t* m_q,

@@ -1,0 +1,162 @@
+// bn_xfer.cu -- copies between pageable host memory and the device.
+//
+// A cudaMemcpy of pageable memory is copied by the driver through its own
+// staging on one host thread (and takes the first-touch page faults of a fresh
+// output array on it): 1.2 MB of r took about as long as the scan that computed
+// it.  Here such copies go through a few pinned slots of the context, filled
+// or emptied by several threads while the previous slot is on the link.
+#include <cuda_runtime.h>
+#include <omp.h>
+
+#include <algorithm>
+#include <cstring>
+
+#include "bn_internal.cuh"
+
+namespace bn {
+namespace api {
+
+namespace {
+
+// Threads for `bytes` of host memory traffic: one per 128 KB, at most 8 (a
+// call from a busy server's thread must not take every core).
+int threads_for(uint64_t bytes) {
+    const uint64_t t = bytes / (128u << 10);
+    return (int)std::max<uint64_t>(1, std::min<uint64_t>({t, 8, (uint64_t)omp_get_max_threads()}));
+}
+
+void parallel_memcpy(void* dst, const void* src, uint64_t bytes) {
+    const int nt = threads_for(bytes);
+    if (nt == 1) {
+        memcpy(dst, src, bytes);
+        return;
+    }
+    const uint64_t per = (bytes / nt + 4095) & ~4095ull;
+#pragma omp parallel for num_threads(nt) schedule(static, 1)
+    for (int t = 0; t < nt; ++t) {
+        const uint64_t b = std::min(bytes, per * t), e = t == nt - 1 ? bytes : std::min(bytes, per * (t + 1));
+        if (e > b) memcpy(static_cast<char*>(dst) + b, static_cast<const char*>(src) + b, e - b);
+    }
+}
+
+bool is_pageable(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+// The context's slots, made on the first staged copy (caller holds st.mu).
+int stage_ready(HostStage& st) {
+    if (st.p) return BN_OK;
+    CU(cudaMallocHost(&st.p, HostStage::SLOTS * HostStage::SLOT_BYTES));
+    for (cudaEvent_t& e : st.ev) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    return BN_OK;
+}
+
+// Bytes per slot of one copy: quarters of it, so that a copy of a few hundred
+// KB also overlaps its two halves, up to a whole slot.
+uint64_t slot_bytes(uint64_t bytes) {
+    return std::min<uint64_t>(HostStage::SLOT_BYTES, std::max<uint64_t>(256u << 10, align_up(bytes / 4, 4096)));
+}
+
+}  // namespace
+
+HostStage::~HostStage() {
+    for (cudaEvent_t e : ev)
+        if (e) cudaEventDestroy(e);
+    if (p) cudaFreeHost(p);
+}
+
+int stage_h2d(bn_ctx* ctx, void* dst, const void* src, uint64_t bytes, cudaStream_t s) {
+    if (!bytes) return BN_OK;
+    HostStage& st = ctx->stage;
+    std::unique_lock<std::mutex> g(st.mu, std::defer_lock);
+    if (bytes < HostStage::MIN_BYTES || !is_pageable(src) || !g.try_lock()) {  // another thread's copy is staged
+        CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+        return BN_OK;
+    }
+    TRY(stage_ready(st));
+    const uint64_t step = slot_bytes(bytes);
+    for (uint64_t off = 0, i = 0; off < bytes; off += step, ++i) {
+        const uint64_t n = std::min(step, bytes - off);
+        const int k = (int)(i % HostStage::SLOTS);
+        char* slot = static_cast<char*>(st.p) + k * HostStage::SLOT_BYTES;
+        CU(cudaEventSynchronize(st.ev[k]));  // the slot's last copy has left it
+        parallel_memcpy(slot, static_cast<const char*>(src) + off, n);
+        CU(cudaMemcpyAsync(static_cast<char*>(dst) + off, slot, n, cudaMemcpyHostToDevice, s));
+        CU(cudaEventRecord(st.ev[k], s));
+    }
+    return BN_OK;
+}
+
+int stage_d2h(bn_ctx* ctx, void* dst, const void* src, uint64_t bytes, cudaStream_t s) {
+    if (!bytes) return BN_OK;
+    HostStage& st = ctx->stage;
+    std::unique_lock<std::mutex> g(st.mu, std::defer_lock);
+    if (bytes < HostStage::MIN_BYTES || !is_pageable(dst) || !g.try_lock()) {
+        CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
+        CU(cudaStreamSynchronize(s));
+        return BN_OK;
+    }
+    TRY(stage_ready(st));
+    const uint64_t step = slot_bytes(bytes), total = (bytes + step - 1) / step;
+    for (uint64_t i = 0; i < total + HostStage::SLOTS - 1; ++i) {
+        if (i < total) {
+            const int k = (int)(i % HostStage::SLOTS);
+            const uint64_t off = i * step, n = std::min(step, bytes - off);
+            if (i < HostStage::SLOTS) CU(cudaEventSynchronize(st.ev[k]));  // an earlier call's copy may still read it
+            CU(cudaMemcpyAsync(static_cast<char*>(st.p) + k * HostStage::SLOT_BYTES, static_cast<const char*>(src) + off, n,
+                               cudaMemcpyDeviceToHost, s));
+            CU(cudaEventRecord(st.ev[k], s));
+        }
+        if (i + 1 >= HostStage::SLOTS) {
+            const uint64_t j = i + 1 - HostStage::SLOTS;  // the oldest copy in flight
+            const int k = (int)(j % HostStage::SLOTS);
+            const uint64_t off = j * step;
+            CU(cudaEventSynchronize(st.ev[k]));
+            parallel_memcpy(static_cast<char*>(dst) + off, static_cast<char*>(st.p) + k * HostStage::SLOT_BYTES,
+                            std::min(step, bytes - off));
+        }
+    }
+    return BN_OK;
+}
+
+// a >= p = 2^61 - 1 exactly when a or a + 1 has a bit from 61 on, so a run is
+// checked with one OR per element; the first offender is named.
+int validate_residues(const uint64_t* a, uint64_t count, const char* what) {
+    constexpr uint64_t RUN = 1u << 15;
+    const int64_t runs = (int64_t)((count + RUN - 1) / RUN);
+    int64_t bad = runs;
+    const int nt = threads_for(count * 8);
+#pragma omp parallel for num_threads(nt) schedule(static) reduction(min : bad) if (nt > 1)
+    for (int64_t b = 0; b < runs; ++b) {
+        const uint64_t i0 = b * RUN, i1 = std::min<uint64_t>(count, i0 + RUN);
+        uint64_t any = 0;
+        for (uint64_t i = i0; i < i1; ++i) any |= a[i] | (a[i] + 1);
+        if (any >> 61) bad = std::min(bad, b);
+    }
+    if (bad == runs) return BN_OK;
+    uint64_t i = bad * RUN;
+    while (a[i] < P) ++i;
+    return fail(BN_EINVAL, "%s[%llu] = %llu is not a canonical residue mod 2^61-1", what, (unsigned long long)i,
+                (unsigned long long)a[i]);
+}
+
+uint64_t first_bad_entry(bn_sparse_csr S, uint64_t nnz) {
+    constexpr uint64_t RUN = 1u << 15;
+    for (uint64_t i0 = 0; i0 < nnz; i0 += RUN) {
+        const uint64_t i1 = std::min(nnz, i0 + RUN);
+        uint32_t any = 0;  // a column from n on, or a sign whose square is not 1
+        for (uint64_t i = i0; i < i1; ++i) any |= S.idx[i] / N;
+        for (uint64_t i = i0; i < i1; ++i) any |= (uint32_t)(S.sign[i] * S.sign[i]) ^ 1u;
+        for (uint64_t i = i0; any && i < i1; ++i)
+            if (S.idx[i] >= N || (S.sign[i] != 1 && S.sign[i] != -1)) return i;
+    }
+    return nnz;
+}
+
+}  // namespace api
+}  // namespace bn
