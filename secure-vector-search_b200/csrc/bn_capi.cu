@@ -197,14 +197,16 @@ int attach_client(bn_ctx* ctx, Corpus& c, const uint64_t* L, const uint64_t* m_p
 
 // Device encryption: m_enc = m_q + H L^T + S (row-major, stays on device in
 // `m_enc`), AL = m_q L (row-major in `al_rm`).  crypto.rs:405-478.
-int device_encrypt_dev(bn_ctx* ctx, const uint64_t* d_mq, uint64_t rows, uint32_t n1, const uint64_t* d_L,
-                       const uint64_t* d_H, const uint64_t* d_rowptr, const uint32_t* d_idx, const int8_t* d_sign,
-                       DevMem& m_enc, DevMem& al_rm, cudaStream_t s) {
+int encrypt_products(bn_ctx* ctx, const uint64_t* d_mq, uint64_t rows, uint32_t n1, const uint64_t* d_L,
+                     const uint64_t* d_H, DevMem& m_enc, DevMem& al_rm, cudaStream_t s) {
     TRY(m_enc.alloc(ctx, rows * N * 8));
     TRY(al_rm.alloc(ctx, rows * n1 * 8));
     if (!rows) return BN_OK;
+    DevMem ws;
+    const int rc = encrypt_dense(ctx, d_mq, rows, n1, d_L, d_H, m_enc.at<uint64_t>(), al_rm.at<uint64_t>(), ws, s);
+    if (rc != BN_EBUDGET) return rc;
+    // no room for its scratch: the CUDA-core GEMMs, which need L^T only
     launch_gemm_abt(d_H, d_L, d_mq, rows, N, n1, m_enc.at<uint64_t>(), s);  // H L^T + M
-    launch_apply_sparse(d_rowptr, d_idx, d_sign, rows, N, m_enc.at<uint64_t>(), s);  // + S
     DevMem lt;  // AL = M L: B operand is L^T (n1 x n), K = n
     TRY(lt.alloc(ctx, (uint64_t)n1 * N * 8));
     launch_transpose_u64(d_L, N, n1, lt.at<uint64_t>(), N, s);
@@ -214,34 +216,30 @@ int device_encrypt_dev(bn_ctx* ctx, const uint64_t* d_mq, uint64_t rows, uint32_
     return BN_OK;
 }
 
+int device_encrypt_dev(bn_ctx* ctx, const uint64_t* d_mq, uint64_t rows, uint32_t n1, const uint64_t* d_L,
+                       const uint64_t* d_H, const uint64_t* d_rowptr, const uint32_t* d_idx, const int8_t* d_sign,
+                       DevMem& m_enc, DevMem& al_rm, cudaStream_t s) {
+    TRY(encrypt_products(ctx, d_mq, rows, n1, d_L, d_H, m_enc, al_rm, s));
+    if (!rows) return BN_OK;
+    launch_apply_sparse(d_rowptr, d_idx, d_sign, rows, N, m_enc.at<uint64_t>(), s);  // + S
+    CU(cudaGetLastError());
+    CU(cudaStreamSynchronize(s));
+    return BN_OK;
+}
+
 int device_encrypt(bn_ctx* ctx, const uint64_t* d_mq, uint64_t rows, uint32_t n1, const uint64_t* d_L,
                    const uint64_t* d_H, bn_sparse_csr S, DevMem& m_enc, DevMem& al_rm, cudaStream_t s) {
-    TRY(m_enc.alloc(ctx, rows * N * 8));
-    TRY(al_rm.alloc(ctx, rows * n1 * 8));
+    TRY(encrypt_products(ctx, d_mq, rows, n1, d_L, d_H, m_enc, al_rm, s));
     if (!rows) return BN_OK;
-    // H L^T + M, K = n1
-    launch_gemm_abt(d_H, d_L, d_mq, rows, N, n1, m_enc.at<uint64_t>(), s);
-    CU(cudaGetLastError());
-    {
-        const uint64_t nnz = S.rowptr[rows];
-        DevMem rp, ix, sg;
-        TRY(rp.alloc(ctx, (rows + 1) * 8));
-        TRY(ix.alloc(ctx, std::max<uint64_t>(nnz, 1) * 4));
-        TRY(sg.alloc(ctx, std::max<uint64_t>(nnz, 1)));
-        TRY(stage_h2d(ctx, rp.p, S.rowptr, (rows + 1) * 8, s));
-        if (nnz) {
-            TRY(stage_h2d(ctx, ix.p, S.idx, nnz * 4, s));
-            TRY(stage_h2d(ctx, sg.p, S.sign, nnz, s));
-        }
-        launch_apply_sparse(rp.at<uint64_t>(), ix.at<uint32_t>(), sg.at<int8_t>(), rows, N, m_enc.at<uint64_t>(), s);
-        CU(cudaGetLastError());
-        CU(cudaStreamSynchronize(s));
-    }
-    // AL = M L: B operand is L^T (n1 x n), K = n
-    DevMem lt;
-    TRY(lt.alloc(ctx, (uint64_t)n1 * N * 8));
-    launch_transpose_u64(d_L, N, n1, lt.at<uint64_t>(), N, s);
-    launch_gemm_abt(d_mq, lt.at<uint64_t>(), nullptr, rows, n1, N, al_rm.at<uint64_t>(), s);
+    const uint64_t nnz = S.rowptr[rows];
+    DevMem rp, ix, sg;
+    TRY(rp.alloc(ctx, (rows + 1) * 8));
+    TRY(ix.alloc(ctx, std::max<uint64_t>(nnz, 1) * 4));
+    TRY(sg.alloc(ctx, std::max<uint64_t>(nnz, 1)));
+    TRY(stage_h2d(ctx, rp.p, S.rowptr, (rows + 1) * 8, s));
+    TRY(stage_h2d(ctx, ix.p, S.idx, nnz * 4, s));
+    TRY(stage_h2d(ctx, sg.p, S.sign, nnz, s));
+    launch_apply_sparse(rp.at<uint64_t>(), ix.at<uint32_t>(), sg.at<int8_t>(), rows, N, m_enc.at<uint64_t>(), s);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(s));
     return BN_OK;

@@ -430,6 +430,11 @@ uint64_t block_plan_estimate(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k
 int block_prepare_engine(Engine& e, const std::vector<uint64_t>* offsets);
 int pick_ctas(uint64_t max_rows_per_query, uint32_t B, int sms);
 int validate_residues(const uint64_t* a, uint64_t count, const char* what);
+// M + H L^T (row-major, to d_enc) and M L (to d_al) of `rows` plaintext rows on
+// the tensor cores (bn_encrypt.cu); ws is its scratch, BN_EBUDGET when that
+// does not fit.  Waits for s.
+int encrypt_dense(bn_ctx* ctx, const uint64_t* d_mq, uint64_t rows, uint32_t n1, const uint64_t* d_L,
+                  const uint64_t* d_H, uint64_t* d_enc, uint64_t* d_al, DevMem& ws, cudaStream_t s);
 // First entry of S below nnz that is not (col < n, sign +-1), or nnz.
 uint64_t first_bad_entry(bn_sparse_csr S, uint64_t nnz);
 // Copies of pageable host memory in s's order (bn_xfer.cu).  stage_h2d: src may

@@ -1406,14 +1406,30 @@ gemm_abt_kernel(const uint64_t* __restrict__ A, const uint64_t* __restrict__ B, 
         }
 }
 
+// A warp per row, 32 entries at a time; entries of one batch that name the same
+// column (a CSR may repeat one) are applied one after the other.
 __global__ void apply_sparse_kernel(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx,
-                                    const int8_t* __restrict__ sign, uint64_t rows, uint32_t cols,
-                                    uint64_t* __restrict__ C) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += (uint64_t)gridDim.x * blockDim.x)
-        for (uint64_t c = rowptr[i]; c < rowptr[i + 1]; ++c) {
-            uint64_t* p = C + i * cols + idx[c];
-            *p = sign[c] > 0 ? add_mod(*p, 1) : sub_mod(*p, 1);
+                                    const int8_t* __restrict__ sign, uint64_t rows, uint32_t cols, uint64_t* C) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t warps = (uint64_t)gridDim.x * blockDim.x / 32;
+    for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; i < rows; i += warps) {
+        const uint64_t b = rowptr[i], e = rowptr[i + 1];
+        for (uint64_t c = b; c < e; c += 32) {
+            const bool on = c + lane < e;
+            const uint32_t col = on ? idx[c + lane] : 0xffffffffu - lane;  // idle lanes: columns of their own
+            const bool neg = on && sign[c + lane] < 0;
+            const uint32_t same = __match_any_sync(FULL, col);
+            const uint32_t rank = __popc(same & ((1u << lane) - 1));
+            const uint32_t turns = __reduce_max_sync(FULL, rank);
+            for (uint32_t t = 0; t <= turns; ++t) {
+                if (on && rank == t) {
+                    uint64_t* p = C + i * cols + col;
+                    *p = neg ? sub_mod(*p, 1) : add_mod(*p, 1);
+                }
+                __syncwarp();
+            }
         }
+    }
 }
 
 __global__ void transpose_u64_kernel(const uint64_t* __restrict__ in, uint64_t rows, uint32_t cols,
@@ -1611,7 +1627,7 @@ void launch_gemm_abt(const uint64_t* d_A, const uint64_t* d_B, const uint64_t* d
 
 void launch_apply_sparse(const uint64_t* d_rowptr, const uint32_t* d_idx, const int8_t* d_sign, uint64_t rows,
                          uint32_t cols, uint64_t* d_C, cudaStream_t s) {
-    apply_sparse_kernel<<<grid_for(rows, 256, 148 * 16), 256, 0, s>>>(d_rowptr, d_idx, d_sign, rows, cols, d_C);
+    apply_sparse_kernel<<<grid_for(rows * 32, 256, 148 * 16), 256, 0, s>>>(d_rowptr, d_idx, d_sign, rows, cols, d_C);
 }
 
 void launch_transpose_u64(const uint64_t* d_in, uint64_t rows, uint32_t cols, uint64_t* d_out, uint64_t out_ld,
