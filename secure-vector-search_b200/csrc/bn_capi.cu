@@ -548,7 +548,7 @@ int enqueue_pipeline(bn_ctx* ctx, const Corpus& c, const Sizes& z, const Meta& m
     }
     if (z.k) {
         launch_decode_topk(sc.r, decode_corpus(c), m.segs, m.seg_unit, m.dq, z.B, in.v, in.g, sc.x, in.t, in.t_nnz, z.k,
-                           z.ctas, sc.topk, out.mv, out.ids, out.scores, out.n, s);
+                           z.ctas, decode_split(m.units, ctx->num_sms), sc.topk, out.mv, out.ids, out.scores, out.n, s);
     } else {
         CU(cudaMemsetAsync(out.n, 0, (uint64_t)z.B * 4, s));
     }
@@ -558,7 +558,8 @@ int enqueue_pipeline(bn_ctx* ctx, const Corpus& c, const Sizes& z, const Meta& m
 
 Meta meta_at(char* d, const RunLayout& o, const HostMeta& hm, const TcMaps* maps) {
     return Meta{reinterpret_cast<ScanSeg*>(d + o.segs), reinterpret_cast<uint64_t*>(d + o.seg_blk),
-                reinterpret_cast<uint64_t*>(d + o.seg_unit), (uint32_t)hm.segs.size(), hm.seg_blk.empty() ? 0 : hm.seg_blk.back(),
+                reinterpret_cast<uint64_t*>(d + o.seg_unit), hm.seg_unit.empty() ? 0 : hm.seg_unit.back(),
+                (uint32_t)hm.segs.size(), hm.seg_blk.empty() ? 0 : hm.seg_blk.back(),
                 reinterpret_cast<VerifySeg*>(d + o.vsegs), (uint32_t)hm.vsegs.size(),
                 reinterpret_cast<DecodeQuery*>(d + o.dq), reinterpret_cast<TcBlock*>(d + o.tc_blocks),
                 (uint32_t)hm.blocks.size(), reinterpret_cast<TcPanel*>(d + o.tc_panels), (uint32_t)hm.panels.size(),
@@ -604,8 +605,8 @@ void engine_free(Engine& e) {
 
 // Decode CTAs of a run: DECODE_CTAS_PER_SM per SM in total (one wave of
 // the decode kernel), shared among the queries in proportion to their
-// units (32-row blocks), at least one per query and at most one per tile
-// of 8 units.  Returns the total.
+// units (32-row blocks), at least one per query and at most one per unit
+// (decode_split) or tile of 8 units.  Returns the total.
 uint32_t assign_decode_ctas(HostMeta& hm, int sms) {
     std::vector<uint64_t> units(hm.dq.size(), 0);
     uint64_t total = 0;
@@ -614,11 +615,11 @@ uint32_t assign_decode_ctas(HostMeta& hm, int sms) {
         if (d.nseg) units[q] = hm.seg_unit[d.seg0 + d.nseg] - hm.seg_unit[d.seg0];
         total += units[q];
     }
-    const uint64_t target = (uint64_t)sms * DECODE_CTAS_PER_SM;
+    const uint64_t target = (uint64_t)sms * DECODE_CTAS_PER_SM, tile = decode_split(total, sms) ? 1 : 8;
     uint32_t next = 0;
     for (size_t q = 0; q < hm.dq.size(); ++q) {
         uint64_t c = total ? (target * units[q] + total - 1) / total : 1;
-        c = std::max<uint64_t>(1, std::min(c, (units[q] + 7) / 8));
+        c = std::max<uint64_t>(1, std::min(c, (units[q] + tile - 1) / tile));
         hm.dq[q].cta0 = next;
         hm.dq[q].ctas = (uint32_t)c;
         next += (uint32_t)c;

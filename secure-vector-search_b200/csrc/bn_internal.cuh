@@ -241,6 +241,7 @@ struct Meta {  // device pointers (+ host tensor maps)
     const ScanSeg* segs;
     const uint64_t* seg_blk;
     const uint64_t* seg_unit;  // decode units (32-row corpus blocks) per segment, prefix sums
+    uint64_t units;            // their total
     uint32_t nseg;
     uint64_t total_blocks;
     const VerifySeg* vsegs;

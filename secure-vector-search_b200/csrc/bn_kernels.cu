@@ -644,30 +644,48 @@ __device__ __forceinline__ void topk_offer(TopkBuf& b, bool valid, int64_t s, ui
 // folded lazily: every term is < 2^61, three terms fit below 2^63.
 __device__ __forceinline__ uint64_t signed_term(uint64_t x, bool neg) { return neg ? P - x : x; }
 
-// The columns [k_begin, k_end) of AL_i . g + H_i . x for corpus row gr from the 32-row-blocked alh_b: the
-// 2 n1 columns of the row's block are contiguous, so a warp's batch of 32
-// column loads is one 8 KB run.  lim[2k], lim[2k+1] hold the limbs of g_k
-// (k < n1) and of x_(k-n1) (k >= n1).  Every column adds lo*b + hi*c <
-// 2^53 + 2^50 (hi < 2^29: residues are < 2^61) to an accumulator, so the
-// 2 n1 <= 1024 columns stay below 2^64 with no fold.
-__device__ __forceinline__ uint64_t dense_terms_row(const uint64_t* __restrict__ alh_b, uint32_t n1, uint64_t gr,
-                                                    const uint4* __restrict__ lim, uint32_t k_begin, uint32_t k_end) {
-    const uint64_t* p = alh_b + (gr >> 5) * (2ull * n1) * 32 + (gr & 31);
-    uint64_t a0 = 0, a1 = 0, a2 = 0;
-    for (uint32_t k0 = k_begin; k0 < k_end; k0 += 32) {  // ranges are multiples of 32 columns
-        uint64_t xs[32];
+// The columns [k_begin, k_end) (multiples of 32) of AL g + H x for the 32 rows of
+// block blk, row l's sum to lane l, from alh_b, where the 2 n1 columns of a block
+// are contiguous.  A 16-byte load takes two rows of two columns per warp (lanes
+// 0-15 rows 2l, 2l + 1 of column k, lanes 16-31 of column k + 1), so a column's
+// limbs, lim[2k], lim[2k + 1] (of g_k for k < n1, of x_(k-n1) for k >= n1), are
+// read from shared memory once for 32 rows of two columns: the decode is bound by
+// the shared-memory pipe as much as by HBM, and one row per lane read them twice
+// as often.  Every column adds lo*b + hi*c < 2^53 + 2^50 (hi < 2^29: residues are
+// < 2^61) to an accumulator, so the 2 n1 <= 1024 columns stay below 2^64 with no
+// fold.
+__device__ __forceinline__ uint64_t dense_terms_block(const uint64_t* __restrict__ alh_b, uint32_t n1, uint64_t blk,
+                                                      const uint4* __restrict__ lim, uint32_t k_begin, uint32_t k_end,
+                                                      uint32_t lane) {
+    const uint32_t half = lane >> 4;
+    const ulonglong2* p =
+        reinterpret_cast<const ulonglong2*>(alh_b + blk * (2ull * n1) * 32 + (uint64_t)half * 32 + 2 * (lane & 15));
+    uint64_t a[2][3] = {};  // rows 2 (l & 15), + 1
+    for (uint32_t k0 = k_begin; k0 < k_end; k0 += 32) {
+        ulonglong2 xs[16];
 #pragma unroll
-        for (int kk = 0; kk < 32; ++kk) xs[kk] = __ldg(p + (uint64_t)(k0 + kk) * 32);
+        for (int kk = 0; kk < 16; ++kk) xs[kk] = __ldg(p + (uint64_t)(k0 + 2 * kk) * 16);
 #pragma unroll
-        for (int kk = 0; kk < 32; ++kk) {
-            const uint4 l0 = lim[2 * (k0 + kk)], l1 = lim[2 * (k0 + kk) + 1];  // {b0,b1,b2,c0}, {c1,c2,-,-}
-            const uint32_t xl = (uint32_t)xs[kk], xh = (uint32_t)(xs[kk] >> 32);
-            a0 = mac(mac(a0, xl, l0.x), xh, l0.w);
-            a1 = mac(mac(a1, xl, l0.y), xh, l1.x);
-            a2 = mac(mac(a2, xl, l0.z), xh, l1.y);
+        for (int kk = 0; kk < 16; ++kk) {
+            const uint32_t col = k0 + 2 * kk + half;
+            const uint4 l0 = lim[2 * col], l1 = lim[2 * col + 1];  // {b0,b1,b2,c0}, {c1,c2,-,-}
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const uint64_t x = e ? xs[kk].y : xs[kk].x;
+                const uint32_t xl = (uint32_t)x, xh = (uint32_t)(x >> 32);
+                a[e][0] = mac(mac(a[e][0], xl, l0.x), xh, l0.w);
+                a[e][1] = mac(mac(a[e][1], xl, l0.y), xh, l1.x);
+                a[e][2] = mac(mac(a[e][2], xl, l0.z), xh, l1.y);
+            }
         }
     }
-    return combine3(a0, a1, a2);
+    // lanes l and l ^ 16 hold the even and the odd columns of the same two rows:
+    // the lower one takes the first row's halves, the upper one the second's
+    uint64_t t[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        t[i] = (half ? a[1][i] : a[0][i]) + __shfl_xor_sync(FULL, half ? a[0][i] : a[1][i], 16);
+    return __shfl_sync(FULL, combine3(t[0], t[1], t[2]), (lane >> 1) | ((lane & 1) << 4));
 }
 
 // Two zero-extended 16-bit halves from bytes 0, 1 (sel 0x4140) or 2, 3
@@ -909,9 +927,15 @@ __device__ __forceinline__ void warp_topk_reduce(int64_t& ls, uint32_t& li, int 
 // warp's own list, merged at the end with no barrier in the loop); the CTA's
 // best k go to the scratch lists, and the last CTA of the query to finish (a
 // ticket taken after a device-scope fence, no waiting) merges them.
+//
+// SPLIT (few units, see launch_decode_topk): the CTA's eight warps share one unit
+// at a time, four a quarter of the dense columns each, two S v and two M T, and
+// take turns in adding the shares up and ranking them: a corpus of 5,000 rows is
+// 157 units, which whole-unit warps put on 20 CTAs (50 us) and this on 157 (32 us).
 constexpr uint32_t DT_WARPS = DT_THREADS / 32;
+constexpr uint32_t DT_DENSE = 4, DT_S = 2, DT_T = 2;  // SPLIT: warps per part (2 n1 / 4 is a multiple of 32)
 
-template <bool WARP_LISTS>
+template <bool WARP_LISTS, bool SPLIT>
 __global__ void __launch_bounds__(DT_THREADS, DECODE_CTAS_PER_SM)
 decode_topk_kernel(const uint64_t* __restrict__ r, DecodeCorpus dc, const ScanSeg* __restrict__ segs,
                    const uint64_t* __restrict__ seg_unit, const DecodeQuery* __restrict__ queries,
@@ -929,7 +953,9 @@ decode_topk_kernel(const uint64_t* __restrict__ r, DecodeCorpus dc, const ScanSe
     const uint32_t cta = blockIdx.x - dq.cta0;
     const uint32_t n1 = dc.n1;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    extern __shared__ uint4 dyn_limbs[];  // 2 x uint4 per column: g's n1 columns, then x's
+    // 2 x uint4 per column: g's n1 columns, then x's; SPLIT: after them the warps'
+    // shares of a unit's 32 rows, units in turn
+    extern __shared__ uint4 dyn_limbs[];
     __shared__ uint64_t vt[ELL_TABLE];  // [v_enc, 0, p - v_enc, 0]: the S . v table
     __shared__ uint32_t tl[N];
     struct WarpXchg {  // the warps' lists on their way to warp 0
@@ -963,20 +989,14 @@ decode_topk_kernel(const uint64_t* __restrict__ r, DecodeCorpus dc, const ScanSe
         u_begin = seg_unit[dq.seg0];
         u_count = seg_unit[dq.seg0 + dq.nseg] - u_begin;
     }
-    const uint64_t tiles = (u_count + DT_WARPS - 1) / DT_WARPS;
-    // The buffer is checked (two CTA barriers) every DT_CHECK tiles, not
-    // every tile, so the warps may drift apart within that window; between
-    // checks at most DT_CHECK * 256 rows append, and a check compacts above
-    // CAND_CAP - DT_CHECK * 256 = 1024 >= k entries.
-    constexpr uint32_t DT_CHECK = 4;
-    static_assert(CAND_CAP - DT_CHECK * DT_THREADS >= TOPK_MAX, "candidate buffer too small for the check interval");
-    uint32_t it = 0;
-    for (uint64_t tile = cta; tile < tiles; tile += dq.ctas, ++it) {
-        const uint64_t u = tile * DT_WARPS + warp;
-        bool valid = false;
-        int64_t score = 0;
-        uint32_t id = 0;
-        if (u < u_count) {  // warp-uniform
+    if constexpr (SPLIT) {
+        // The buffer is checked (two CTA barriers) every SP_CHECK units; between
+        // checks at most SP_CHECK * 32 rows append, and a check compacts above
+        // CAND_CAP - SP_CHECK * 32 = 1024 >= k entries.
+        constexpr uint32_t SP_CHECK = 32;
+        static_assert(CAND_CAP - SP_CHECK * 32 >= TOPK_MAX, "candidate buffer too small for the check interval");
+        uint32_t it = 0;
+        for (uint64_t u = cta; u < u_count; u += dq.ctas, ++it) {
             const uint64_t gu = u_begin + u;
             uint32_t sa = dq.seg0, sb = dq.seg0 + dq.nseg;  // last segment with seg_unit <= gu
             while (sb - sa > 1) {
@@ -986,36 +1006,102 @@ decode_topk_kernel(const uint64_t* __restrict__ r, DecodeCorpus dc, const ScanSe
             const ScanSeg sg = segs[sa];
             const uint64_t blk = (sg.row0 >> 5) + (gu - seg_unit[sa]);
             const uint64_t gr = blk * 32 + lane;
-            valid = gr >= sg.row0 && gr < sg.row0 + sg.rows;
+            const bool valid = gr >= sg.row0 && gr < sg.row0 + sg.rows;
             const uint64_t ridx = sg.out0 + (gr - sg.row0);
+            const bool mine = it % DT_WARPS == warp;  // this warp adds the unit up
             uint64_t rv = 0;
-            if (valid) {
+            uint32_t id = 0;
+            if (mine && valid) {
                 rv = r[ridx];
                 id = dc.ids ? dc.ids[gr] : (uint32_t)gr;
             }
-            uint64_t m_t = 0;
-            if (dc.m8_cm) {
-                const int32_t mt = m_times_t_warp(dc.m8_cm, (dc.rows + 31) & ~31ull, blk, tl, tn, lane);
-                m_t = mt >= 0 ? (uint64_t)mt : P - (uint64_t)(-(int64_t)mt);
+            uint64_t part = 0;
+            if (warp < DT_DENSE) {
+                const uint32_t cols = 2 * n1 / DT_DENSE;
+                part = dense_terms_block(dc.alh_b, n1, blk, dyn_limbs, warp * cols, (warp + 1) * cols, lane);
+            } else if (warp < DT_DENSE + DT_S) {
+                part = s_times_v_part<DT_S>(dc, blk, vt, warp - DT_DENSE, lane);
+            } else {  // half of the T entries each, whole groups of 32
+                const uint32_t per = (tn / DT_T + 31) & ~31u, c0 = min(tn, (warp - DT_DENSE - DT_S) * per);
+                const uint32_t c1 = warp == DT_WARPS - 1 ? tn : min(tn, per);
+                if (dc.m8_cm) {
+                    const int32_t mt = m_times_t_warp(dc.m8_cm, (dc.rows + 31) & ~31ull, blk, tl + c0, c1 - c0, lane);
+                    part = mt >= 0 ? (uint64_t)mt : P - (uint64_t)(-(int64_t)mt);
+                } else if (valid) {
+                    part = m_times_t_cm(dc.mp_cm, dc.rows, gr, tl, c0, c1);
+                }
             }
-            const uint64_t s_v = s_times_v_part<1>(dc, blk, vt, 0, lane);
-            if (valid) {
-                if (!dc.m8_cm) m_t = m_times_t_cm(dc.mp_cm, dc.rows, gr, tl, 0, tn);
-                const uint64_t dense = dense_terms_row(dc.alh_b, n1, gr, dyn_limbs, 0, 2 * n1);
-                const uint64_t mv = sub_mod(sub_mod(rv, add_mod(dense, m_t)), s_v);
-                if (mv_out) mv_out[ridx] = mv;
-                score = to_signed(mv);
+            auto sh = reinterpret_cast<uint64_t(*)[32]>(dyn_limbs + 4 * n1) + (it & 1) * DT_WARPS;
+            sh[warp][lane] = part;
+            __syncthreads();  // one per unit: the other buffer is rewritten only after the next one
+            if (mine) {
+                uint64_t sum = part;
+#pragma unroll
+                for (uint32_t w = 1; w < DT_WARPS; ++w) sum = add_mod(sum, sh[(warp + w) % DT_WARPS][lane]);
+                const uint64_t mv = sub_mod(rv, sum);
+                if (valid && mv_out) mv_out[ridx] = mv;
+                const int64_t score = to_signed(mv);
+                if constexpr (WARP_LISTS) warp_topk_offer(ls, li, (int)k, valid, score, id, lane);
+                else topk_offer(buf, valid, score, id, buf.thr_s, buf.thr_i, buf.have_thr);
             }
+            if constexpr (!WARP_LISTS)
+                if (it % SP_CHECK == SP_CHECK - 1 && topk_full(buf, CAND_CAP - SP_CHECK * 32)) topk_compact(buf, (int)k);
         }
-        if constexpr (WARP_LISTS) {
-            warp_topk_offer(ls, li, (int)k, valid, score, id, lane);
-        } else {
-            const int64_t th_s = buf.thr_s;
-            const uint32_t th_i = buf.thr_i;
-            const int ht = buf.have_thr;
-            topk_offer(buf, valid, score, id, th_s, th_i, ht);
-            if (it % DT_CHECK == DT_CHECK - 1 && topk_full(buf, CAND_CAP - DT_CHECK * DT_THREADS))
-                topk_compact(buf, (int)k);
+    } else {
+        const uint64_t tiles = (u_count + DT_WARPS - 1) / DT_WARPS;
+        // The buffer is checked (two CTA barriers) every DT_CHECK tiles, not
+        // every tile, so the warps may drift apart within that window; between
+        // checks at most DT_CHECK * 256 rows append, and a check compacts above
+        // CAND_CAP - DT_CHECK * 256 = 1024 >= k entries.
+        constexpr uint32_t DT_CHECK = 4;
+        static_assert(CAND_CAP - DT_CHECK * DT_THREADS >= TOPK_MAX, "candidate buffer too small for the check interval");
+        uint32_t it = 0;
+        for (uint64_t tile = cta; tile < tiles; tile += dq.ctas, ++it) {
+            const uint64_t u = tile * DT_WARPS + warp;
+            bool valid = false;
+            int64_t score = 0;
+            uint32_t id = 0;
+            if (u < u_count) {  // warp-uniform
+                const uint64_t gu = u_begin + u;
+                uint32_t sa = dq.seg0, sb = dq.seg0 + dq.nseg;  // last segment with seg_unit <= gu
+                while (sb - sa > 1) {
+                    const uint32_t mid = (sa + sb) >> 1;
+                    if (seg_unit[mid] <= gu) sa = mid; else sb = mid;
+                }
+                const ScanSeg sg = segs[sa];
+                const uint64_t blk = (sg.row0 >> 5) + (gu - seg_unit[sa]);
+                const uint64_t gr = blk * 32 + lane;
+                valid = gr >= sg.row0 && gr < sg.row0 + sg.rows;
+                const uint64_t ridx = sg.out0 + (gr - sg.row0);
+                uint64_t rv = 0;
+                if (valid) {
+                    rv = r[ridx];
+                    id = dc.ids ? dc.ids[gr] : (uint32_t)gr;
+                }
+                uint64_t m_t = 0;
+                if (dc.m8_cm) {
+                    const int32_t mt = m_times_t_warp(dc.m8_cm, (dc.rows + 31) & ~31ull, blk, tl, tn, lane);
+                    m_t = mt >= 0 ? (uint64_t)mt : P - (uint64_t)(-(int64_t)mt);
+                }
+                const uint64_t s_v = s_times_v_part<1>(dc, blk, vt, 0, lane);
+                const uint64_t dense = dense_terms_block(dc.alh_b, n1, blk, dyn_limbs, 0, 2 * n1, lane);
+                if (valid) {
+                    if (!dc.m8_cm) m_t = m_times_t_cm(dc.mp_cm, dc.rows, gr, tl, 0, tn);
+                    const uint64_t mv = sub_mod(sub_mod(rv, add_mod(dense, m_t)), s_v);
+                    if (mv_out) mv_out[ridx] = mv;
+                    score = to_signed(mv);
+                }
+            }
+            if constexpr (WARP_LISTS) {
+                warp_topk_offer(ls, li, (int)k, valid, score, id, lane);
+            } else {
+                const int64_t th_s = buf.thr_s;
+                const uint32_t th_i = buf.thr_i;
+                const int ht = buf.have_thr;
+                topk_offer(buf, valid, score, id, th_s, th_i, ht);
+                if (it % DT_CHECK == DT_CHECK - 1 && topk_full(buf, CAND_CAP - DT_CHECK * DT_THREADS))
+                    topk_compact(buf, (int)k);
+            }
         }
     }
     const uint32_t ctas = dq.ctas;
@@ -1450,6 +1536,13 @@ __global__ void transpose_u64_kernel(const uint64_t* __restrict__ in, uint64_t r
     }
 }
 
+// The entries of a row may stand in any of its slots; they are dealt out so that
+// the decode's table loads meet few bank conflicts.  One of those loads reads, in
+// each half of a warp, 4 consecutive slots x 4 groups of 8 rows, and the 16
+// 8-byte bank pairs are the table index mod 16: slot k of row group g prefers
+// indices of class (k mod 4) + 4 ((g + k / 4) mod 4), which are 16 different ones
+// over such a load, and every row meets every class once in 16 slots.  Entries
+// whose class has no slot left (7 % at the mean of 128 per row) fill the others.
 __global__ void csr_to_ell_kernel(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx,
                                   const int8_t* __restrict__ sign, uint64_t rows, const uint32_t* __restrict__ s_off,
                                   const uint16_t* __restrict__ s_w, uint16_t* __restrict__ ell) {
@@ -1458,12 +1551,23 @@ __global__ void csr_to_ell_kernel(const uint64_t* __restrict__ rowptr, const uin
     const uint64_t rows32 = (rows + 31) & ~31ull;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows32; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t slice = i >> 5;
-        const uint32_t sl = (uint32_t)(i & 31), off = s_off[slice], w = s_w[slice];
+        const uint32_t sl = (uint32_t)(i & 31), w = s_w[slice], grp = sl >> 3;
+        uint16_t* out = ell + s_off[slice] + sl;
         const uint64_t b = i < rows ? rowptr[i] : 0, e = i < rows ? rowptr[i + 1] : 0;
-        for (uint32_t c = 0; c < w; ++c) {
-            uint16_t v = (uint16_t)ELL_PAD;
-            if (b + c < e) v = (uint16_t)(idx[b + c] + (sign[b + c] < 0 ? ELL_NEG : 0u));
-            ell[off + (uint64_t)c * 32 + sl] = v;
+        for (uint32_t c = 0; c < w; ++c) out[c * 32] = (uint16_t)ELL_PAD;
+        uint32_t fill = 0;  // second pass: slots below are taken
+        for (int pass = 0; pass < 2; ++pass) {
+            uint8_t period[16] = {};  // per class: entries met so far, one per 16 slots
+            for (uint64_t c = b; c < e; ++c) {
+                const uint32_t f = idx[c] + (sign[c] < 0 ? ELL_NEG : 0u), cls = f & 15;
+                const uint32_t k = (cls & 3) + 4 * (((cls >> 2) - grp) & 3) + 16u * period[cls];
+                if (period[cls] < 255) ++period[cls];
+                if (pass == 0 && k < w) out[k * 32] = (uint16_t)f;
+                if (pass == 1 && k >= w) {
+                    while (out[fill * 32] != ELL_PAD) ++fill;  // the row has at most w entries
+                    out[fill * 32] = (uint16_t)f;
+                }
+            }
         }
     }
 }
@@ -1586,22 +1690,17 @@ void launch_decode_layout(const uint64_t* d_al_cm, const uint64_t* d_h_cm, const
 
 void launch_decode_topk(const uint64_t* d_r, const DecodeCorpus& dc, const ScanSeg* d_segs, const uint64_t* d_seg_unit,
                         const DecodeQuery* d_q, uint32_t nq, const uint64_t* d_v, const uint64_t* d_g, const uint64_t* d_x, const uint32_t* d_t,
-                        const uint32_t* d_t_nnz, uint32_t k, uint32_t total_ctas, TopkScratch scratch,
+                        const uint32_t* d_t_nnz, uint32_t k, uint32_t total_ctas, bool split, TopkScratch scratch,
                         uint64_t* d_mv_out, uint32_t* d_out_ids, int64_t* d_out_scores, uint32_t* d_out_n,
                         cudaStream_t s) {
     if (!nq) return;
-    const unsigned dyn = 2 * 2 * dc.n1 * 16;
-    if (k >= 1 && k <= (uint32_t)WARP_TOPK_MAX) {  // every warp keeps its own list
-        cudaFuncSetAttribute(decode_topk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 2 * 512 * 16);
-        decode_topk_kernel<true><<<total_ctas, DT_THREADS, dyn, s>>>(d_r, dc, d_segs, d_seg_unit, d_q, d_v, d_g, d_x,
-                                                                     d_t, d_t_nnz, k, scratch, d_mv_out, d_out_ids,
-                                                                     d_out_scores, d_out_n, nq);
-    } else {
-        cudaFuncSetAttribute(decode_topk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 2 * 512 * 16);
-        decode_topk_kernel<false><<<total_ctas, DT_THREADS, dyn, s>>>(d_r, dc, d_segs, d_seg_unit, d_q, d_v, d_g, d_x,
-                                                                      d_t, d_t_nnz, k, scratch, d_mv_out, d_out_ids,
-                                                                      d_out_scores, d_out_n, nq);
-    }
+    const unsigned shares = split ? 2 * DT_WARPS * 32 * 8 : 0, dyn = 2 * 2 * dc.n1 * 16 + shares;
+    const bool lists = k >= 1 && k <= (uint32_t)WARP_TOPK_MAX;  // every warp keeps its own list
+    auto fn = split ? (lists ? decode_topk_kernel<true, true> : decode_topk_kernel<false, true>)
+                    : (lists ? decode_topk_kernel<true, false> : decode_topk_kernel<false, false>);
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * 2 * 512 * 16 + shares));
+    fn<<<total_ctas, DT_THREADS, dyn, s>>>(d_r, dc, d_segs, d_seg_unit, d_q, d_v, d_g, d_x, d_t, d_t_nnz, k, scratch,
+                                           d_mv_out, d_out_ids, d_out_scores, d_out_n, nq);
 }
 
 void launch_topk_rows(const uint64_t* d_a, const uint64_t* d_b, const uint64_t* d_c, uint64_t ld, uint64_t rows,

@@ -142,6 +142,11 @@ struct DecodeQuery {
 // Resident decode_topk CTAs per SM (its register bound); the host sizes
 // the decode grid to one wave of them.
 constexpr int DECODE_CTAS_PER_SM = 3;
+// Whether a run of `units` decode units in all gives its CTAs one unit at a time:
+// up to DECODE_SPLIT units per CTA of the wave; beyond, whole units per warp keep
+// more loads in flight.
+constexpr uint64_t DECODE_SPLIT = 2;
+constexpr bool decode_split(uint64_t units, int sms) { return units <= DECODE_SPLIT * DECODE_CTAS_PER_SM * (uint64_t)sms; }
 
 // Top-k candidate lists.
 constexpr int TOPK_MAX = 1024;
@@ -182,9 +187,10 @@ void launch_decode_layout(const uint64_t* d_al_cm, const uint64_t* d_h_cm, const
 // units [d_seg_unit[s], d_seg_unit[s + 1]) (nseg + 1 entries).  The launch
 // has total_ctas CTAs, query q owning d_q[q].cta0 .. + d_q[q].ctas (every
 // query at least one; cta0 ascending); the scratch lists are indexed by CTA.
+// split: a CTA takes one unit at a time (decode_split), else tiles of 8.
 void launch_decode_topk(const uint64_t* d_r, const DecodeCorpus& dc, const ScanSeg* d_segs, const uint64_t* d_seg_unit,
                         const DecodeQuery* d_q, uint32_t nq, const uint64_t* d_v, const uint64_t* d_g, const uint64_t* d_x, const uint32_t* d_t,
-                        const uint32_t* d_t_nnz, uint32_t k, uint32_t total_ctas, TopkScratch scratch,
+                        const uint32_t* d_t_nnz, uint32_t k, uint32_t total_ctas, bool split, TopkScratch scratch,
                         uint64_t* d_mv_out, uint32_t* d_out_ids, int64_t* d_out_scores, uint32_t* d_out_n,
                         cudaStream_t s);
 
