@@ -515,7 +515,7 @@ int enqueue_pipeline(bn_ctx* ctx, const Corpus& c, const Sizes& z, const Meta& m
             const uint32_t tc = std::min<uint32_t>(TC_MAX_TRIALS, z.trials - t0), nr = pass_rows(tc);
             if (ps == 0) {
                 launch_tc_ugen(m.vsegs, m.tc_blocks, m.nblocks, keys, nullptr, t0, tc, nr, sc.u_buf, sc.ur_part,
-                               z.trials, sc.flags, s);
+                               z.trials, sc.flags, s, 0, true);
                 if (prof0) CU(cudaEventRecord(prof0, s));
                 launch_tc_fused(c.tmap_m, m.maps->u[ps], m.maps->w, m.tc_panels, m.npanels, m.vsegs, tc, nr,
                                 z.trials, sc.z_part, sc.r_part, z.total_out, sc.err, ctx->num_sms, s,

@@ -488,6 +488,7 @@ query_prep_kernel(const uint64_t* __restrict__ L, uint32_t n1, const uint64_t* _
                   uint32_t run, uint32_t lt_ctas, uint64_t* __restrict__ x, uint32_t wimg_ctas, uint8_t* __restrict__ w,
                   uint32_t* __restrict__ zero, uint32_t zero_words) {
     __shared__ LtShared sh;
+    after_go();
     if (blockIdx.x < lt_ctas) {
         const uint32_t cols = n1 / LT_COLS, q0 = blockIdx.x / cols * run;
         lt_block(sh, L, n1, v, blockIdx.x % cols * LT_COLS, q0, min(nq, q0 + run), x);
@@ -965,12 +966,13 @@ decode_topk_kernel(const uint64_t* __restrict__ r, DecodeCorpus dc, const ScanSe
     __shared__ typename std::conditional<WARP_LISTS, WarpXchg, TopkBuf>::type buf;
     __shared__ int last_s;
     const uint32_t tn = min(t_nnz[q], (uint32_t)N);
-    for (uint32_t kk = threadIdx.x; kk < 2 * n1; kk += blockDim.x) {
-        const uint64_t w = kk < n1 ? gg[(uint64_t)q * n1 + kk] : xx[(uint64_t)q * n1 + (kk - n1)];
+    // the query's inputs, then x and r, which earlier kernels of this run compute
+    auto put_limbs = [&](uint32_t kk, uint64_t w) {
         const Limbs3 b = limbs(w), c = limbs_hi(w);
         dyn_limbs[2 * kk] = make_uint4(b.b0, b.b1, b.b2, c.b0);
         dyn_limbs[2 * kk + 1] = make_uint4(c.b1, c.b2, 0u, 0u);
-    }
+    };
+    for (uint32_t kk = threadIdx.x; kk < n1; kk += blockDim.x) put_limbs(kk, gg[(uint64_t)q * n1 + kk]);
     for (uint32_t j = threadIdx.x; j < N; j += blockDim.x) {
         const uint64_t x = vv[(uint64_t)q * N + j];
         vt[j] = x;
@@ -978,6 +980,8 @@ decode_topk_kernel(const uint64_t* __restrict__ r, DecodeCorpus dc, const ScanSe
     }
     if (threadIdx.x == 0) vt[ELL_PAD] = vt[ELL_TABLE - 1] = 0;
     for (uint32_t c = threadIdx.x; c < tn; c += blockDim.x) tl[c] = t_ent[(uint64_t)q * N + c];
+    after_wait();
+    for (uint32_t kk = threadIdx.x; kk < n1; kk += blockDim.x) put_limbs(n1 + kk, __ldcg(xx + (uint64_t)q * n1 + kk));
     if constexpr (!WARP_LISTS)
         if (threadIdx.x == 0) { buf.cnt = 0; buf.have_thr = 0; buf.thr_s = INT64_MIN; buf.thr_i = 0xffffffffu; }
     __syncthreads();
@@ -1012,7 +1016,7 @@ decode_topk_kernel(const uint64_t* __restrict__ r, DecodeCorpus dc, const ScanSe
             uint64_t rv = 0;
             uint32_t id = 0;
             if (mine && valid) {
-                rv = r[ridx];
+                rv = __ldcg(r + ridx);
                 id = dc.ids ? dc.ids[gr] : (uint32_t)gr;
             }
             uint64_t part = 0;
@@ -1075,7 +1079,7 @@ decode_topk_kernel(const uint64_t* __restrict__ r, DecodeCorpus dc, const ScanSe
                 const uint64_t ridx = sg.out0 + (gr - sg.row0);
                 uint64_t rv = 0;
                 if (valid) {
-                    rv = r[ridx];
+                    rv = __ldcg(r + ridx);
                     id = dc.ids ? dc.ids[gr] : (uint32_t)gr;
                 }
                 uint64_t m_t = 0;
@@ -1699,8 +1703,16 @@ void launch_decode_topk(const uint64_t* d_r, const DecodeCorpus& dc, const ScanS
     auto fn = split ? (lists ? decode_topk_kernel<true, true> : decode_topk_kernel<false, true>)
                     : (lists ? decode_topk_kernel<true, false> : decode_topk_kernel<false, false>);
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * 2 * 512 * 16 + shares));
-    fn<<<total_ctas, DT_THREADS, dyn, s>>>(d_r, dc, d_segs, d_seg_unit, d_q, d_v, d_g, d_x, d_t, d_t_nnz, k, scratch,
-                                           d_mv_out, d_out_ids, d_out_scores, d_out_n, nq);
+    // A split decode is short, and its set-up is worth overlapping with the kernels
+    // before it (5,000 rows: 118 -> 105 us for the call with the whole chain).  A long
+    // one is not: started among the CTAs of the kernels before it, it lost more than
+    // the 3 us of set-up (four queries over 100,003 rows 1032 -> 1091 us).
+    if (split)
+        launch_after(fn, total_ctas, DT_THREADS, dyn, s, d_r, dc, d_segs, d_seg_unit, d_q, d_v, d_g, d_x, d_t, d_t_nnz, k,
+                     scratch, d_mv_out, d_out_ids, d_out_scores, d_out_n, nq);
+    else
+        fn<<<total_ctas, DT_THREADS, dyn, s>>>(d_r, dc, d_segs, d_seg_unit, d_q, d_v, d_g, d_x, d_t, d_t_nnz, k, scratch,
+                                               d_mv_out, d_out_ids, d_out_scores, d_out_n, nq);
 }
 
 void launch_topk_rows(const uint64_t* d_a, const uint64_t* d_b, const uint64_t* d_c, uint64_t ld, uint64_t rows,

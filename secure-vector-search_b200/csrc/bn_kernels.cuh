@@ -31,6 +31,33 @@
 
 namespace bn {
 
+// Programmatic dependent launch: a kernel launched by launch_after may become
+// resident while the kernel before it in the stream still runs, does what does not
+// depend on it (set-up, inputs that were complete before the run's first kernel,
+// which is launched plainly) and waits for its results in after_wait; every
+// kernel of such a chain waits, so each is complete before the next passes its own
+// wait.  Launched plainly, both calls do nothing.  after_go lets the next kernel of
+// the chain start its own set-up.  What the kernels before it wrote is read after
+// the wait through L2 (__ldcg or TMA): no load of it may be taken for an invariant
+// one and moved up.  One query over 5,000 rows (six kernels): 119 -> 105 us,
+// 100,000 rows 345 -> 337 us.
+__device__ __forceinline__ void after_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void after_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // Sliced-ELL entries of S (layout note above); ELL_TABLE entries of the
 // decode's signed table, the last one a zero past every valid entry.
 constexpr uint32_t ELL_PAD = 1024, ELL_NEG = 1025, ELL_TABLE = 2 * 1024 + 2;

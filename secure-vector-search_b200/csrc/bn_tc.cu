@@ -53,8 +53,10 @@ tc_ugen_kernel(const VerifySeg* __restrict__ vsegs, const TcBlock* __restrict__ 
     const uint32_t here = min((uint32_t)TC_ROWS, vs.rows - tb.i0);
     const ChaChaKey key = keys[vs.query];
     __shared__ uint64_t us[TC_MAX_TRIALS][UG_PAD];
+    after_go();
 
     // draws: 128 consecutive indices per trial span at most 17 keystream blocks
+    bool hit = false;
     for (uint32_t item = threadIdx.x; item < t_cnt * 17; item += blockDim.x) {
         const uint32_t tl = item / 17, bi = item % 17;
         const uint64_t first = draw_index(vs, t_base + tl, tb.i0);
@@ -69,11 +71,13 @@ tc_ugen_kernel(const VerifySeg* __restrict__ vsegs, const TcBlock* __restrict__ 
                 const uint32_t ii = (uint32_t)(idx - first);
                 uint64_t x = ((uint64_t)w[2 * q] | ((uint64_t)w[2 * q + 1] << 32)) & P;
                 if (ii >= here) x = 0;  // rows past the segment end
-                else if (x == P) { atomicOr(flags, DRAW_HIT_P); x = 0; }
+                else if (x == P) { hit = true; x = 0; }
                 us[tl][ug_idx(ii)] = x;
             }
         }
     }
+    after_wait();  // the draws need the seeds only; the flag word is cleared by the kernel before
+    if (hit) atomicOr(flags, DRAW_HIT_P);
     __syncthreads();
     // U tile image: row (t, b) holds byte b of u_t[i] for the 128 rows i.
     // Thread (t, chunk) reads its 16 draws once and writes all 8 byte rows.
@@ -661,6 +665,8 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_constan
     __syncthreads();
     tc_after();
     const uint32_t tmem = tmem_base_s;
+    after_go();
+    after_wait();
 
     if (warp == 0) {
         if (lane == 0) {  // ------------------------------------------ TMA producer
@@ -868,6 +874,8 @@ tc_rreduce_kernel(const VerifySeg* __restrict__ vsegs, const TcBlock* __restrict
     const uint32_t blk = blockIdx.x;
     const TcBlock tb = blocks[blk];
     const VerifySeg vs = vsegs[tb.seg];
+    after_go();
+    after_wait();
     const uint32_t i = threadIdx.x;
     const bool valid = tb.i0 + i < vs.rows;
     const uint64_t ri = vs.r0 + tb.i0 + i;
@@ -875,7 +883,7 @@ tc_rreduce_kernel(const VerifySeg* __restrict__ vsegs, const TcBlock* __restrict
     uint64_t rv = 0;
     if (valid) {
 #pragma unroll 8
-        for (uint32_t g = 0; g < groups; ++g) rv = add_mod(rv, r_part[(uint64_t)g * r_stride + ri]);
+        for (uint32_t g = 0; g < groups; ++g) rv = add_mod(rv, __ldcg(r_part + (uint64_t)g * r_stride + ri));
         r[ri] = rv;
     }
     rs[i] = rv;  // 0 past the segment's last row
@@ -887,7 +895,7 @@ tc_rreduce_kernel(const VerifySeg* __restrict__ vsegs, const TcBlock* __restrict
         const uint32_t t = warp + 4 * j;
 #pragma unroll
         for (int b = 0; b < 8; ++b)
-            w[j][b] = t < t_cnt ? *reinterpret_cast<const uint32_t*>(img + (uint64_t)(8 * t + b) * TC_ROWS) : 0u;
+            w[j][b] = t < t_cnt ? __ldcg(reinterpret_cast<const uint32_t*>(img + (uint64_t)(8 * t + b) * TC_ROWS)) : 0u;
     }
     __syncthreads();
     const uint64_t rr[4] = {rs[4 * lane], rs[4 * lane + 1], rs[4 * lane + 2], rs[4 * lane + 3]};
@@ -935,6 +943,8 @@ tc_finish_kernel(const uint64_t* __restrict__ z_part, const uint64_t* __restrict
     const uint32_t z_ctas = split > 1 ? FIN_CHUNKS : 1;
     __shared__ uint64_t sh[4];
     __shared__ int32_t last_s, first;
+    after_go();
+    after_wait();
     uint64_t part = 0;
     if (y < z_ctas) {
         const VerifySeg vs = vsegs[seg];
@@ -944,21 +954,21 @@ tc_finish_kernel(const uint64_t* __restrict__ z_part, const uint64_t* __restrict
             const uint32_t j = y * 128 + threadIdx.x;
             uint64_t z = 0;
 #pragma unroll 4
-            for (uint32_t p = p0 + sp; p < p1; p += split) z = add_mod(z, z_part[((uint64_t)p * trials + t) * N + j]);
+            for (uint32_t p = p0 + sp; p < p1; p += split) z = add_mod(z, __ldcg(z_part + ((uint64_t)p * trials + t) * N + j));
             part = mul_mod(z, v[j]);
         } else {
             uint64_t z[FIN_CHUNKS] = {};
             for (uint32_t p = p0; p < p1; ++p)
 #pragma unroll
                 for (int c = 0; c < FIN_CHUNKS; ++c)
-                    z[c] = add_mod(z[c], z_part[((uint64_t)p * trials + t) * N + c * 128 + threadIdx.x]);
+                    z[c] = add_mod(z[c], __ldcg(z_part + ((uint64_t)p * trials + t) * N + c * 128 + threadIdx.x));
 #pragma unroll
             for (int c = 0; c < FIN_CHUNKS; ++c) part = add_mod(part, mul_mod(z[c], v[c * 128 + threadIdx.x]));
         }
     } else {
         const uint32_t b0 = seg_block0[seg], b1 = seg_block0[seg + 1];
         for (uint32_t b = b0 + sp + split * threadIdx.x; b < b1; b += split * blockDim.x)
-            part = add_mod(part, ur_part[(uint64_t)b * trials + t]);
+            part = add_mod(part, __ldcg(ur_part + (uint64_t)b * trials + t));
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) part = add_mod(part, __shfl_xor_sync(FULLMASK, part, off));
@@ -1046,10 +1056,14 @@ cudaError_t make_tmap_u8_ksteps2(CUtensorMap* map, const void* base, uint64_t ro
 void launch_tc_ugen(const VerifySeg* d_vsegs, const TcBlock* d_blocks, uint32_t nblocks, const ChaChaKey* d_keys,
                     const uint64_t* d_r, uint32_t t_base, uint32_t t_cnt, uint32_t n_rows, uint8_t* d_u,
                     uint64_t* d_ur_part, uint32_t trials_total, uint32_t* d_flags, cudaStream_t s,
-                    uint64_t u_row_pitch) {
+                    uint64_t u_row_pitch, bool after) {
     if (!nblocks) return;
-    tc_ugen_kernel<<<nblocks, UG_THREADS, 0, s>>>(d_vsegs, d_blocks, d_keys, d_r, t_base, t_cnt, n_rows, d_u,
-                                                  u_row_pitch, d_ur_part, trials_total, d_flags);
+    if (after)
+        launch_after(tc_ugen_kernel, nblocks, UG_THREADS, 0, s, d_vsegs, d_blocks, d_keys, d_r, t_base, t_cnt, n_rows, d_u,
+                     u_row_pitch, d_ur_part, trials_total, d_flags);
+    else
+        tc_ugen_kernel<<<nblocks, UG_THREADS, 0, s>>>(d_vsegs, d_blocks, d_keys, d_r, t_base, t_cnt, n_rows, d_u,
+                                                      u_row_pitch, d_ur_part, trials_total, d_flags);
 }
 
 void launch_tc_freivalds(const CUtensorMap& tmap_m, const CUtensorMap& tmap_u, const TcPanel* d_panels,
@@ -1117,17 +1131,16 @@ void launch_tc_fused(const CUtensorMap& tmap_m, const CUtensorMap& tmap_u, const
     const uint32_t items = npanels * ((64 + FU_S - 1) / FU_S);
     const unsigned grid = items < (uint32_t)num_sms ? items : (unsigned)num_sms;
     cudaFuncSetAttribute(tc_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    tc_fused_kernel<<<grid, FU_THREADS, smem, s>>>(tmap_m, tmap_u, tmap_w, d_panels, npanels, d_vsegs, t_cnt, n_rows,
-                                                   trials_total, stages, stage_bytes, d_z_part, d_r_part, r_stride,
-                                                   d_err, wl);
+    launch_after(tc_fused_kernel, grid, FU_THREADS, smem, s, tmap_m, tmap_u, tmap_w, d_panels, npanels, d_vsegs, t_cnt,
+                 n_rows, trials_total, stages, stage_bytes, d_z_part, d_r_part, r_stride, d_err, wl);
 }
 
 void launch_tc_rreduce(const VerifySeg* d_vsegs, const TcBlock* d_blocks, uint32_t nblocks, const uint64_t* d_r_part,
                        uint64_t r_stride, uint32_t groups, const uint8_t* d_u, uint32_t t_cnt, uint32_t n_rows,
                        uint32_t trials_total, uint64_t* d_r, uint64_t* d_ur_part, cudaStream_t s) {
     if (!nblocks) return;
-    tc_rreduce_kernel<<<nblocks, TC_ROWS, 0, s>>>(d_vsegs, d_blocks, d_r_part, r_stride, groups, d_u, t_cnt, n_rows,
-                                                  trials_total, d_r, d_ur_part);
+    launch_after(tc_rreduce_kernel, nblocks, TC_ROWS, 0, s, d_vsegs, d_blocks, d_r_part, r_stride, groups, d_u, t_cnt,
+                 n_rows, trials_total, d_r, d_ur_part);
 }
 
 void launch_tc_finish(const uint64_t* d_z_part, const uint64_t* d_ur_part, const uint32_t* d_seg_panel0,
@@ -1139,10 +1152,10 @@ void launch_tc_finish(const uint64_t* d_z_part, const uint64_t* d_ur_part, const
     const uint32_t per_launch = 65535u / split;  // grid.z limit
     for (uint32_t s0 = 0; s0 < nseg; s0 += per_launch) {
         const uint32_t ns = nseg - s0 < per_launch ? nseg - s0 : per_launch;
-        tc_finish_kernel<<<dim3(trials, split > 1 ? FIN_CHUNKS + 1 : 2, ns * split), 128, 0, s>>>(
-            d_z_part, d_ur_part, d_seg_panel0 + s0, d_seg_block0 + s0, d_v_enc, d_vsegs + s0, trials, split,
-            d_chunks + (uint64_t)s0 * trials * (FIN_CHUNKS + 1) * split, d_done + s0, d_ur + (uint64_t)s0 * trials,
-            d_zv + (uint64_t)s0 * trials, d_failed + s0);
+        const dim3 grid(trials, split > 1 ? FIN_CHUNKS + 1 : 2, ns * split);
+        launch_after(tc_finish_kernel, grid, 128, 0, s, d_z_part, d_ur_part, d_seg_panel0 + s0, d_seg_block0 + s0, d_v_enc,
+                     d_vsegs + s0, trials, split, d_chunks + (uint64_t)s0 * trials * (FIN_CHUNKS + 1) * split, d_done + s0,
+                     d_ur + (uint64_t)s0 * trials, d_zv + (uint64_t)s0 * trials, d_failed + s0);
     }
 }
 

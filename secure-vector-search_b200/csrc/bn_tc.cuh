@@ -80,11 +80,12 @@ cudaError_t make_tmap_u8_ksteps2(CUtensorMap* map, const void* base, uint64_t ro
 // and u_t . r partial sums per block.  *flags bit 0: a draw hit p.
 // u_row_pitch = 0: per-block images (block b at d_u + b * n_rows * 128);
 // otherwise one flat image, row (t,b) at d_u + (t*8+b) * u_row_pitch and the
-// draw for r index x at byte column x (x = segment r0 + row).
+// draw for r index x at byte column x (x = segment r0 + row).  after: as the next
+// kernel of a launch_after chain (its draws then overlap the kernel before it).
 void launch_tc_ugen(const VerifySeg* d_vsegs, const TcBlock* d_blocks, uint32_t nblocks, const ChaChaKey* d_keys,
                     const uint64_t* d_r, uint32_t t_base, uint32_t t_cnt, uint32_t n_rows, uint8_t* d_u,
                     uint64_t* d_ur_part, uint32_t trials_total, uint32_t* d_flags, cudaStream_t s,
-                    uint64_t u_row_pitch = 0);
+                    uint64_t u_row_pitch = 0, bool after = false);
 
 // The GEMM + drain: z_part[panel][t_base + t][j] (canonical residues) for
 // t < t_cnt.  tmap_m: m_enc bytes {8192, rows}, box {128, 128}, swizzle 128B;
