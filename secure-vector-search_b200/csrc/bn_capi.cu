@@ -381,6 +381,29 @@ int keygen_lists(bn_ctx* ctx, uint32_t lists, const uint64_t* off, const uint8_t
 }
 
 // ------------------------------------------------------------------ pipeline
+// The z panels of every verify segment, `per` segments to a pass: a panel is listed
+// for the first segment of a group only and stands for the others' too (z partials
+// keep a place for every segment's panels, seg_panel0).
+void make_panels(HostMeta& hm, uint32_t per) {
+    hm.per = per;
+    hm.panels.clear();
+    hm.seg_panel0.assign(hm.vsegs.size() + 1, 0);
+    uint64_t max_blocks = 0;
+    for (const VerifySeg& v : hm.vsegs) max_blocks = std::max<uint64_t>(max_blocks, (v.rows + TC_ROWS - 1) / TC_ROWS);
+    const uint32_t panel_rows = tc_panel_rows(max_blocks, (hm.vsegs.size() + per - 1) / per);
+    uint32_t z0 = 0, tile0 = 0;  // next z partial and U tile
+    for (uint32_t s = 0; s < hm.vsegs.size(); ++s) {
+        const VerifySeg& v = hm.vsegs[s];
+        hm.seg_panel0[s] = z0;
+        for (uint64_t p0 = 0; p0 < v.rows; p0 += panel_rows, ++z0)
+            if (s % per == 0)
+                hm.panels.push_back(TcPanel{v.row0 + p0, (uint32_t)std::min<uint64_t>(panel_rows, v.rows - p0),
+                                            tile0 + (uint32_t)(p0 / TC_ROWS), s, z0});
+        if (s % per == 0) tile0 += (v.rows + TC_ROWS - 1) / TC_ROWS;
+    }
+    hm.seg_panel0.back() = z0;
+}
+
 void finish_meta(HostMeta& hm) {
     hm.seg_blk.assign(hm.segs.size() + 1, 0);
     hm.seg_unit.assign(hm.segs.size() + 1, 0);
@@ -390,23 +413,13 @@ void finish_meta(HostMeta& hm) {
         hm.seg_unit[i + 1] = hm.seg_unit[i] + (sg.rows ? ((sg.row0 + sg.rows - 1) >> 5) - (sg.row0 >> 5) + 1 : 0);
     }
     hm.blocks.clear();
-    hm.panels.clear();
     hm.seg_block0.assign(hm.vsegs.size() + 1, 0);
-    hm.seg_panel0.assign(hm.vsegs.size() + 1, 0);
-    uint64_t max_blocks = 0;
-    for (const VerifySeg& v : hm.vsegs) max_blocks = std::max<uint64_t>(max_blocks, (v.rows + TC_ROWS - 1) / TC_ROWS);
-    const uint32_t panel_rows = tc_panel_rows(max_blocks, hm.vsegs.size());
     for (uint32_t s = 0; s < hm.vsegs.size(); ++s) {
-        const VerifySeg& v = hm.vsegs[s];
         hm.seg_block0[s] = (uint32_t)hm.blocks.size();
-        hm.seg_panel0[s] = (uint32_t)hm.panels.size();
-        for (uint32_t i0 = 0; i0 < v.rows; i0 += TC_ROWS) hm.blocks.push_back(TcBlock{s, i0});
-        for (uint64_t p0 = 0; p0 < v.rows; p0 += panel_rows)
-            hm.panels.push_back(TcPanel{v.row0 + p0, (uint32_t)std::min<uint64_t>(panel_rows, v.rows - p0),
-                                        hm.seg_block0[s] + (uint32_t)(p0 / TC_ROWS), s, 0});
+        for (uint32_t i0 = 0; i0 < hm.vsegs[s].rows; i0 += TC_ROWS) hm.blocks.push_back(TcBlock{s, i0});
     }
     hm.seg_block0.back() = (uint32_t)hm.blocks.size();
-    hm.seg_panel0.back() = (uint32_t)hm.panels.size();
+    make_panels(hm, 1);
 }
 
 void flat_meta(uint64_t m, uint32_t B, HostMeta& hm) {
@@ -418,6 +431,7 @@ void flat_meta(uint64_t m, uint32_t B, HostMeta& hm) {
     }
     hm.total_out = (uint64_t)B * m;
     hm.max_rows = m;
+    hm.same_rows = true;
     finish_meta(hm);
 }
 
@@ -486,11 +500,11 @@ RunLayout make_layout(const Sizes& z, bool want_mv) {
 int make_tc_maps(const Sizes& z, const uint8_t* d_u, const uint8_t* d_w, TcMaps& maps) {
     if (z.engine != BN_ENGINE_TENSOR || !z.trials || !z.nblocks) return BN_OK;
     {
-        cudaError_t e = make_tmap_u8(&maps.w, d_w, 128, (uint64_t)z.B * 64 * 16, 128, WIMG_BOX_ROWS);
+        cudaError_t e = make_tmap_u8(&maps.w, d_w, 128, (uint64_t)z.B * 64 * 16, 128, tc_wimg_box(z.per));
         if (e != cudaSuccess) return fail(BN_ECUDA, "tensor map for the query images: %s", cudaGetErrorString(e));
     }
     for (uint32_t t0 = 0, ps = 0; t0 < z.trials; t0 += TC_MAX_TRIALS, ++ps) {
-        const uint32_t nr = pass_rows(std::min<uint32_t>(TC_MAX_TRIALS, z.trials - t0));
+        const uint32_t nr = pass_rows(z.per * std::min<uint32_t>(TC_MAX_TRIALS, z.trials - t0));
         cudaError_t e = make_tmap_u8(&maps.u[ps], d_u, TC_ROWS, z.nblocks * (uint64_t)nr, TC_ROWS, nr);
         if (e != cudaSuccess) return fail(BN_ECUDA, "tensor map for the Freivalds draws: %s", cudaGetErrorString(e));
     }
@@ -512,17 +526,17 @@ int enqueue_pipeline(bn_ctx* ctx, const Corpus& c, const Sizes& z, const Meta& m
         // One pass over m_enc yields r and the first <= 20 trials' z (tensor
         // cores); later passes of 20 trials reuse the now-known r.
         for (uint32_t t0 = 0, ps = 0; t0 < z.trials; t0 += TC_MAX_TRIALS, ++ps) {
-            const uint32_t tc = std::min<uint32_t>(TC_MAX_TRIALS, z.trials - t0), nr = pass_rows(tc);
+            const uint32_t tc = std::min<uint32_t>(TC_MAX_TRIALS, z.trials - t0), nr = pass_rows(z.per * tc);
             if (ps == 0) {
                 launch_tc_ugen(m.vsegs, m.tc_blocks, m.nblocks, keys, nullptr, t0, tc, nr, sc.u_buf, sc.ur_part,
-                               z.trials, sc.flags, s, 0, true);
+                               z.trials, sc.flags, s, 0, true, m.share);
                 if (prof0) CU(cudaEventRecord(prof0, s));
                 launch_tc_fused(c.tmap_m, m.maps->u[ps], m.maps->w, m.tc_panels, m.npanels, m.vsegs, tc, nr,
                                 z.trials, sc.z_part, sc.r_part, z.total_out, sc.err, ctx->num_sms, s,
-                                ctx->debug_wait_cycles);
+                                ctx->debug_wait_cycles, m.share);
                 if (prof1) CU(cudaEventRecord(prof1, s));
                 launch_tc_rreduce(m.vsegs, m.tc_blocks, m.nblocks, sc.r_part, z.total_out, tc_groups(nr), sc.u_buf, tc,
-                                  nr, z.trials, sc.r, sc.ur_part, s);
+                                  nr, z.trials, sc.r, sc.ur_part, s, m.share);
             } else {
                 launch_tc_ugen(m.vsegs, m.tc_blocks, m.nblocks, keys, sc.r, t0, tc, nr, sc.u_buf, sc.ur_part, z.trials,
                                sc.flags, s);
@@ -563,7 +577,9 @@ Meta meta_at(char* d, const RunLayout& o, const HostMeta& hm, const TcMaps* maps
                 reinterpret_cast<VerifySeg*>(d + o.vsegs), (uint32_t)hm.vsegs.size(),
                 reinterpret_cast<DecodeQuery*>(d + o.dq), reinterpret_cast<TcBlock*>(d + o.tc_blocks),
                 (uint32_t)hm.blocks.size(), reinterpret_cast<TcPanel*>(d + o.tc_panels), (uint32_t)hm.panels.size(),
-                reinterpret_cast<uint32_t*>(d + o.seg_panel0), reinterpret_cast<uint32_t*>(d + o.seg_block0), maps};
+                reinterpret_cast<uint32_t*>(d + o.seg_panel0), reinterpret_cast<uint32_t*>(d + o.seg_block0), maps,
+                hm.per == 1 ? TcShare{}
+                            : TcShare{hm.per, (uint32_t)hm.vsegs.size(), hm.seg_block0[1], hm.seg_panel0[1]}};
 }
 Scratch scratch_at(char* d, const RunLayout& o) {
     return Scratch{reinterpret_cast<QLimb*>(d + o.limbs), reinterpret_cast<uint64_t*>(d + o.x),
@@ -628,11 +644,13 @@ uint32_t assign_decode_ctas(HostMeta& hm, int sms) {
 }
 
 Sizes sizes_for(const Engine& e, HostMeta& hm, uint32_t B, uint32_t trials, uint32_t k) {
+    const uint32_t per = hm.same_rows && e.ctx->engine == BN_ENGINE_TENSOR ? tc_share(B, trials, hm.seg_block0[1]) : 1;
+    if (per != hm.per) make_panels(hm, per);
     return Sizes{B, e.c.n1, trials, k, assign_decode_ctas(hm, e.ctx->num_sms), hm.total_out,
-                 hm.segs.size(), hm.vsegs.size(), hm.blocks.size(), hm.panels.size(),
+                 hm.segs.size(), hm.vsegs.size(), hm.blocks.size(), hm.seg_panel0.back(),
                  plan_freivalds(std::max<uint64_t>(hm.max_rows, 1), (uint32_t)std::max<size_t>(hm.vsegs.size(), 1),
                                 e.ctx->num_sms),
-                 e.ctx->engine};
+                 e.ctx->engine, per};
 }
 
 // One pipeline run over host inputs, split so that a caller can keep several

@@ -254,6 +254,7 @@ struct Meta {  // device pointers (+ host tensor maps)
     const uint32_t* seg_panel0;
     const uint32_t* seg_block0;
     const TcMaps* maps;
+    TcShare share;
 };
 struct Scratch {  // device pointers
     QLimb* limbs;
@@ -299,6 +300,8 @@ struct HostMeta {
     std::vector<TcPanel> panels;        // 4096-row panels of every verify segment
     std::vector<uint32_t> seg_block0, seg_panel0;
     uint64_t total_out = 0, max_rows = 0;
+    bool same_rows = false;  // every segment is the same rows for the next query (flat_meta)
+    uint32_t per = 1;        // queries per pass that `panels` is laid out for (share_passes)
 };
 
 struct Sizes {
@@ -306,6 +309,7 @@ struct Sizes {
     uint64_t total_out, nseg, nvseg, nblocks, npanels;
     FreivaldsPlan fp;  // CUDA-core engine
     int engine;        // BN_ENGINE_*
+    uint32_t per = 1;  // queries per fused pass (TcShare)
 };
 
 

@@ -42,11 +42,19 @@ __device__ __forceinline__ void transpose_bytes4(const uint32_t w[4], uint32_t& 
     o3 = __byte_perm(t2, t3, 0x7632);
 }
 
+// The U tile of a block's group and its first row in it.
+__device__ __forceinline__ uint64_t u_tile_off(const TcBlock& tb, uint32_t blk, uint32_t t_cnt, uint32_t n_rows,
+                                               const TcShare& sh) {
+    if (sh.per == 1) return (uint64_t)blk * n_rows * TC_ROWS;
+    const uint32_t tile = tb.seg / sh.per * sh.blocks + tb.i0 / TC_ROWS;
+    return ((uint64_t)tile * n_rows + tb.seg % sh.per * t_cnt * 8) * TC_ROWS;
+}
+
 __global__ void __launch_bounds__(UG_THREADS)
 tc_ugen_kernel(const VerifySeg* __restrict__ vsegs, const TcBlock* __restrict__ blocks, const ChaChaKey* __restrict__ keys,
                const uint64_t* __restrict__ r, uint32_t t_base, uint32_t t_cnt, uint32_t n_rows,
                uint8_t* __restrict__ u_out, uint64_t u_row_pitch, uint64_t* __restrict__ ur_part,
-               uint32_t trials_total, uint32_t* __restrict__ flags) {
+               uint32_t trials_total, uint32_t* __restrict__ flags, TcShare share) {
     const uint32_t blk = blockIdx.x;
     const TcBlock tb = blocks[blk];
     const VerifySeg vs = vsegs[tb.seg];
@@ -84,7 +92,7 @@ tc_ugen_kernel(const VerifySeg* __restrict__ vsegs, const TcBlock* __restrict__ 
     // per-block image: rows of 128 bytes, blocks n_rows * 128 apart; flat
     // image: rows u_row_pitch apart, this block at byte column r0 + i0
     const uint64_t pitch = u_row_pitch ? u_row_pitch : TC_ROWS;
-    uint8_t* dst = u_row_pitch ? u_out + vs.r0 + tb.i0 : u_out + (uint64_t)blk * n_rows * TC_ROWS;
+    uint8_t* dst = u_row_pitch ? u_out + vs.r0 + tb.i0 : u_out + u_tile_off(tb, blk, t_cnt, n_rows, share);
     for (uint32_t c = threadIdx.x; c < t_cnt * (TC_ROWS / 16); c += blockDim.x) {
         const uint32_t tl = c / (TC_ROWS / 16), ch = c % (TC_ROWS / 16);
         uint32_t pl[8][4];  // pl[b][j]: byte b of draws 4j .. 4j + 3
@@ -105,8 +113,11 @@ tc_ugen_kernel(const VerifySeg* __restrict__ vsegs, const TcBlock* __restrict__ 
             reinterpret_cast<uint4*>(dst + (uint64_t)(tl * 8 + b) * pitch)[ch] =
                 make_uint4(pl[b][0], pl[b][1], pl[b][2], pl[b][3]);
     }
-    for (uint32_t c = threadIdx.x; c < (n_rows - 8 * t_cnt) * (TC_ROWS / 16); c += blockDim.x) {  // zero pad rows
-        const uint32_t row = 8 * t_cnt + c / (TC_ROWS / 16), ch = c % (TC_ROWS / 16);
+    // zero pad rows, by the group's first segment (a smaller last group's tiles keep
+    // whatever is in the absent queries' rows: their columns are not read)
+    const uint32_t used = 8 * t_cnt * share.per, pad = tb.seg % share.per ? 0 : n_rows - used;
+    for (uint32_t c = threadIdx.x; c < pad * (TC_ROWS / 16); c += blockDim.x) {
+        const uint32_t row = used + c / (TC_ROWS / 16), ch = c % (TC_ROWS / 16);
         reinterpret_cast<uint4*>(dst + (uint64_t)row * pitch)[ch] = make_uint4(0, 0, 0, 0);
     }
     // u_t . r over this block's rows (skipped when r is not known yet)
@@ -171,11 +182,27 @@ __device__ __forceinline__ void z_drain32(uint32_t taddr, uint32_t lane, uint32_
     if ((a & 1) == 0 && t < t_cnt) z_out[(uint64_t)t * N + j] = canon(k1);
 }
 
+// Where z_t[j] of a work item goes: trial t at t * N, or, when `tq` trials each of
+// several queries lie side by side, query t / tq's panel `extra` words further per query.
+struct ZOut {
+    uint64_t* p;
+    __device__ __forceinline__ uint64_t* operator()(uint32_t t) const { return p + (uint64_t)t * N; }
+};
+struct ZOutShared {
+    uint64_t* p;
+    uint32_t inv;    // 65536 / tq + 1: t / tq = t * inv >> 16 for t < TC_MAX_TRIALS
+    uint64_t extra;
+    __device__ __forceinline__ uint64_t* operator()(uint32_t t) const {
+        return p + (uint64_t)t * N + (t * inv >> 16) * extra;
+    }
+};
+
 // One 64-column chunk (8 trials) of a strip: lane (xi, a) folds its 8
 // trials' byte products to (lo + hi 2^32) 2^(8a) mod p, a butterfly over the
 // 8 lanes of one element leaves lane a with trial c0/8 + a's sum.
+template <class Out>
 __device__ __forceinline__ void z_drain64(uint32_t taddr, uint32_t lane, uint32_t j, uint32_t c0, uint32_t t_cnt,
-                                          uint64_t* __restrict__ z_out) {
+                                          const Out& z_out) {
     const uint32_t a = lane & 7;
     const uint32_t w1 = 8 * a;
     const bool b2 = (a & 4) != 0, b1 = (a & 2) != 0, b0 = (a & 1) != 0;
@@ -201,12 +228,13 @@ __device__ __forceinline__ void z_drain64(uint32_t taddr, uint32_t lane, uint32_
         k2[i] = (b1 ? k4[i + 2] : k4[i]) + __shfl_xor_sync(FULLMASK, b1 ? k4[i] : k4[i + 2], 2);
     const uint64_t z = canon((b0 ? k2[1] : k2[0]) + __shfl_xor_sync(FULLMASK, b0 ? k2[0] : k2[1], 1));
     const uint32_t t = c0 / 8 + a;
-    if (t < t_cnt) z_out[(uint64_t)t * N + j] = z;
+    if (t < t_cnt) z_out(t)[j] = z;
 }
 
 // One 16-column chunk (2 trials) of a strip: plain 3-level reduction.
+template <class Out>
 __device__ __forceinline__ void z_drain16(uint32_t taddr, uint32_t lane, uint32_t j, uint32_t c0, uint32_t t_cnt,
-                                          uint64_t* __restrict__ z_out) {
+                                          const Out& z_out) {
     const uint32_t a = lane & 7;
     const uint32_t w1 = 8 * a;
     uint32_t v[16];
@@ -224,7 +252,7 @@ __device__ __forceinline__ void z_drain16(uint32_t taddr, uint32_t lane, uint32_
         zc += __shfl_xor_sync(FULLMASK, zc, 1);
         zc += __shfl_xor_sync(FULLMASK, zc, 2);
         zc += __shfl_xor_sync(FULLMASK, zc, 4);
-        if (a == 0 && t < t_cnt) z_out[(uint64_t)t * N + j] = canon(zc);
+        if (a == 0 && t < t_cnt) z_out(t)[j] = canon(zc);
     }
 }
 
@@ -233,9 +261,10 @@ __device__ __forceinline__ void z_drain16(uint32_t taddr, uint32_t lane, uint32_
 // (element j = lane / 8, byte a = lane % 8) and columns (t, b) (trial t, byte
 // b of u_t).  Warp (lane quarter q, half) reads every other 64-column chunk,
 // then every other 16-column remainder chunk.
-// z_out[t * N + j] receives z_t[j] for t < t_cnt.
+// z_out(t)[j] receives z_t[j] for t < t_cnt.
+template <class Out>
 __device__ __forceinline__ void z_drain(uint32_t tmem, uint32_t q, uint32_t half, uint32_t lane, uint32_t sg,
-                                        uint32_t strip0, uint32_t n_rows, uint32_t t_cnt, uint64_t* __restrict__ z_out) {
+                                        uint32_t strip0, uint32_t n_rows, uint32_t t_cnt, const Out& z_out) {
     const uint32_t jl = q * 4 + (lane >> 3);
     const uint32_t wide = n_rows & ~63u;
     for (uint32_t s = 0; s < sg; ++s) {
@@ -380,7 +409,8 @@ tc_freivalds_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_con
             if (!ok && lane == 0) { abort_s = 1; atomicOr(err, 16u); }
             if (__any_sync(FULLMASK, !ok || abort_s)) { stop = true; break; }
             tc_after();
-            z_drain(tmem, q, half, lane, sg, g * S, n_rows, t_cnt, z_part + ((uint64_t)p * trials_total + t_base) * N);
+            z_drain(tmem, q, half, lane, sg, g * S, n_rows, t_cnt,
+                    ZOut{z_part + ((uint64_t)p * trials_total + t_base) * N});
             tc_before();
             __syncwarp();
             if (lane == 0) bar_arrive(&acce_b);
@@ -574,7 +604,7 @@ tc_freivalds_small_kernel(const __grid_constant__ CUtensorMap tmap_m, const __gr
                 const uint32_t j = s * 16 + jl;
                 for (uint32_t k = part; k < tasks; k += SM_DRAIN_PARTS) {
                     if (32 * k + 32 <= n_rows) z_drain32(tbase + 32 * k, lane, j, 32 * k, t_cnt, z_out);
-                    else z_drain16(tbase + 32 * k, lane, j, 32 * k, t_cnt, z_out);
+                    else z_drain16(tbase + 32 * k, lane, j, 32 * k, t_cnt, ZOut{z_out});
                 }
                 tc_before();
                 __syncwarp();
@@ -603,22 +633,29 @@ tc_freivalds_small_kernel(const __grid_constant__ CUtensorMap tmap_m, const __gr
 //      E is per stage (new rows every stage): two 16-column TMEM buffers at
 //      column 480 alternate, and four drain warps turn each into r partials
 //      r_part[group][r index] while the next stage accumulates.
+// Several queries over the same rows (TcShare) take the pass together: their
+// draws are the U tile's rows (slot, t, b), their images the r MMA's columns
+// (slot, s), with E buffers of 16 columns per query from column 512 - 32 per.
+// Bytes of m_enc bound the pass, so four queries at 3 trials cost what one does.
 // The z and r MMAs are issued by two warps (1 and FU_R_WARP), so neither
 // instruction stream waits for the other; a stage is free once the z issuer
-// has committed and a drain warp has seen the stage's r MMAs complete.  TMEM: z in columns [0, 3 n_rows) (n_rows <= 160), E in [480, 512).
+// has committed and a drain warp has seen the stage's r MMAs complete.  TMEM: z in columns [0, 3 n_rows) (n_rows <= 160), E behind.
 constexpr int FU_S = 3;
 constexpr int FU_DRAIN_WARPS = 4;
 constexpr int FU_R_WARP = 2 + TC_EPI_WARPS + FU_DRAIN_WARPS;           // issues the r MMAs
 constexpr int FU_THREADS = TC_THREADS + 32 * (FU_DRAIN_WARPS + 1);  // 480
-constexpr uint32_t FU_E_COL = 480;
 constexpr uint32_t W_STRIP_BYTES = 16 * 128;  // one strip's 16 diagonal rows
 
+// SHARED: several queries take the pass together (with the sizes of a group left
+// to run time, a single query took 0.7 % longer).
+template <bool SHARED>
 __global__ void __launch_bounds__(FU_THREADS, 1)
 tc_fused_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_constant__ CUtensorMap tmap_u,
                 const __grid_constant__ CUtensorMap tmap_w, const TcPanel* __restrict__ panels, uint32_t npanels,
                 const VerifySeg* __restrict__ vsegs, uint32_t t_cnt, uint32_t n_rows, uint32_t trials_total,
-                uint32_t stages, uint32_t stage_bytes, uint64_t* __restrict__ z_part, uint64_t* __restrict__ r_part,
-                uint64_t r_stride, uint32_t* __restrict__ err, long long wait_limit) {
+                uint32_t stages, uint32_t stage_bytes, uint32_t w_bufs_, uint64_t* __restrict__ z_part,
+                uint64_t* __restrict__ r_part, uint64_t r_stride, uint32_t* __restrict__ err, long long wait_limit,
+                TcShare share) {
     constexpr int S = FU_S;
     extern __shared__ uint8_t tc_dyn[];
     __shared__ uint64_t full_b[4], empty_b[4], accf_b, acce_b, done_b, racc_b[2], rfree_b[2], wfull_b[2], wfree_b[2];
@@ -630,10 +667,13 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_constan
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t u_off = S * STRIP_BYTES;
     const uint32_t u_bytes = n_rows * TC_ROWS;
-    // the query's diagonal image of an item's strip group: loaded once per item
-    // into one of two buffers behind the stage ring (1024-aligned: stage_bytes
-    // and w_bytes are multiples of 1024)
-    const uint32_t w_bytes = S * W_STRIP_BYTES;
+    // the queries' diagonal images of an item's strip group, [strip][query][16 rows]:
+    // loaded once per item into one of w_bufs (1 or 2) buffers behind the stage ring
+    // (1024-aligned: stage_bytes and w_bytes are multiples of 1024)
+    const uint32_t per = SHARED ? share.per : 1, w_bufs = SHARED ? w_bufs_ : 2;
+    const uint32_t w_strip = per * W_STRIP_BYTES, w_bytes = S * w_strip, w_sh = w_bufs - 1;
+    const uint32_t e_col = 512 - 32 * per;  // two row-product buffers of 16 columns per query
+    auto queries = [&](const TcPanel& pn) { return SHARED ? min(per, share.nseg - pn.seg) : 1u; };
     const uint32_t w_ring = stages * stage_bytes;
     const uint32_t groups = (64 + S - 1) / S;
     const uint32_t items = npanels * groups;
@@ -679,15 +719,25 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_constan
                 const uint32_t query = vsegs[pn.seg].query;
                 const uint32_t nrb = (pn.rows + TC_ROWS - 1) / TC_ROWS;
                 const uint32_t sg = min((uint32_t)S, 64u - g * S);
-                const uint32_t ib = ic & 1;  // W buffer of this item: free once item ic - 2's r MMAs are done
-                if (ic >= 2 && !bar_wait(&wfree_b[ib], ((ic >> 1) - 1) & 1, wait_limit)) {
+                const uint32_t ib = ic & w_sh;  // W buffer of this item: free once item ic - w_bufs's r MMAs are done
+                if (ic >= w_bufs && !bar_wait(&wfree_b[ib], ((ic >> w_sh) - 1) & 1, wait_limit)) {
                     abort_s = 1;
                     atomicOr(err, 4u);
                     break;
                 }
                 if (abort_s) break;
-                bar_expect_tx(&wfull_b[ib], w_bytes);
-                tma_2d(ring + w_ring + ib * w_bytes, &tmap_w, 0, (int)((query * 64 + g * S) * 16), &wfull_b[ib]);
+                uint8_t* wd = ring + w_ring + ib * w_bytes;
+                if (!SHARED) {
+                    bar_expect_tx(&wfull_b[ib], w_bytes);
+                    tma_2d(wd, &tmap_w, 0, (int)((query * 64 + g * S) * 16), &wfull_b[ib]);
+                } else {
+                    const uint32_t qn = queries(pn);
+                    bar_expect_tx(&wfull_b[ib], sg * qn * W_STRIP_BYTES);
+                    for (uint32_t s = 0; s < sg; ++s)
+                        for (uint32_t c = 0; c < qn; ++c)
+                            tma_2d(wd + s * w_strip + c * W_STRIP_BYTES, &tmap_w, 0,
+                                   (int)(((query + c) * 64 + g * S + s) * 16), &wfull_b[ib]);
+                }
                 ++w_issued;
                 for (uint32_t rb = 0; rb < nrb; ++rb, ++it) {
                     const uint32_t st = (uint32_t)(it % stages);
@@ -710,8 +760,8 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_constan
             // the last ring stages and the W images of the last two items
             for (uint64_t j = it > stages ? it - stages : 0; j < it; ++j)
                 bar_wait(&full_b[j % stages], (uint32_t)((j / stages) & 1));
-            for (uint32_t x = w_issued > 2 ? w_issued - 2 : 0; x < w_issued; ++x)
-                bar_wait(&wfull_b[x & 1], (x >> 1) & 1);
+            for (uint32_t x = w_issued > w_bufs ? w_issued - w_bufs : 0; x < w_issued; ++x)
+                bar_wait(&wfull_b[x & w_sh], (x >> w_sh) & 1);
         }
     } else if (warp == 1) {
         if (lane == 0) {  // ------------------------------------------ z MMA issuer
@@ -754,7 +804,7 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_constan
         }
     } else if (warp == FU_R_WARP) {
         if (lane == 0) {  // ------------------------------------------ r MMA issuer
-            const uint32_t idesc_r = (2u << 4) | ((16u >> 3) << 17) | ((uint32_t)(TC_ROWS >> 4) << 24);
+            const uint32_t idesc_r = (2u << 4) | ((16u * per >> 3) << 17) | ((uint32_t)(TC_ROWS >> 4) << 24);
             uint64_t it = 0;
             uint32_t ic = 0;
             bool stop = false;
@@ -763,8 +813,8 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_constan
                 const TcPanel pn = panels[p];
                 const uint32_t nrb = (pn.rows + TC_ROWS - 1) / TC_ROWS;
                 const uint32_t sg = min((uint32_t)S, 64u - g * S);
-                const uint32_t ib = ic & 1;
-                if (!bar_wait(&wfull_b[ib], (ic >> 1) & 1, wait_limit) || abort_s) {
+                const uint32_t ib = ic & w_sh;
+                if (!bar_wait(&wfull_b[ib], (ic >> w_sh) & 1, wait_limit) || abort_s) {
                     abort_s = 1;
                     atomicOr(err, 8u);
                     break;
@@ -784,8 +834,8 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_constan
                     for (uint32_t s = 0; s < sg; ++s)
 #pragma unroll
                         for (uint32_t ks = 0; ks < TC_ROWS / 32; ++ks)  // strip read K-major
-                            mma_i8(tmem + FU_E_COL + 16 * eb, sdesc(sb + s * STRIP_BYTES + ks * 32u, 16, 1024),
-                                   sdesc(wb + s * W_STRIP_BYTES + ks * 32u, 16, 1024), idesc_r, (s | ks) != 0);
+                            mma_i8(tmem + e_col + 16 * per * eb, sdesc(sb + s * STRIP_BYTES + ks * 32u, 16, 1024),
+                                   sdesc(wb + s * w_strip + ks * 32u, 16, 1024), idesc_r, (s | ks) != 0);
                     mma_commit(&racc_b[eb]);  // the stage's row products are ready (and its strips read)
                 }
                 if (stop) break;
@@ -798,6 +848,9 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_constan
         // ---------------------------------------------------------- TMEM epilogue (z)
         const uint32_t q = (uint32_t)(warp & 3);
         const uint32_t half = (uint32_t)(warp - 2) >> 2;
+        // from a query's z partials of a panel to the next query's
+        const uint32_t z_inv = 65536u / t_cnt + 1;
+        const uint64_t z_extra = ((uint64_t)share.panels * trials_total - t_cnt) * N;
         uint64_t gc = 0;
         for (uint32_t item = blockIdx.x; item < items; item += gridDim.x, ++gc) {
             const uint32_t p = item / groups, g = item % groups;
@@ -806,7 +859,12 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_constan
             if (!ok && lane == 0) { abort_s = 1; atomicOr(err, 16u); }
             if (__any_sync(FULLMASK, !ok || abort_s)) break;
             tc_after();
-            z_drain(tmem, q, half, lane, sg, g * S, n_rows, t_cnt, z_part + (uint64_t)p * trials_total * N);
+            const TcPanel pn = panels[p];
+            if constexpr (SHARED)
+                z_drain(tmem, q, half, lane, sg, g * S, n_rows, queries(pn) * t_cnt,
+                        ZOutShared{z_part + (uint64_t)pn.z0 * trials_total * N, z_inv, z_extra});
+            else
+                z_drain(tmem, q, half, lane, sg, g * S, n_rows, t_cnt, ZOut{z_part + (uint64_t)p * trials_total * N});
             tc_before();
             __syncwarp();
             if (lane == 0) bar_arrive(&acce_b);
@@ -826,6 +884,7 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_constan
             const VerifySeg vs = vsegs[pn.seg];
             const uint32_t nrb = (pn.rows + TC_ROWS - 1) / TC_ROWS;
             const uint64_t r0 = vs.r0 + (pn.row0 - vs.row0);  // r index of the panel's first row
+            const uint32_t qn = queries(pn);
             for (uint32_t rb = 0; rb < nrb; ++rb, ++it) {
                 const uint32_t eb = (uint32_t)(it & 1);
                 const bool ok = __all_sync(FULLMASK, bar_wait(&racc_b[eb], (uint32_t)((it >> 1) & 1), wait_limit));
@@ -836,19 +895,23 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmap_m, const __grid_constan
                 // stage for the r issuer)
                 if (q == 0 && lane == 0) bar_arrive(&empty_b[it % stages]);
                 tc_after();
-                uint32_t v[16];
-                tmem_ld16(tmem + ((q * 32) << 16) + FU_E_COL + 16 * eb, v);
-                tc_before();
-                __syncwarp();
-                if (lane == 0) bar_arrive(&rfree_b[eb]);  // the buffer may take stage it + 2
-                uint64_t gsum[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    gsum[k] = (uint64_t)v[4 * k] + ((uint64_t)v[4 * k + 1] << 8) + ((uint64_t)v[4 * k + 2] << 16) +
-                              ((uint64_t)v[4 * k + 3] << 24);
-                const uint64_t rv = canon(gsum[0] + rotl61(gsum[1], 32) + rotl61(gsum[2], 3) + rotl61(gsum[3], 35));
                 const uint32_t lr = rb * TC_ROWS + rr;
-                if (lr < pn.rows) r_part[(uint64_t)g * r_stride + r0 + lr] = rv;
+                for (uint32_t c = 0; c < qn; ++c) {
+                    uint32_t v[16];
+                    tmem_ld16(tmem + ((q * 32) << 16) + e_col + 16 * (per * eb + c), v);
+                    if (c + 1 == qn) {
+                        tc_before();
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(&rfree_b[eb]);  // the buffer may take stage it + 2
+                    }
+                    uint64_t gsum[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        gsum[k] = (uint64_t)v[4 * k] + ((uint64_t)v[4 * k + 1] << 8) + ((uint64_t)v[4 * k + 2] << 16) +
+                                  ((uint64_t)v[4 * k + 3] << 24);
+                    const uint64_t rv = canon(gsum[0] + rotl61(gsum[1], 32) + rotl61(gsum[2], 3) + rotl61(gsum[3], 35));
+                    if (lr < pn.rows) r_part[(uint64_t)g * r_stride + r0 + (uint64_t)c * vs.rows + lr] = rv;
+                }
             }
         }
     }
@@ -869,7 +932,7 @@ __global__ void __launch_bounds__(TC_ROWS)
 tc_rreduce_kernel(const VerifySeg* __restrict__ vsegs, const TcBlock* __restrict__ blocks,
                   const uint64_t* __restrict__ r_part, uint64_t r_stride, uint32_t groups,
                   const uint8_t* __restrict__ u_img, uint32_t t_cnt, uint32_t n_rows, uint32_t trials_total,
-                  uint64_t* __restrict__ r, uint64_t* __restrict__ ur_part) {
+                  uint64_t* __restrict__ r, uint64_t* __restrict__ ur_part, TcShare share) {
     constexpr int TPW = TC_MAX_TRIALS / (TC_ROWS / 32);  // trials per warp
     const uint32_t blk = blockIdx.x;
     const TcBlock tb = blocks[blk];
@@ -888,7 +951,7 @@ tc_rreduce_kernel(const VerifySeg* __restrict__ vsegs, const TcBlock* __restrict
     }
     rs[i] = rv;  // 0 past the segment's last row
     const int warp = i >> 5, lane = i & 31;
-    const uint8_t* img = u_img + (uint64_t)blk * n_rows * TC_ROWS + 4 * lane;
+    const uint8_t* img = u_img + u_tile_off(tb, blk, t_cnt, n_rows, share) + 4 * lane;
     uint32_t w[TPW][8];
 #pragma unroll
     for (int j = 0; j < TPW; ++j) {
@@ -1056,14 +1119,14 @@ cudaError_t make_tmap_u8_ksteps2(CUtensorMap* map, const void* base, uint64_t ro
 void launch_tc_ugen(const VerifySeg* d_vsegs, const TcBlock* d_blocks, uint32_t nblocks, const ChaChaKey* d_keys,
                     const uint64_t* d_r, uint32_t t_base, uint32_t t_cnt, uint32_t n_rows, uint8_t* d_u,
                     uint64_t* d_ur_part, uint32_t trials_total, uint32_t* d_flags, cudaStream_t s,
-                    uint64_t u_row_pitch, bool after) {
+                    uint64_t u_row_pitch, bool after, TcShare share) {
     if (!nblocks) return;
     if (after)
         launch_after(tc_ugen_kernel, nblocks, UG_THREADS, 0, s, d_vsegs, d_blocks, d_keys, d_r, t_base, t_cnt, n_rows, d_u,
-                     u_row_pitch, d_ur_part, trials_total, d_flags);
+                     u_row_pitch, d_ur_part, trials_total, d_flags, share);
     else
         tc_ugen_kernel<<<nblocks, UG_THREADS, 0, s>>>(d_vsegs, d_blocks, d_keys, d_r, t_base, t_cnt, n_rows, d_u,
-                                                      u_row_pitch, d_ur_part, trials_total, d_flags);
+                                                      u_row_pitch, d_ur_part, trials_total, d_flags, share);
 }
 
 void launch_tc_freivalds(const CUtensorMap& tmap_m, const CUtensorMap& tmap_u, const TcPanel* d_panels,
@@ -1120,27 +1183,32 @@ void launch_tc_freivalds_small(const CUtensorMap& tmap_m, const CUtensorMap& tma
 void launch_tc_fused(const CUtensorMap& tmap_m, const CUtensorMap& tmap_u, const CUtensorMap& tmap_w,
                      const TcPanel* d_panels, uint32_t npanels, const VerifySeg* d_vsegs, uint32_t t_cnt,
                      uint32_t n_rows, uint32_t trials_total, uint64_t* d_z_part, uint64_t* d_r_part, uint64_t r_stride,
-                     uint32_t* d_err, int num_sms, cudaStream_t s, long long wait_cycles) {
+                     uint32_t* d_err, int num_sms, cudaStream_t s, long long wait_cycles, TcShare share) {
     if (!npanels) return;
     const long long wl = wait_cycles > 0 ? wait_cycles : TC_WAIT_CYCLES;
     const uint32_t stage_bytes = (uint32_t)FU_S * STRIP_BYTES + ((n_rows * TC_ROWS + 1023u) & ~1023u);
-    const uint32_t w_two = 2u * FU_S * W_STRIP_BYTES;  // the two per-item W buffers
-    uint32_t stages = (227u * 1024u - 2048u - w_two) / stage_bytes;
+    // two per-item W buffers, or one where the second would cost the third stage
+    // (an item's image then waits for the last row products of the item before,
+    // while that one's z drain runs)
+    const uint32_t w_bytes = FU_S * share.per * W_STRIP_BYTES, room = 227u * 1024u - 2048u;
+    const uint32_t w_bufs = (room - 2 * w_bytes) / stage_bytes >= 3 ? 2 : 1;
+    uint32_t stages = (room - w_bufs * w_bytes) / stage_bytes;
     stages = stages < 2 ? 2 : (stages > 4 ? 4 : stages);
-    const int smem = (int)(stages * stage_bytes + w_two + 1024);
+    const int smem = (int)(stages * stage_bytes + w_bufs * w_bytes + 1024);
     const uint32_t items = npanels * ((64 + FU_S - 1) / FU_S);
     const unsigned grid = items < (uint32_t)num_sms ? items : (unsigned)num_sms;
-    cudaFuncSetAttribute(tc_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    launch_after(tc_fused_kernel, grid, FU_THREADS, smem, s, tmap_m, tmap_u, tmap_w, d_panels, npanels, d_vsegs, t_cnt,
-                 n_rows, trials_total, stages, stage_bytes, d_z_part, d_r_part, r_stride, d_err, wl);
+    auto fn = share.per > 1 ? tc_fused_kernel<true> : tc_fused_kernel<false>;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    launch_after(fn, grid, FU_THREADS, smem, s, tmap_m, tmap_u, tmap_w, d_panels, npanels, d_vsegs, t_cnt,
+                 n_rows, trials_total, stages, stage_bytes, w_bufs, d_z_part, d_r_part, r_stride, d_err, wl, share);
 }
 
 void launch_tc_rreduce(const VerifySeg* d_vsegs, const TcBlock* d_blocks, uint32_t nblocks, const uint64_t* d_r_part,
                        uint64_t r_stride, uint32_t groups, const uint8_t* d_u, uint32_t t_cnt, uint32_t n_rows,
-                       uint32_t trials_total, uint64_t* d_r, uint64_t* d_ur_part, cudaStream_t s) {
+                       uint32_t trials_total, uint64_t* d_r, uint64_t* d_ur_part, cudaStream_t s, TcShare share) {
     if (!nblocks) return;
     launch_after(tc_rreduce_kernel, nblocks, TC_ROWS, 0, s, d_vsegs, d_blocks, d_r_part, r_stride, groups, d_u, t_cnt,
-                 n_rows, trials_total, d_r, d_ur_part);
+                 n_rows, trials_total, d_r, d_ur_part, share);
 }
 
 void launch_tc_finish(const uint64_t* d_z_part, const uint64_t* d_ur_part, const uint32_t* d_seg_panel0,

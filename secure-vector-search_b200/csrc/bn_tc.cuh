@@ -49,14 +49,44 @@ inline uint32_t tc_panel_rows(uint64_t blocks, uint64_t nseg) {
 }
 
 // One panel of a verify segment: rows [row0, row0 + rows) of m_enc, whose U
-// tiles start at row block `rb0` of the U buffer.
+// tiles start at row block `rb0` of the U buffer.  z0 (fused pass): the index of
+// its z partials.
 struct TcPanel {
     uint64_t row0;
     uint32_t rows;
     uint32_t rb0;
     uint32_t seg;
-    uint32_t pad;
+    uint32_t z0;
 };
+
+// Queries that take one pass over the same rows together (fused pass): `per`
+// consecutive segments with equal rows, whose r indices follow one another, form a
+// group; the last group may be smaller.  Their draws lie side by side in the group's U
+// tiles (rows (slot, t, b)), and a panel of the group's first segment stands for
+// all of them.  per = 1: every segment by itself.
+struct TcShare {
+    uint32_t per = 1;
+    uint32_t nseg = 0;    // segments in all
+    uint32_t blocks = 0;  // row blocks of a segment
+    uint32_t panels = 0;  // panels of a segment
+};
+
+// Queries per group for nq queries over the same `blocks` row blocks at `trials`
+// trials each: as many as fit the trial slots of a pass and, beside their z
+// accumulators, two 16-column row-product buffers each in TMEM (3 n_rows + 32 per <=
+// 512); then groups of even size.  One pass over m_enc costs about the same for one
+// query at 20 trials and for four at 3: four queries over 100,003 rows 1028 -> 640
+// us, over 2,000 rows 117 -> 107.  Below TC_SHARE_BLOCKS a pass each fits on
+// SMs that would be idle (500 rows, five queries: 99 against 104 us).
+constexpr uint32_t TC_SHARE_BLOCKS = 16;
+inline uint32_t tc_share(uint32_t nq, uint32_t trials, uint32_t blocks) {
+    if (blocks < TC_SHARE_BLOCKS) return 1;
+    uint32_t most = 1;
+    for (uint32_t q = 2; q <= nq && q * trials <= (uint32_t)TC_MAX_TRIALS; ++q)
+        if (trials && 3 * 8 * ((q * trials + 1) & ~1u) + 32 * q <= 512) most = q;
+    const uint32_t groups = (nq + most - 1) / most;
+    return (nq + groups - 1) / groups;
+}
 
 // Row block of the U generator: 128 rows of segment `seg` starting at local row `i0`.
 struct TcBlock {
@@ -85,7 +115,7 @@ cudaError_t make_tmap_u8_ksteps2(CUtensorMap* map, const void* base, uint64_t ro
 void launch_tc_ugen(const VerifySeg* d_vsegs, const TcBlock* d_blocks, uint32_t nblocks, const ChaChaKey* d_keys,
                     const uint64_t* d_r, uint32_t t_base, uint32_t t_cnt, uint32_t n_rows, uint8_t* d_u,
                     uint64_t* d_ur_part, uint32_t trials_total, uint32_t* d_flags, cudaStream_t s,
-                    uint64_t u_row_pitch = 0, bool after = false);
+                    uint64_t u_row_pitch = 0, bool after = false, TcShare share = {});
 
 // The GEMM + drain: z_part[panel][t_base + t][j] (canonical residues) for
 // t < t_cnt.  tmap_m: m_enc bytes {8192, rows}, box {128, 128}, swizzle 128B;
@@ -114,19 +144,21 @@ void launch_tc_freivalds_small(const CUtensorMap& tmap_m, const CUtensorMap& tma
 // the tensor cores: z_part as above plus r_part[group][r index] (3-strip
 // group partial dots with the query, r_stride = total r entries, 22 groups),
 // summed by launch_tc_rreduce.  tmap_w: the queries' diagonal byte images
-// (launch_query_prep) {128, nq * 1024}, box {128, 48}, swizzle 128B.
+// (launch_query_prep) {128, nq * 1024}, box {128, tc_wimg_box(per)}, swizzle 128B.
+// t_cnt: trials per query, n_rows: of a group's U tile.
 void launch_tc_fused(const CUtensorMap& tmap_m, const CUtensorMap& tmap_u, const CUtensorMap& tmap_w,
                      const TcPanel* d_panels, uint32_t npanels, const VerifySeg* d_vsegs, uint32_t t_cnt,
                      uint32_t n_rows, uint32_t trials_total, uint64_t* d_z_part, uint64_t* d_r_part, uint64_t r_stride,
-                     uint32_t* d_err, int num_sms, cudaStream_t s, long long wait_cycles = 0);
+                     uint32_t* d_err, int num_sms, cudaStream_t s, long long wait_cycles = 0, TcShare share = {});
 inline uint32_t tc_groups(uint32_t) { return 22u; }  // strip groups of the fused pass (3 strips each)
 constexpr uint32_t WIMG_BYTES_PER_QUERY = 64u * 16u * 128u;
-constexpr uint32_t WIMG_BOX_ROWS = 48;  // one strip group's diagonal rows
+// one strip group's diagonal rows, or (several queries) one strip's
+inline uint32_t tc_wimg_box(uint32_t per) { return per > 1 ? 16u : 48u; }
 // r = sum of the group partials, and u_t . r partials for the pass's trials
 // from the U byte image.
 void launch_tc_rreduce(const VerifySeg* d_vsegs, const TcBlock* d_blocks, uint32_t nblocks, const uint64_t* d_r_part,
                        uint64_t r_stride, uint32_t groups, const uint8_t* d_u, uint32_t t_cnt, uint32_t n_rows,
-                       uint32_t trials_total, uint64_t* d_r, uint64_t* d_ur_part, cudaStream_t s);
+                       uint32_t trials_total, uint64_t* d_r, uint64_t* d_ur_part, cudaStream_t s, TcShare share = {});
 
 // Per segment: z_t = sum of its panels' partials, zv_t = z_t . v, ur_t =
 // sum of its blocks' partials; failed = first t with ur_t != zv_t or -1.
