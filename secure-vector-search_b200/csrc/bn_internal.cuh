@@ -18,12 +18,13 @@
 namespace bn {
 namespace api {
 // Pinned slots for copies of pageable host memory (bn_xfer.cu): one set per
-// context, made on first use, given back with it; one copy at a time uses them
+// context, made when its copies repay them, given back with it; one copy at a time uses them
 // (a copy that finds them taken goes to the driver directly).
 struct HostStage {
     static constexpr int SLOTS = 3;
-    static constexpr uint64_t SLOT_BYTES = 2u << 20, MIN_BYTES = 128u << 10;
+    static constexpr uint64_t SLOT_BYTES = 2u << 20, MIN_BYTES = 128u << 10, FROM_BYTES = 64u << 20;
     std::mutex mu;
+    uint64_t asked = 0;  // bytes of copies before the slots were made
     void* p = nullptr;
     cudaEvent_t ev[SLOTS] = {};
     ~HostStage();
@@ -297,11 +298,11 @@ struct HostMeta {
     std::vector<DecodeQuery> dq;
     std::vector<uint32_t> seg_cluster;  // IVF: list id of each segment
     std::vector<TcBlock> blocks;        // 128-row blocks of every verify segment
-    std::vector<TcPanel> panels;        // 4096-row panels of every verify segment
+    std::vector<TcPanel> panels;        // z panels of the verify segments (make_panels)
     std::vector<uint32_t> seg_block0, seg_panel0;
     uint64_t total_out = 0, max_rows = 0;
     bool same_rows = false;  // every segment is the same rows for the next query (flat_meta)
-    uint32_t per = 1;        // queries per pass that `panels` is laid out for (share_passes)
+    uint32_t per = 1;        // queries per pass that `panels` is laid out for (make_panels)
 };
 
 struct Sizes {

@@ -318,11 +318,6 @@ __global__ void query_decide_kernel(const IvPair* __restrict__ pairs, const uint
     ft[q] = t;
 }
 
-unsigned grid_cap(uint64_t work, unsigned threads, unsigned cap) {
-    const uint64_t g = (work + threads - 1) / threads;
-    return (unsigned)(g < 1 ? 1 : (g > cap ? cap : g));
-}
-
 int tmap_u8(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint32_t box_rows, const char* what) {
     cudaError_t e = make_tmap_u8(m, base, inner, rows, 128, box_rows);
     if (e != cudaSuccess) return fail(BN_ECUDA, "tensor map of %s: %s", what, cudaGetErrorString(e));

@@ -3,7 +3,7 @@
 // (tcgen05.mma kind::i8, s32 accumulators in TMEM), fed by TMA, drained by
 // four epilogue warps that recombine the byte limbs modulo p = 2^61 - 1.
 //
-// Roles per CTA (one CTA per SM, persistent over 4096-row panels):
+// Roles per CTA (one CTA per SM, persistent over panels of tc_panel_rows rows):
 //   warp 0  TMA producer: per 128-row stage, S boxes of 128 rows x 128 bytes
 //           of M_enc (S strips of 16 columns) + the 8T x 128 U tile
 //   warp 1  MMA issuer: per stage S x 4 tcgen05.mma (M=128, N=8T, K=32),

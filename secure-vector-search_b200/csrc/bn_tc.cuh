@@ -163,7 +163,7 @@ void launch_tc_rreduce(const VerifySeg* d_vsegs, const TcBlock* d_blocks, uint32
 // Per segment: z_t = sum of its panels' partials, zv_t = z_t . v, ur_t =
 // sum of its blocks' partials; failed = first t with ur_t != zv_t or -1.
 // d_chunks: scratch of tc_finish_words(nseg, trials) words (the shares of z . v
-// and u . r that the finish kernel's CTAs write and the decide kernel sums).
+// and u . r that the kernel's CTAs write and a segment's last CTA sums).
 // With few segments each one's panels are split over tc_finish_split CTAs.
 // d_done: nseg tickets, zero before the launch (the last CTA of a segment
 // decides it and leaves its ticket zero).

@@ -48,12 +48,27 @@ bool is_pageable(const void* p) {
     return a.type == cudaMemoryTypeUnregistered;
 }
 
-// The context's slots, made on the first staged copy (caller holds st.mu).
-int stage_ready(HostStage& st) {
-    if (st.p) return BN_OK;
-    CU(cudaMallocHost(&st.p, HostStage::SLOTS * HostStage::SLOT_BYTES));
-    for (cudaEvent_t& e : st.ev) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    return BN_OK;
+// Whether a copy of `bytes` may use the context's slots (caller holds st.mu); if not
+// it goes to the driver, as it would without them.  They are made once the copies
+// they could have served add up to FROM_BYTES: to pin and to release 6 MB takes 6 + 5 ms,
+// about what the slots save on 64 MB of copies (a context that only drew the keys of
+// 4,096 rows took 10 ms for it with slots made at once, 4.3 ms without).
+bool stage_ready(HostStage& st, uint64_t bytes) {
+    if (st.p) return true;
+    st.asked += bytes;
+    if (st.asked < HostStage::FROM_BYTES) return false;
+    for (cudaEvent_t& e : st.ev)
+        if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+            e = nullptr;
+            cudaGetLastError();
+            return false;
+        }
+    if (cudaMallocHost(&st.p, HostStage::SLOTS * HostStage::SLOT_BYTES) != cudaSuccess) {
+        st.p = nullptr;
+        cudaGetLastError();
+        return false;
+    }
+    return true;
 }
 
 // Bytes per slot of one copy: quarters of it, so that a copy of a few hundred
@@ -74,11 +89,11 @@ int stage_h2d(bn_ctx* ctx, void* dst, const void* src, uint64_t bytes, cudaStrea
     if (!bytes) return BN_OK;
     HostStage& st = ctx->stage;
     std::unique_lock<std::mutex> g(st.mu, std::defer_lock);
-    if (bytes < HostStage::MIN_BYTES || !is_pageable(src) || !g.try_lock()) {  // another thread's copy is staged
+    if (bytes < HostStage::MIN_BYTES || !is_pageable(src) || !g.try_lock() ||  // another thread's copy is staged
+        !stage_ready(st, bytes)) {
         CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
         return BN_OK;
     }
-    TRY(stage_ready(st));
     const uint64_t step = slot_bytes(bytes);
     for (uint64_t off = 0, i = 0; off < bytes; off += step, ++i) {
         const uint64_t n = std::min(step, bytes - off);
@@ -96,12 +111,11 @@ int stage_d2h(bn_ctx* ctx, void* dst, const void* src, uint64_t bytes, cudaStrea
     if (!bytes) return BN_OK;
     HostStage& st = ctx->stage;
     std::unique_lock<std::mutex> g(st.mu, std::defer_lock);
-    if (bytes < HostStage::MIN_BYTES || !is_pageable(dst) || !g.try_lock()) {
+    if (bytes < HostStage::MIN_BYTES || !is_pageable(dst) || !g.try_lock() || !stage_ready(st, bytes)) {
         CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
         CU(cudaStreamSynchronize(s));
         return BN_OK;
     }
-    TRY(stage_ready(st));
     const uint64_t step = slot_bytes(bytes), total = (bytes + step - 1) / step;
     for (uint64_t i = 0; i < total + HostStage::SLOTS - 1; ++i) {
         if (i < total) {
