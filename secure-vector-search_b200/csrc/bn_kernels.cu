@@ -510,34 +510,56 @@ query_prep_kernel(const uint64_t* __restrict__ L, uint32_t n1, const uint64_t* _
 }
 
 // ------------------------------------------------------------------ decode
-// Dot of a column-major row with a vector whose limbs sit in shared memory.
-__device__ __forceinline__ uint64_t cm_dot(const uint64_t* __restrict__ a_cm, uint64_t rows, uint64_t row,
-                                           const uint32_t (*vl)[6], uint32_t n1) {
-    uint64_t a0 = 0, a1 = 0, a2 = 0;
-#pragma unroll 8
-    for (uint32_t k = 0; k < n1; ++k) {
-        const uint64_t x = __ldg(a_cm + (uint64_t)k * rows + row);
-        const uint32_t lo = (uint32_t)x, hi = (uint32_t)(x >> 32);
-        a0 = mac(mac(a0, lo, vl[k][0]), hi, vl[k][3]);
-        a1 = mac(mac(a1, lo, vl[k][1]), hi, vl[k][4]);
-        a2 = mac(mac(a2, lo, vl[k][2]), hi, vl[k][5]);
-    }
-    return combine3(a0, a1, a2);
-}
+// AL g + H x alone, from the column-major arrays.  A CTA takes 32 rows at a time, a
+// warp an eighth of the 2 n1 columns with 16 loads in flight; the warps' shares meet
+// in shared memory and a warp in turn adds them up.  Bound by HBM (2 n1 x 8 bytes per
+// row): a thread per row over all columns had 8 loads in flight and, with few rows,
+// few CTAs.
+constexpr uint32_t DN_WARPS = 8;
 
-__global__ void dense_terms_kernel(const uint64_t* __restrict__ al_cm, const uint64_t* __restrict__ h_cm, uint64_t rows,
-                                   uint32_t n1, const uint64_t* __restrict__ g, const uint64_t* __restrict__ x,
-                                   uint64_t* __restrict__ out) {
-    __shared__ uint32_t gl[512][6], xl[512][6];
-    for (uint32_t k = threadIdx.x; k < n1; k += blockDim.x) {
-        Limbs3 b = limbs(g[k]), c = limbs_hi(g[k]);
-        gl[k][0] = b.b0; gl[k][1] = b.b1; gl[k][2] = b.b2; gl[k][3] = c.b0; gl[k][4] = c.b1; gl[k][5] = c.b2;
-        b = limbs(x[k]); c = limbs_hi(x[k]);
-        xl[k][0] = b.b0; xl[k][1] = b.b1; xl[k][2] = b.b2; xl[k][3] = c.b0; xl[k][4] = c.b1; xl[k][5] = c.b2;
+__global__ void __launch_bounds__(32 * DN_WARPS, 4)
+dense_terms_kernel(const uint64_t* __restrict__ al_cm, const uint64_t* __restrict__ h_cm, uint64_t rows, uint32_t n1,
+                   const uint64_t* __restrict__ g, const uint64_t* __restrict__ x, uint64_t* __restrict__ out) {
+    __shared__ uint4 lim[2 * 2 * 512];  // {b0,b1,b2,c0}, {c1,c2,-,-} per column of g, then of x
+    __shared__ uint64_t sh[2][DN_WARPS][32];
+    for (uint32_t k = threadIdx.x; k < 2 * n1; k += blockDim.x) {
+        const uint64_t w = k < n1 ? g[k] : x[k - n1];
+        const Limbs3 b = limbs(w), c = limbs_hi(w);
+        lim[2 * k] = make_uint4(b.b0, b.b1, b.b2, c.b0);
+        lim[2 * k + 1] = make_uint4(c.b1, c.b2, 0u, 0u);
     }
     __syncthreads();
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += (uint64_t)gridDim.x * blockDim.x)
-        out[i] = add_mod(cm_dot(al_cm, rows, i, gl, n1), cm_dot(h_cm, rows, i, xl, n1));
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t cols = 2 * n1 / DN_WARPS, c0 = warp * cols;  // a multiple of 16 (n1 >= 64), all of AL or all of H
+    const uint64_t* base = c0 < n1 ? al_cm + (uint64_t)c0 * rows : h_cm + (uint64_t)(c0 - n1) * rows;
+    uint32_t it = 0;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * 32; i0 < rows; i0 += (uint64_t)gridDim.x * 32, ++it) {
+        const uint64_t i = i0 + lane;
+        const uint64_t* p = base + (i < rows ? i : rows - 1);
+        uint64_t a0 = 0, a1 = 0, a2 = 0;  // at most 128 columns of 2^53 + 2^50 each
+        for (uint32_t k0 = 0; k0 < cols; k0 += 16) {
+            uint64_t xs[16];
+#pragma unroll
+            for (int kk = 0; kk < 16; ++kk) xs[kk] = __ldg(p + (uint64_t)(k0 + kk) * rows);
+#pragma unroll
+            for (int kk = 0; kk < 16; ++kk) {
+                const uint32_t lo = (uint32_t)xs[kk], hi = (uint32_t)(xs[kk] >> 32);
+                const uint4 l0 = lim[2 * (c0 + k0 + kk)], l1 = lim[2 * (c0 + k0 + kk) + 1];
+                a0 = mac(mac(a0, lo, l0.x), hi, l0.w);
+                a1 = mac(mac(a1, lo, l0.y), hi, l1.x);
+                a2 = mac(mac(a2, lo, l0.z), hi, l1.y);
+            }
+        }
+        auto& part = sh[it & 1];
+        part[warp][lane] = combine3(a0, a1, a2);
+        __syncthreads();  // one per block of rows: the other buffer is rewritten only after the next one
+        if (it % DN_WARPS == warp && i < rows) {
+            uint64_t sum = part[0][lane];
+#pragma unroll
+            for (uint32_t w = 1; w < DN_WARPS; ++w) sum = add_mod(sum, part[w][lane]);
+            out[i] = sum;
+        }
+    }
 }
 
 // Decode copies of the client state in 32-row blocks (layouts in
@@ -1682,7 +1704,7 @@ void launch_query_prep(const uint64_t* d_L, uint32_t n1, const uint64_t* d_v, ui
 
 void launch_dense_terms(const uint64_t* d_al_cm, const uint64_t* d_h_cm, uint64_t rows, uint32_t n1,
                         const uint64_t* d_g, const uint64_t* d_x, uint64_t* d_out, cudaStream_t s) {
-    dense_terms_kernel<<<grid_for(rows, 256, 148 * 8), 256, 0, s>>>(d_al_cm, d_h_cm, rows, n1, d_g, d_x, d_out);
+    dense_terms_kernel<<<grid_for(rows, 32, 148 * 4), 32 * DN_WARPS, 0, s>>>(d_al_cm, d_h_cm, rows, n1, d_g, d_x, d_out);
 }
 
 void launch_decode_layout(const uint64_t* d_al_cm, const uint64_t* d_h_cm, const uint64_t* d_mp_cm, uint64_t rows,
