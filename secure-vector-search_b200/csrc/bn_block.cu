@@ -56,7 +56,17 @@ void block_plan_free(BlockPlan* b) { delete b; }
 
 namespace {
 
-uint32_t kpanels_of(const BlockPlan& b) { return (uint32_t)((b.npad + b.k_panel4 - 1) / b.k_panel4); }
+// The u . r GEMM takes its K = rows in panels of the plan's (tuned) size, or shorter
+// ones where even panels of 4096 rows would leave SMs without one (8 queries over
+// 200,000 rows: 49 panels for 148 SMs).
+uint32_t k_panel_of(uint64_t npad, uint32_t B, uint32_t planned) {
+    const uint64_t a_tiles = (8ull * B + BG_AROWS - 1) / BG_AROWS, most = TC_SMS / std::min<uint64_t>(a_tiles, TC_SMS);
+    if ((npad + 4095) / 4096 >= most) return planned;
+    return (uint32_t)std::max<uint64_t>(512, align_up((npad + most - 1) / most, 128));
+}
+uint32_t k_panel_of(const BlockPlan& b) { return k_panel_of(b.npad, b.B, b.k_panel4); }
+
+uint32_t kpanels_of(const BlockPlan& b) { return (uint32_t)((b.npad + k_panel_of(b) - 1) / k_panel_of(b)); }
 
 uint32_t stages_for(const BgParams& p) { return bgemm_max_stages(p); }
 
@@ -265,7 +275,7 @@ int autotune(BlockPlan& b, cudaStream_t s) {
             p.w_tiles = 1;
             p.w_tile = b.n_rows;
             p.k_bytes = (uint32_t)b.npad;
-            p.k_panel = kp;
+            p.k_panel = k_panel_of(b);
             p.x_count = b.B;
             p.y_count = b.t_pass;
             p.out = reinterpret_cast<uint64_t*>(d + b.o_urpart);
@@ -322,7 +332,7 @@ uint64_t block_layout(BlockPlan& b, uint32_t n1, uint32_t k_alh, bool verify_onl
     b.o_zpart = L.take<uint64_t>(trials ? (uint64_t)b.npanels * tt * N : 0);
     b.o_z = L.take<uint64_t>((uint64_t)tt * N);
     b.o_zv = L.take<uint64_t>((uint64_t)tt * B);
-    b.o_urpart = L.take<uint64_t>(trials ? (uint64_t)((b.npad + 4095) / 4096) * tt * B : 0);
+    b.o_urpart = L.take<uint64_t>(trials ? (b.npad / k_panel_of(b.npad, B, 4096) + 1) * tt * B : 0);
     b.o_ur = L.take<uint64_t>((uint64_t)tt * B);
     b.o_fail = L.take<int32_t>(B);
     b.o_cs = L.take<int64_t>((uint64_t)B * b.topk_ctas * ks);
@@ -499,7 +509,7 @@ static void enqueue_verify(BlockPlan& b, const uint64_t* d_v, const uint8_t* d_s
         p.w_tiles = 1;
         p.w_tile = b.n_rows;
         p.k_bytes = (uint32_t)b.npad;
-        p.k_panel = b.k_panel4;
+        p.k_panel = k_panel_of(b);
         p.x_count = b.B;
         p.y_count = tc;
         p.out = urpart + (uint64_t)t0 * b.B;
