@@ -716,6 +716,16 @@ uint32_t bgemm_max_stages(const BgParams& p) {
 
 void launch_bgemm(const CUtensorMap& tmap_a, const CUtensorMap& tmap_w, const BgParams& p, uint32_t stages, int ctas,
                   uint32_t* d_err, cudaStream_t s, const CUtensorMap* tmap_a2, const CUtensorMap* tmap_w2) {
+    if (!stages && (p.ksteps2 || p.a_resident)) {
+        // No two stages of this form fit (an A tile of n1 = 512 resident leaves 97 KB
+        // beside it, one stage of two K steps at W = 256 is 64): one K step per
+        // stage, and where even that does not fit, A streamed.
+        BgParams q = p;
+        if (q.ksteps2) q.ksteps2 = 0;
+        else q.a_resident = 0;
+        launch_bgemm(tmap_a, tmap_w, q, bgemm_max_stages(q), ctas, d_err, s, tmap_a2, tmap_w2);
+        return;
+    }
     if (p.ksteps2 && (p.k_panel % (2 * BG_KSTEP) || !tmap_w2 || (!p.a_resident && (!p.a_blocked || !tmap_a2)))) {
         BgParams q = p;  // two K steps per stage do not apply: one per stage
         q.ksteps2 = 0;

@@ -77,7 +77,8 @@ struct BgParams {
 
 // tmap_a: A bytes {k_bytes, A rows}, box {128, 128}; tmap_w: W bytes
 // {k_bytes, W rows}, box {128, w_tile}; both 128-byte swizzle.  stages in
-// [2, BG_MAX_STAGES].  *err: bit 2/3/4 set when a bounded wait timed out,
+// [2, BG_MAX_STAGES], or 0 when bgemm_max_stages(p) found none (the launch then
+// takes a form that fits).  *err: bit 2/3/4 set when a bounded wait timed out,
 // bit 64 when the wind-down wait for the CTA's own MMAs did.
 // A-resident mode needs k_panel == k_bytes <= BG_MAX_ASLOTS * 128 and
 // bgemm_smem_bytes(p, stages) <= BG_MAX_SMEM.
