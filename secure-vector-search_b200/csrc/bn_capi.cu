@@ -562,7 +562,7 @@ int enqueue_pipeline(bn_ctx* ctx, const Corpus& c, const Sizes& z, const Meta& m
     }
     if (z.k) {
         launch_decode_topk(sc.r, decode_corpus(c), m.segs, m.seg_unit, m.dq, z.B, in.v, in.g, sc.x, in.t, in.t_nnz, z.k,
-                           z.ctas, decode_split(m.units, ctx->num_sms), sc.topk, out.mv, out.ids, out.scores, out.n, s);
+                           z.ctas, z.split, sc.topk, out.mv, out.ids, out.scores, out.n, s);
     } else {
         CU(cudaMemsetAsync(out.n, 0, (uint64_t)z.B * 4, s));
     }
@@ -572,8 +572,7 @@ int enqueue_pipeline(bn_ctx* ctx, const Corpus& c, const Sizes& z, const Meta& m
 
 Meta meta_at(char* d, const RunLayout& o, const HostMeta& hm, const TcMaps* maps) {
     return Meta{reinterpret_cast<ScanSeg*>(d + o.segs), reinterpret_cast<uint64_t*>(d + o.seg_blk),
-                reinterpret_cast<uint64_t*>(d + o.seg_unit), hm.seg_unit.empty() ? 0 : hm.seg_unit.back(),
-                (uint32_t)hm.segs.size(), hm.seg_blk.empty() ? 0 : hm.seg_blk.back(),
+                reinterpret_cast<uint64_t*>(d + o.seg_unit), (uint32_t)hm.segs.size(), hm.seg_blk.empty() ? 0 : hm.seg_blk.back(),
                 reinterpret_cast<VerifySeg*>(d + o.vsegs), (uint32_t)hm.vsegs.size(),
                 reinterpret_cast<DecodeQuery*>(d + o.dq), reinterpret_cast<TcBlock*>(d + o.tc_blocks),
                 (uint32_t)hm.blocks.size(), reinterpret_cast<TcPanel*>(d + o.tc_panels), (uint32_t)hm.panels.size(),
@@ -622,16 +621,18 @@ void engine_free(Engine& e) {
 // Decode CTAs of a run: DECODE_CTAS_PER_SM per SM in total (one wave of
 // the decode kernel), shared among the queries in proportion to their
 // units (32-row blocks), at least one per query and at most one per unit
-// (decode_split) or tile of 8 units.  Returns the total.
-uint32_t assign_decode_ctas(HostMeta& hm, int sms) {
+// (split: decode_split) or tile of 8 units.  Returns the total.
+uint32_t assign_decode_ctas(HostMeta& hm, int sms, uint32_t k, bool& split) {
     std::vector<uint64_t> units(hm.dq.size(), 0);
-    uint64_t total = 0;
+    uint64_t total = 0, most = 0;
     for (size_t q = 0; q < hm.dq.size(); ++q) {
         const DecodeQuery& d = hm.dq[q];
         if (d.nseg) units[q] = hm.seg_unit[d.seg0 + d.nseg] - hm.seg_unit[d.seg0];
         total += units[q];
+        most = std::max(most, units[q]);
     }
-    const uint64_t target = (uint64_t)sms * DECODE_CTAS_PER_SM, tile = decode_split(total, sms) ? 1 : 8;
+    split = decode_split(total, most, k, sms);
+    const uint64_t target = (uint64_t)sms * DECODE_CTAS_PER_SM, tile = split ? 1 : 8;
     uint32_t next = 0;
     for (size_t q = 0; q < hm.dq.size(); ++q) {
         uint64_t c = total ? (target * units[q] + total - 1) / total : 1;
@@ -646,11 +647,13 @@ uint32_t assign_decode_ctas(HostMeta& hm, int sms) {
 Sizes sizes_for(const Engine& e, HostMeta& hm, uint32_t B, uint32_t trials, uint32_t k) {
     const uint32_t per = hm.same_rows && e.ctx->engine == BN_ENGINE_TENSOR ? tc_share(B, trials, hm.seg_block0[1]) : 1;
     if (per != hm.per) make_panels(hm, per);
-    return Sizes{B, e.c.n1, trials, k, assign_decode_ctas(hm, e.ctx->num_sms), hm.total_out,
+    bool split = false;
+    const uint32_t ctas = assign_decode_ctas(hm, e.ctx->num_sms, k, split);
+    return Sizes{B, e.c.n1, trials, k, ctas, hm.total_out,
                  hm.segs.size(), hm.vsegs.size(), hm.blocks.size(), hm.seg_panel0.back(),
                  plan_freivalds(std::max<uint64_t>(hm.max_rows, 1), (uint32_t)std::max<size_t>(hm.vsegs.size(), 1),
                                 e.ctx->num_sms),
-                 e.ctx->engine, per};
+                 e.ctx->engine, per, split};
 }
 
 // One pipeline run over host inputs, split so that a caller can keep several

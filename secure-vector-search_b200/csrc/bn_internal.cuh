@@ -242,7 +242,6 @@ struct Meta {  // device pointers (+ host tensor maps)
     const ScanSeg* segs;
     const uint64_t* seg_blk;
     const uint64_t* seg_unit;  // decode units (32-row corpus blocks) per segment, prefix sums
-    uint64_t units;            // their total
     uint32_t nseg;
     uint64_t total_blocks;
     const VerifySeg* vsegs;
@@ -310,7 +309,8 @@ struct Sizes {
     uint64_t total_out, nseg, nvseg, nblocks, npanels;
     FreivaldsPlan fp;  // CUDA-core engine
     int engine;        // BN_ENGINE_*
-    uint32_t per = 1;  // queries per fused pass (TcShare)
+    uint32_t per = 1;    // queries per fused pass (TcShare)
+    bool split = false;  // form of the decode (decode_split)
 };
 
 

@@ -884,8 +884,6 @@ __device__ __forceinline__ uint64_t s_times_v_part(const DecodeCorpus& dc, uint6
 // inserted one at a time, each at the rank the ballot of the list entries
 // better than it gives, the entries below it moving down one lane.  No
 // shared memory and no block barrier.
-constexpr int WARP_TOPK_MAX = 32;
-
 __device__ __forceinline__ void warp_topk_offer(int64_t& ls, uint32_t& li, int k, bool valid, int64_t s, uint32_t id,
                                                 uint32_t lane) {
     const int64_t ts = __shfl_sync(FULL, ls, k - 1);
@@ -951,10 +949,10 @@ __device__ __forceinline__ void warp_topk_reduce(int64_t& ls, uint32_t& li, int 
 // best k go to the scratch lists, and the last CTA of the query to finish (a
 // ticket taken after a device-scope fence, no waiting) merges them.
 //
-// SPLIT (few units, see launch_decode_topk): the CTA's eight warps share one unit
-// at a time, four a quarter of the dense columns each, two S v and two M T, and
-// take turns in adding the shares up and ranking them: a corpus of 5,000 rows is
-// 157 units, which whole-unit warps put on 20 CTAs (50 us) and this on 157 (32 us).
+// SPLIT (decode_split): the CTA's eight warps share one unit at a time, four a
+// quarter of the dense columns each, two S v and two M T, and one of them, the next
+// for the next unit, adds the shares up and ranks them: a corpus of 5,000 rows is 157
+// units, which whole-unit warps put on 20 CTAs (50 us) and this on 157 (37 us).
 constexpr uint32_t DT_WARPS = DT_THREADS / 32;
 constexpr uint32_t DT_DENSE = 4, DT_S = 2, DT_T = 2;  // SPLIT: warps per part (2 n1 / 4 is a multiple of 32)
 
@@ -1016,11 +1014,9 @@ decode_topk_kernel(const uint64_t* __restrict__ r, DecodeCorpus dc, const ScanSe
         u_count = seg_unit[dq.seg0 + dq.nseg] - u_begin;
     }
     if constexpr (SPLIT) {
-        // The buffer is checked (two CTA barriers) every SP_CHECK units; between
-        // checks at most SP_CHECK * 32 rows append, and a check compacts above
-        // CAND_CAP - SP_CHECK * 32 = 1024 >= k entries.
-        constexpr uint32_t SP_CHECK = 32;
-        static_assert(CAND_CAP - SP_CHECK * 32 >= TOPK_MAX, "candidate buffer too small for the check interval");
+        // The candidate buffer needs no check: it takes all rows of a query that
+        // decode_split sends here with it.
+        static_assert(WARP_LISTS || DECODE_SPLIT_UNITS * 32 <= CAND_CAP, "candidate buffer smaller than a query's rows");
         uint32_t it = 0;
         for (uint64_t u = cta; u < u_count; u += dq.ctas, ++it) {
             const uint64_t gu = u_begin + u;
@@ -1070,8 +1066,6 @@ decode_topk_kernel(const uint64_t* __restrict__ r, DecodeCorpus dc, const ScanSe
                 if constexpr (WARP_LISTS) warp_topk_offer(ls, li, (int)k, valid, score, id, lane);
                 else topk_offer(buf, valid, score, id, buf.thr_s, buf.thr_i, buf.have_thr);
             }
-            if constexpr (!WARP_LISTS)
-                if (it % SP_CHECK == SP_CHECK - 1 && topk_full(buf, CAND_CAP - SP_CHECK * 32)) topk_compact(buf, (int)k);
         }
     } else {
         const uint64_t tiles = (u_count + DT_WARPS - 1) / DT_WARPS;
@@ -1448,7 +1442,7 @@ void launch_topk(const uint64_t* d_a, const uint64_t* d_b, const uint64_t* d_c, 
                  const TopkScratch& scratch, uint32_t* d_out_ids, int64_t* d_out_scores, uint32_t* d_out_n,
                  uint64_t* d_mv_out, cudaStream_t s) {
     if (!nq) return;
-    const bool warp_lists = k >= 1 && k <= (uint32_t)WARP_TOPK_MAX;
+    const bool warp_lists = k >= 1 && k <= WARP_TOPK_MAX;
     const dim3 grid(ctas_per_query, nq);
     auto rows_fn = warp_lists ? topk_rows_warp_kernel : topk_rows_kernel;
     auto merge_fn = warp_lists ? topk_merge_warp_kernel : topk_merge_kernel;
@@ -1721,7 +1715,7 @@ void launch_decode_topk(const uint64_t* d_r, const DecodeCorpus& dc, const ScanS
                         cudaStream_t s) {
     if (!nq) return;
     const unsigned shares = split ? 2 * DT_WARPS * 32 * 8 : 0, dyn = 2 * 2 * dc.n1 * 16 + shares;
-    const bool lists = k >= 1 && k <= (uint32_t)WARP_TOPK_MAX;  // every warp keeps its own list
+    const bool lists = k >= 1 && k <= WARP_TOPK_MAX;  // every warp keeps its own list
     auto fn = split ? (lists ? decode_topk_kernel<true, true> : decode_topk_kernel<false, true>)
                     : (lists ? decode_topk_kernel<true, false> : decode_topk_kernel<false, false>);
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * 2 * 512 * 16 + shares));

@@ -169,11 +169,21 @@ struct DecodeQuery {
 // Resident decode_topk CTAs per SM (its register bound); the host sizes
 // the decode grid to one wave of them.
 constexpr int DECODE_CTAS_PER_SM = 3;
-// Whether a run of `units` decode units in all gives its CTAs one unit at a time:
-// up to DECODE_SPLIT units per CTA of the wave; beyond, whole units per warp keep
-// more loads in flight.
-constexpr uint64_t DECODE_SPLIT = 2;
-constexpr bool decode_split(uint64_t units, int sms) { return units <= DECODE_SPLIT * DECODE_CTAS_PER_SM * (uint64_t)sms; }
+// Largest k whose ranking a warp's lanes hold as a sorted list.
+constexpr uint32_t WARP_TOPK_MAX = 32;
+// Whether a run's CTAs take one decode unit at a time (`units` in all, at most
+// `most` of one query): up to DECODE_SPLIT units per CTA of the wave; beyond, whole
+// units per warp keep more loads in flight.  Every CTA leaves a list of k candidates
+// that one CTA per query merges, so for k > 32, where that is a sort in shared memory,
+// only for queries of at most DECODE_SPLIT_UNITS units and k up to DECODE_SPLIT_K:
+// 1,000 rows (32 units), k = 200, 114 us against 124 with whole units per warp;
+// 2,000 rows, k = 33, 147 against 112; 20,000 rows, k = 1000, 1316 against 571.
+constexpr uint64_t DECODE_SPLIT = 2, DECODE_SPLIT_UNITS = 32;
+constexpr uint32_t DECODE_SPLIT_K = 256;
+constexpr bool decode_split(uint64_t units, uint64_t most, uint32_t k, int sms) {
+    return units <= DECODE_SPLIT * DECODE_CTAS_PER_SM * (uint64_t)sms && k >= 1 &&
+           (k <= WARP_TOPK_MAX || (most <= DECODE_SPLIT_UNITS && k <= DECODE_SPLIT_K));
+}
 
 // Top-k candidate lists.
 constexpr int TOPK_MAX = 1024;

@@ -112,3 +112,34 @@ def test_ivf_segments_inside_blocks(ctx):
             assert np.array_equal(hits[b][0], ids) and np.array_equal(hits[b][1], sc)
             assert fc[b] == ft[b] == -1
     v.close()
+
+
+@pytest.mark.parametrize("m,k", [(300, 100), (1024, 256), (1024, 257), (1025, 256), (6001, 1000)])
+def test_large_k(ctx, m, k):
+    """k > 32 on both sides of the line between the forms: the oracle's hits, and a
+    candidate list per eight units only (a list per unit cost more to merge than the
+    whole decode) where a query has more than 32 units or k is above 256."""
+    from bn_b200 import capi as c
+
+    M = int8_matrix(m, 768, 30 + m)
+    L = O.generate_subspace(bytes([9]) * 32)
+    cl = O.encrypt_cluster(M.reshape(-1), m, L, O.derive_h_seed(2, 0))
+    f = c.Flat.build(ctx, cl.m_enc, cl.a_l, cl.h_mat, m)
+    f.attach_client(L, M.reshape(-1), cl.s_mat.rowptr, cl.s_mat.idx, cl.s_mat.sign)
+    encs = [O.encode_query(int8_matrix(1, 768, 31 + b)[0], L, O.derive_h_seed(22, b)) for b in range(2)]
+    hits, failed, _, mv = f.query(np.stack([e.v_enc for e in encs]), np.stack([e.g for e in encs]),
+                                  [(e.t_idx, e.t_sign) for e in encs], None, 0, k, want_mv=True)
+    for b, enc in enumerate(encs):
+        want = O.decode_scores(O.matvec(cl.m_enc, m, N, enc.v_enc), cl, L, enc)
+        assert np.array_equal(mv[b], want)
+        ids, sc = O.topk(O.to_signed(want), k)
+        assert np.array_equal(hits[b][0], ids) and np.array_equal(hits[b][1], sc)
+    used = ctx.memory()[1]
+    plan = f.plan(1, 0, k)
+    grown = ctx.memory()[1] - used
+    plan.close()
+    units = (m + 31) // 32
+    lists = units if units <= 32 and k <= 256 else (units + 7) // 8
+    # beside the lists: r (8 m) and the query's own arrays (below 64 KB)
+    assert grown <= 12 * k * lists + 16 * m + (64 << 10), (grown, lists)
+    f.close()
