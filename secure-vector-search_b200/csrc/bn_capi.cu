@@ -1612,6 +1612,8 @@ int bn_keygen_h_s(bn_ctx* ctx, const uint8_t* h_seed, uint64_t m, uint32_t n1, u
             if (hrp[m] > s_cap) {
                 rc = fail(BN_EINVAL, "S has %llu entries, more than s_cap = %llu", (unsigned long long)hrp[m],
                           (unsigned long long)s_cap);
+            } else if (hrp[m] && (!s_idx || !s_sign)) {
+                rc = fail(BN_EINVAL, "null s_idx / s_sign for %llu entries", (unsigned long long)hrp[m]);
             } else {
                 memcpy(s_rowptr, hrp.data(), (m + 1) * 8);
                 rc = stage_d2h(ctx, H, dH.p, m * n1 * 8, s);

@@ -81,3 +81,24 @@ def test_ivf_built_from_device_keys_equals_host_keys(ctx):
             assert np.array_equal(dev.compute_products(ci, v), O.matvec(case.clusters[ci].m_enc, case.sizes[ci], N, v))
     host.close()
     dev.close()
+
+
+@pytest.mark.parametrize("missing", ["idx", "sign"])
+def test_keys_without_room_for_s_are_refused(missing):
+    """A null s_idx or s_sign with a sufficient s_cap is an error, also once the
+    context stages its host copies (after 64 MB of them)."""
+    import ctypes
+
+    c = capi()
+    own = c.Context(0)
+    m = 70_000
+    for _ in range(2):  # H is 72 MB
+        c.keygen_h_s(own, O.derive_h_seed(4, 0), m)
+    H, rp = np.zeros(m * 128, np.uint64), np.zeros(m + 1, np.uint64)
+    seed = np.frombuffer(O.derive_h_seed(4, 0), np.uint8).copy()
+    ix, sg = np.zeros(m * 160, np.uint32), np.zeros(m * 160, np.int8)
+    nnz = ctypes.c_uint64(0)
+    rc = c.lib.bn_keygen_h_s(own.h, c.ptr(seed), m, 128, c.ptr(H), c.ptr(rp), None if missing == "idx" else c.ptr(ix),
+                             None if missing == "sign" else c.ptr(sg), m * 160, ctypes.byref(nnz))
+    assert rc == c.BN_EINVAL and 0 < nnz.value <= m * 160
+    own.close()
