@@ -24,7 +24,7 @@ struct HostStage {
     static constexpr int SLOTS = 3;
     static constexpr uint64_t SLOT_BYTES = 2u << 20, MIN_BYTES = 128u << 10, FROM_BYTES = 64u << 20;
     std::mutex mu;
-    uint64_t asked = 0;  // bytes of copies before the slots were made
+    uint64_t asked = 0;  // bytes of copies since the slots were last tried to be made
     void* p = nullptr;
     cudaEvent_t ev[SLOTS] = {};
     ~HostStage();

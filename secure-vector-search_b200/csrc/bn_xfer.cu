@@ -55,11 +55,13 @@ bool is_pageable(const void* p) {
 // it goes to the driver, as it would without them.  They are made once the copies
 // they could have served add up to FROM_BYTES: to pin and to release 6 MB takes 6 + 5 ms,
 // about what the slots save on 64 MB of copies (a context that only drew the keys of
-// 4,096 rows took 10 ms for it with slots made at once, 4.3 ms without).
+// 4,096 rows took 10 ms for it with slots made at once, 4.3 ms without).  Where they
+// cannot be made, the next try comes after as many bytes again.
 bool stage_ready(HostStage& st, uint64_t bytes) {
     if (st.p) return true;
     st.asked += bytes;
     if (st.asked < HostStage::FROM_BYTES) return false;
+    st.asked = 0;
     for (cudaEvent_t& e : st.ev)
         if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
             e = nullptr;
