@@ -1428,6 +1428,7 @@ int bn_ivf_build(bn_ctx* ctx, uint32_t nlist, const uint64_t* off, const uint32_
         rc = fail(BN_ECUDA, "upload ids failed");
     if (rc == BN_OK) rc = upload_colmajor(ctx, a_l, rows, n1, c.al_cm, v->e.stream);
     if (rc == BN_OK) rc = upload_colmajor(ctx, h, rows, n1, c.h_cm, v->e.stream);
+    if (rc == BN_OK && cudaStreamSynchronize(v->e.stream) != cudaSuccess) rc = fail(BN_ECUDA, "upload sync failed");
     if (rc != BN_OK) {
         engine_free(v->e);
         delete v;

@@ -443,9 +443,11 @@ int encrypt_dense(bn_ctx* ctx, const uint64_t* d_mq, uint64_t rows, uint32_t n1,
                   const uint64_t* d_H, uint64_t* d_enc, uint64_t* d_al, DevMem& ws, cudaStream_t s);
 // First entry of S below nnz that is not (col < n, sign +-1), or nnz.
 uint64_t first_bad_entry(bn_sparse_csr S, uint64_t nnz);
-// Copies of pageable host memory in s's order (bn_xfer.cu).  stage_h2d: src may
-// be reused on return, the copy may still be under way on s; stage_d2h: dst is
-// written on return.
+// Copies between host memory and the device in s's order (bn_xfer.cu).  stage_h2d: the
+// copy may still be under way on s on return; a pageable src may be reused then, a
+// pinned one only once s has passed the copy (callers wait for s before they
+// return, engine_free on their error exits).  stage_d2h: dst is written on return,
+// and s has passed everything before the copy.
 int stage_h2d(bn_ctx* ctx, void* dst, const void* src, uint64_t bytes, cudaStream_t s);
 int stage_d2h(bn_ctx* ctx, void* dst, const void* src, uint64_t bytes, cudaStream_t s);
 // bn_ivf_build_keygen over lists whose global indices start at list0 (the

@@ -1,5 +1,5 @@
 """Host copies and checks beside the kernels: the threads that share them stay the
-same from call to call."""
+same from call to call, and pinned arrays may be reused when a call returns."""
 from __future__ import annotations
 
 import os
@@ -39,3 +39,36 @@ def test_calls_do_not_make_threads(ctx):
             assert seen is None or _threads() == seen
             seen = _threads()
     f.close()
+
+
+def _pinned(a):
+    import torch
+
+    return torch.from_numpy(a.view(np.int64)).pin_memory().numpy().view(np.uint64)
+
+
+def test_pinned_arrays_are_free_on_return(ctx):
+    """Pinned sources are copied asynchronously: the call has to wait for them."""
+    from bn_b200 import capi as c
+
+    m = 6000
+    off = np.array([0, 2500, m], np.uint64)
+    m_enc, a_l, h = uniform_fp((m, N), 43), uniform_fp((m, 128), 44), uniform_fp((m, 128), 45)
+    v = uniform_fp((N,), 46)
+    pins = [_pinned(x.reshape(-1)) for x in (m_enc, a_l, h)]
+    ivf = c.Ivf.build(ctx, off, np.arange(m, dtype=np.uint32), *pins)
+    flat = c.Flat.build(ctx, *[_pinned(x.reshape(-1)) for x in (m_enc, a_l, h)], m)
+    for p in pins:
+        p[:] = 0
+    want = O.matvec(m_enc, m, N, v)
+    assert np.array_equal(ivf.compute_products(1, v), want[2500:])
+    g = uniform_fp((2, 128), 47)
+    assert np.array_equal(ivf.decode_dense_terms(1, g[0], g[1]), flat.decode_dense_terms(g[0], g[1])[2500:])
+    r = _pinned(np.tile(want, 1))
+    for bad in (False, True):
+        r[m - 1] = (int(want[m - 1]) + bad) % O.P
+        assert flat.verify(r, v, bytes([5]) * 32, 3)[0] == (0 if bad else -1)
+        r[:] = 1
+        r[:] = want
+    ivf.close()
+    flat.close()
