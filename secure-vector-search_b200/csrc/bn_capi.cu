@@ -873,9 +873,8 @@ int run_scan(Engine& e, uint64_t row0, uint64_t rows, const uint64_t* v_encs, ui
                 e.ctx->num_sms, reinterpret_cast<uint32_t*>(d + o_e), e.stream, e.ctx->debug_wait_cycles);
     CU(cudaGetLastError());
     TRY(stage_d2h(e.ctx, r, d + o_r, (uint64_t)B * rows * 8, e.stream));
-    uint32_t ev = 0;
+    uint32_t ev = 0;  // pageable: the copy has reached it on return
     CU(cudaMemcpyAsync(&ev, d + o_e, 4, cudaMemcpyDeviceToHost, e.stream));
-    CU(cudaStreamSynchronize(e.stream));
     if (ev) return fail(BN_ECUDA, "a device pipeline wait timed out (flags 0x%x); results discarded", ev);
     return BN_OK;
 }
