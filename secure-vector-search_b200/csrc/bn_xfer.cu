@@ -24,7 +24,9 @@ namespace {
 // TEAM.  With one thread per 128 KB a call's check and its copies took teams of
 // different sizes: verify of 150,000 rows 512 us (378 without any), now 373; a
 // quantise between such calls 196 us, now 11.  Below CHECK_FROM and COPY_FROM bytes
-// one core is done before a team that has gone to sleep wakes up (50 us).
+// one core is done before a team that has gone to sleep wakes up (50 us), and a copy
+// up is left to the driver (verify of 60,000 rows, 480 KB: staged 199 us, now 196; a
+// copy down gains by its slots from MIN_BYTES on: products of 40,000 rows 170 -> 113).
 constexpr int TEAM = 16;
 constexpr uint64_t CHECK_FROM = 1u << 20, COPY_FROM = 512u << 10;
 int threads_for(uint64_t bytes, uint64_t from) { return bytes < from ? 1 : std::min(TEAM, omp_get_max_threads()); }
@@ -94,7 +96,7 @@ int stage_h2d(bn_ctx* ctx, void* dst, const void* src, uint64_t bytes, cudaStrea
     if (!bytes) return BN_OK;
     HostStage& st = ctx->stage;
     std::unique_lock<std::mutex> g(st.mu, std::defer_lock);
-    if (bytes < HostStage::MIN_BYTES || !is_pageable(src) || !g.try_lock() ||  // another thread's copy is staged
+    if (bytes < COPY_FROM || !is_pageable(src) || !g.try_lock() ||  // another thread's copy is staged
         !stage_ready(st, bytes)) {
         CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
         return BN_OK;
