@@ -167,7 +167,8 @@ void launch_tc_rreduce(const VerifySeg* d_vsegs, const TcBlock* d_blocks, uint32
 // With few segments each one's panels are split over tc_finish_split CTAs.
 // d_done: nseg tickets, zero before the launch (the last CTA of a segment
 // decides it and leaves its ticket zero).
-inline uint32_t tc_finish_split(uint32_t nseg) { return nseg <= 4 ? 16u : 1u; }
+constexpr uint32_t FIN_SPLIT = 16;
+inline uint32_t tc_finish_split(uint32_t nseg) { return nseg <= 4 ? FIN_SPLIT : 1u; }
 inline uint64_t tc_finish_words(uint32_t nseg, uint32_t trials) {
     return (uint64_t)nseg * trials * (N / 128 + 1) * tc_finish_split(nseg);
 }
