@@ -35,6 +35,7 @@ struct BlockPlan {
     bool verify_only = false;  // Protocol 2 over claimed responses only
     uint64_t rows = 0, nld = 0, npad = 0;
     uint32_t t_pass = 0, n_rows = 0;   // trials per Freivalds pass, U rows (8 * even trials)
+    bool compact = false;  // panels of TC_PANEL_ROWS rows (see Sizes): a smaller workspace
     uint32_t panel_rows = TC_PANEL_ROWS;
     uint32_t nblocks = 0, npanels = 0;  // U row blocks, z panels
     // tuned GEMM configuration
@@ -65,7 +66,10 @@ uint32_t k_panel_of(uint64_t npad, uint32_t B, uint32_t planned) {
     if ((npad + 4095) / 4096 >= most) return planned;
     return (uint32_t)std::max<uint64_t>(512, align_up((npad + most - 1) / most, 128));
 }
-uint32_t k_panel_of(const BlockPlan& b) { return k_panel_of(b.npad, b.B, b.k_panel4); }
+uint32_t k_panel_of(const BlockPlan& b, uint32_t planned) {
+    return b.compact ? planned : k_panel_of(b.npad, b.B, planned);
+}
+uint32_t k_panel_of(const BlockPlan& b) { return k_panel_of(b, b.k_panel4); }
 
 uint32_t kpanels_of(const BlockPlan& b) { return (uint32_t)((b.npad + k_panel_of(b) - 1) / k_panel_of(b)); }
 
@@ -333,7 +337,8 @@ uint64_t block_layout(BlockPlan& b, uint32_t n1, uint32_t k_alh, bool verify_onl
     b.o_zpart = L.take<uint64_t>(trials ? (uint64_t)b.npanels * tt * N : 0);
     b.o_z = L.take<uint64_t>((uint64_t)tt * N);
     b.o_zv = L.take<uint64_t>((uint64_t)tt * B);
-    b.o_urpart = L.take<uint64_t>(trials ? (b.npad / k_panel_of(b.npad, B, 4096) + 1) * tt * B : 0);
+    const uint64_t kp = k_panel_of(b, 4096);
+    b.o_urpart = L.take<uint64_t>(trials ? (b.npad + kp - 1) / kp * tt * B : 0);
     b.o_ur = L.take<uint64_t>((uint64_t)tt * B);
     b.o_fail = L.take<int32_t>(B);
     b.o_cs = L.take<int64_t>((uint64_t)B * b.topk_ctas * ks);
@@ -360,6 +365,20 @@ int block_prepare(bn_flat* f) {
     return block_prepare_locked(f->e, nullptr);
 }
 
+// The sizes that a plan's workspace depends on; returns its bytes.
+static uint64_t block_sizes(BlockPlan& b, const Corpus& c, int sms, bool verify_only, bool compact) {
+    b.compact = compact;
+    b.nld = align_up(c.rows, 16);
+    b.npad = align_up(c.rows, 128);
+    b.t_pass = std::min<uint32_t>(std::max<uint32_t>(b.trials, 1), TC_MAX_TRIALS);
+    b.n_rows = 8 * ((b.t_pass + 1) & ~1u);
+    b.nblocks = (uint32_t)((c.rows + TC_ROWS - 1) / TC_ROWS);
+    b.panel_rows = compact ? TC_PANEL_ROWS : tc_panel_rows(b.nblocks, 1);
+    b.npanels = (uint32_t)((c.rows + b.panel_rows - 1) / b.panel_rows);
+    b.topk_ctas = (int)std::max<uint64_t>(1, std::min<uint64_t>((c.rows + 511) / 512, (uint64_t)sms * 4 / b.B));
+    return block_layout(b, c.n1, (uint32_t)align_up(2ull * c.n1, 128), verify_only);
+}
+
 int block_plan_create(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k, uint32_t flags, BlockPlan** out) {
     *out = nullptr;
     if (!B || B > 8192) return fail(BN_EINVAL, "B = %u is outside 1..=8192 queries per block", B);
@@ -377,13 +396,6 @@ int block_plan_create(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k, uint3
     b->trials = trials;
     b->k = k;
     b->rows = c.rows;
-    b->nld = align_up(c.rows, 16);
-    b->npad = align_up(c.rows, 128);
-    b->t_pass = std::min<uint32_t>(std::max<uint32_t>(trials, 1), TC_MAX_TRIALS);
-    b->n_rows = 8 * ((b->t_pass + 1) & ~1u);
-    b->nblocks = (uint32_t)((c.rows + TC_ROWS - 1) / TC_ROWS);
-    b->panel_rows = tc_panel_rows(b->nblocks, 1);
-    b->npanels = (uint32_t)((c.rows + b->panel_rows - 1) / b->panel_rows);
     b->w_tile = (uint32_t)std::min<uint64_t>(256, align_up(8ull * B, 16));
     // Both operands stream, two K steps per stage where three or two such stages
     // fit: with several W tiles an A tile kept in shared memory leaves room for
@@ -400,8 +412,8 @@ int block_plan_create(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k, uint3
         }
     }
     const int sms = f->e.ctx->num_sms;
-    b->topk_ctas = (int)std::max<uint64_t>(1, std::min<uint64_t>((c.rows + 511) / 512, (uint64_t)sms * 4 / B));
-    const uint64_t total = block_layout(*b, c.n1, c.k_alh, verify_only);
+    uint64_t total = block_sizes(*b, c, sms, verify_only, (flags & BLOCK_COMPACT) != 0);
+    if (!b->compact && !b->ws.fits(f->e.ctx, total)) total = block_sizes(*b, c, sms, verify_only, true);
     int rc = b->ws.alloc(f->e.ctx, total);
     cudaStream_t s = f->e.stream;
     if (rc == BN_OK) {
@@ -443,22 +455,12 @@ int block_plan_create(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k, uint3
 
 // Workspace bytes a block plan of B queries would allocate (the corpus's
 // byte-planar copies, made once per handle, are not included).
-uint64_t block_plan_estimate(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k) {
-    const Corpus& c = f->e.c;
+uint64_t block_plan_estimate(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k, bool compact) {
     BlockPlan b;
     b.B = B;
     b.trials = trials;
     b.k = k;
-    b.rows = c.rows;
-    b.nld = align_up(c.rows, 16);
-    b.npad = align_up(c.rows, 128);
-    b.t_pass = std::min<uint32_t>(std::max<uint32_t>(trials, 1), TC_MAX_TRIALS);
-    b.n_rows = 8 * ((b.t_pass + 1) & ~1u);
-    b.nblocks = (uint32_t)((c.rows + TC_ROWS - 1) / TC_ROWS);
-    b.panel_rows = tc_panel_rows(b.nblocks, 1);
-    b.npanels = (uint32_t)((c.rows + b.panel_rows - 1) / b.panel_rows);
-    b.topk_ctas = (int)std::max<uint64_t>(1, std::min<uint64_t>((c.rows + 511) / 512, (uint64_t)f->e.ctx->num_sms * 4 / B));
-    return block_layout(b, c.n1, (uint32_t)align_up(2ull * c.n1, 128), false);
+    return block_sizes(b, f->e.c, f->e.ctx->num_sms, false, compact);
 }
 
 void block_plan_config(const BlockPlan* b, uint32_t cfg[6], float tuned_ms[2]) {

@@ -384,13 +384,14 @@ int keygen_lists(bn_ctx* ctx, uint32_t lists, const uint64_t* off, const uint8_t
 // The z panels of every verify segment, `per` segments to a pass: a panel is listed
 // for the first segment of a group only and stands for the others' too (z partials
 // keep a place for every segment's panels, seg_panel0).
-void make_panels(HostMeta& hm, uint32_t per) {
+void make_panels(HostMeta& hm, uint32_t per, bool compact = false) {
     hm.per = per;
+    hm.compact = compact;
     hm.panels.clear();
     hm.seg_panel0.assign(hm.vsegs.size() + 1, 0);
     uint64_t max_blocks = 0;
     for (const VerifySeg& v : hm.vsegs) max_blocks = std::max<uint64_t>(max_blocks, (v.rows + TC_ROWS - 1) / TC_ROWS);
-    const uint32_t panel_rows = tc_panel_rows(max_blocks, (hm.vsegs.size() + per - 1) / per);
+    const uint32_t panel_rows = compact ? TC_PANEL_ROWS : tc_panel_rows(max_blocks, (hm.vsegs.size() + per - 1) / per);
     uint32_t z0 = 0, tile0 = 0;  // next z partial and U tile
     for (uint32_t s = 0; s < hm.vsegs.size(); ++s) {
         const VerifySeg& v = hm.vsegs[s];
@@ -466,18 +467,18 @@ RunLayout make_layout(const Sizes& z, bool want_mv) {
     o.vfailed = L.take<int32_t>(std::max<uint64_t>(z.nvseg, 1));
     o.ur = L.take<uint64_t>(std::max<uint64_t>(z.nvseg * z.trials, 1));
     o.zv = L.take<uint64_t>(std::max<uint64_t>(z.nvseg * z.trials, 1));
-    o.err = L.take<uint32_t>(1);
-    o.flags = L.take<uint32_t>(1);  // DRAW_HIT_P when a Protocol 2 draw equalled p
+    const bool tc = z.engine == BN_ENGINE_TENSOR;
+    o.err = L.take<uint32_t>(2);
+    o.flags = o.err + 4;  // DRAW_HIT_P when a Protocol 2 draw equalled p
     o.out_end = L.off;
     // cleared with err and flags in one go (o.err .. o.zero_end)
-    o.cand_done = L.take<uint32_t>(z.B);
-    o.fin_done = L.take<uint32_t>(z.nvseg);
+    o.cand_done = L.take<uint32_t>(z.B + (tc && z.trials ? z.nvseg : 0));
+    o.fin_done = o.cand_done + z.B * 4ull;
     o.zero_end = L.off;
     o.limbs = L.take<QLimb>((uint64_t)z.B * N);
     o.x = L.take<uint64_t>((uint64_t)z.B * z.n1);
     o.r = L.take<uint64_t>(std::max<uint64_t>(z.total_out, 1));
     o.mv = want_mv ? L.take<uint64_t>(std::max<uint64_t>(z.total_out, 1)) : 0;
-    const bool tc = z.engine == BN_ENGINE_TENSOR;
     const uint64_t zp = !z.trials ? 1 : tc ? z.npanels * z.trials * N : (uint64_t)z.nvseg * z.fp.chunks * z.trials * N;
     const uint64_t up = !z.trials ? 1 : tc ? z.nblocks * z.trials : (uint64_t)z.nvseg * z.fp.chunks * z.trials;
     o.z_part = L.take<uint64_t>(std::max<uint64_t>(zp, 1));
@@ -622,7 +623,7 @@ void engine_free(Engine& e) {
 // the decode kernel), shared among the queries in proportion to their
 // units (32-row blocks), at least one per query and at most one per unit
 // (split: decode_split) or tile of 8 units.  Returns the total.
-uint32_t assign_decode_ctas(HostMeta& hm, int sms, uint32_t k, bool& split) {
+uint32_t assign_decode_ctas(HostMeta& hm, int sms, uint32_t k, bool compact, bool& split) {
     std::vector<uint64_t> units(hm.dq.size(), 0);
     uint64_t total = 0, most = 0;
     for (size_t q = 0; q < hm.dq.size(); ++q) {
@@ -631,7 +632,7 @@ uint32_t assign_decode_ctas(HostMeta& hm, int sms, uint32_t k, bool& split) {
         total += units[q];
         most = std::max(most, units[q]);
     }
-    split = decode_split(total, most, k, sms);
+    split = !compact && decode_split(total, most, k, sms);
     const uint64_t target = (uint64_t)sms * DECODE_CTAS_PER_SM, tile = split ? 1 : 8;
     uint32_t next = 0;
     for (size_t q = 0; q < hm.dq.size(); ++q) {
@@ -644,16 +645,30 @@ uint32_t assign_decode_ctas(HostMeta& hm, int sms, uint32_t k, bool& split) {
     return next;
 }
 
-Sizes sizes_for(const Engine& e, HostMeta& hm, uint32_t B, uint32_t trials, uint32_t k) {
+Sizes sizes_for(const Engine& e, HostMeta& hm, uint32_t B, uint32_t trials, uint32_t k, bool compact) {
     const uint32_t per = hm.same_rows && e.ctx->engine == BN_ENGINE_TENSOR ? tc_share(B, trials, hm.seg_block0[1]) : 1;
-    if (per != hm.per) make_panels(hm, per);
+    if (per != hm.per || compact != hm.compact) make_panels(hm, per, compact);
     bool split = false;
-    const uint32_t ctas = assign_decode_ctas(hm, e.ctx->num_sms, k, split);
+    const uint32_t ctas = assign_decode_ctas(hm, e.ctx->num_sms, k, compact, split);
     return Sizes{B, e.c.n1, trials, k, ctas, hm.total_out,
                  hm.segs.size(), hm.vsegs.size(), hm.blocks.size(), hm.seg_panel0.back(),
                  plan_freivalds(std::max<uint64_t>(hm.max_rows, 1), (uint32_t)std::max<size_t>(hm.vsegs.size(), 1),
                                 e.ctx->num_sms),
                  e.ctx->engine, per, split};
+}
+
+// Lays out a run of *j.hm and reserves its workspace: in the compact form (Sizes)
+// where the other does not fit.
+int lay_out(Engine& e, QueryJob& j, DevMem& ws) {
+    for (bool compact = j.compact;; compact = true) {
+        j.z = sizes_for(e, *j.hm, j.B, j.trials, j.k, compact);
+        j.o = make_layout(j.z, j.want_mv);
+        if (compact || ws.fits(e.ctx, j.o.total)) {
+            const int rc = ws.reserve_grow(e.ctx, j.o.total);
+            if (rc == BN_OK || compact) return rc;
+            cudaGetLastError();  // the device has no room for it
+        }
+    }
 }
 
 // One pipeline run over host inputs, split so that a caller can keep several
@@ -680,10 +695,8 @@ int job_prepare(Engine& e, QueryJob& j, DevMem& ws, PinnedMem& host, const uint6
     TRY(validate_residues(v_enc, (uint64_t)B * N, "v_enc"));
     TRY(validate_residues(g, (uint64_t)B * c.n1, "g"));
 
-    j.z = sizes_for(e, hm, B, trials, k);
-    j.o = make_layout(j.z, j.want_mv);
+    TRY(lay_out(e, j, ws));
     const RunLayout& o = j.o;
-    TRY(ws.reserve_grow(e.ctx, o.total));
     TRY(host.reserve(o.out_end));
     char* d = ws.at<char>();
     TRY(make_tc_maps(j.z, reinterpret_cast<uint8_t*>(d + o.u_buf), reinterpret_cast<uint8_t*>(d + o.wimg), j.maps));
@@ -796,7 +809,12 @@ int run_verify(Engine& e, uint64_t row0, uint64_t rows, const uint64_t* r, const
     finish_meta(hm);
     Sizes z{1, e.c.n1, trials, 0, 1, rows, 0, 1, hm.blocks.size(), hm.panels.size(),
             plan_freivalds(rows, 1, e.ctx->num_sms), e.ctx->engine};
-    const RunLayout o = make_layout(z, false);
+    RunLayout o = make_layout(z, false);
+    if (!e.ws.fits(e.ctx, o.total)) {  // the compact form (Sizes)
+        make_panels(hm, 1, true);
+        z.npanels = hm.panels.size();
+        o = make_layout(z, false);
+    }
     TRY(e.ws.reserve(e.ctx, o.total));
     TRY(e.host.reserve(o.out_end));
     char* h = e.host.at<char>();
@@ -1196,9 +1214,14 @@ int bn_flat_plan(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k, bn_plan** 
     auto* p = new bn_plan();
     p->h = f;
     flat_meta(f->m, B, p->hm);
-    p->z = sizes_for(f->e, p->hm, B, trials, k);
-    p->o = make_layout(p->z, false);
-    int rc = p->ws.alloc(f->e.ctx, p->o.total);
+    QueryJob j;
+    j.hm = &p->hm;
+    j.B = B;
+    j.trials = trials;
+    j.k = k;
+    int rc = lay_out(f->e, j, p->ws);
+    p->z = j.z;
+    p->o = j.o;
     if (rc == BN_OK)
         rc = make_tc_maps(p->z, reinterpret_cast<uint8_t*>(p->ws.at<char>() + p->o.u_buf),
                           reinterpret_cast<uint8_t*>(p->ws.at<char>() + p->o.wimg), p->maps);

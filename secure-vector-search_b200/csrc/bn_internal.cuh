@@ -124,6 +124,12 @@ struct DevMem {
         bytes = b;
         return BN_OK;
     }
+    // Whether `b` bytes are there or would be within the budget.
+    bool fits(bn_ctx* c, uint64_t b) const {
+        if (p && bytes >= b) return true;
+        std::lock_guard<std::mutex> g(c->mu);
+        return c->used - (p ? bytes : 0) + b <= c->budget;
+    }
     // Grow-only reallocation (contents not kept).
     int reserve(bn_ctx* c, uint64_t b) { return (p && bytes >= b) ? BN_OK : alloc(c, b); }
     // The size reserve_grow makes room for: at least `need`, and half again
@@ -302,6 +308,7 @@ struct HostMeta {
     uint64_t total_out = 0, max_rows = 0;
     bool same_rows = false;  // every segment is the same rows for the next query (flat_meta)
     uint32_t per = 1;        // queries per pass that `panels` is laid out for (make_panels)
+    bool compact = false;    // and its form (Sizes)
 };
 
 struct Sizes {
@@ -311,6 +318,9 @@ struct Sizes {
     int engine;        // BN_ENGINE_*
     uint32_t per = 1;    // queries per fused pass (TcShare)
     bool split = false;  // form of the decode (decode_split)
+    // compact: z panels of TC_PANEL_ROWS and a candidate list per eight units, whatever
+    // the launches' schedules would like: up to 7.5 MB less at a few thousand rows.
+    // Taken where the other form's workspace does not fit its budget.
 };
 
 
@@ -332,13 +342,14 @@ struct QueryJob {
     HostMeta* hm = nullptr;  // job_prepare assigns the decode CTAs into it
     uint32_t B = 0, trials = 0, k = 0;
     bool want_mv = false;
+    bool compact = false;  // only the compact form (a caller with a budget of its own)
     Sizes z{};
     RunLayout o{};
     TcMaps maps;
 };
 void finish_meta(HostMeta& hm);
 void flat_meta(uint64_t m, uint32_t B, HostMeta& hm);
-Sizes sizes_for(const Engine& e, HostMeta& hm, uint32_t B, uint32_t trials, uint32_t k);
+Sizes sizes_for(const Engine& e, HostMeta& hm, uint32_t B, uint32_t trials, uint32_t k, bool compact = false);
 RunLayout make_layout(const Sizes& z, bool want_mv);
 // Validates and packs the inputs into host (pinned, grown as needed) and
 // sizes ws (grown as needed, budget-accounted).
@@ -361,7 +372,7 @@ IvfBlockJob* ivf_block_job_new();
 void ivf_block_job_free(IvfBlockJob* j);
 uint64_t ivf_block_job_bytes(const IvfBlockJob* j);
 int ivf_block_plan(const bn_ivf& v, IvfBlockJob& j, uint32_t B, const uint32_t* probe_off, const uint32_t* probes,
-                   uint32_t trials, uint32_t k, bool verify_only, int sms);
+                   uint32_t trials, uint32_t k, bool verify_only, int sms, bool compact = false);
 int ivf_block_pack(Engine& e, IvfBlockJob& j, DevMem& ws, PinnedMem& host, const uint64_t* v_enc, const uint64_t* g,
                    const uint32_t* t_idx, const int8_t* t_sign, const uint32_t* t_nnz, const uint8_t* seed);
 // ev (nullable): 9 events recorded on s at the stage boundaries (start; operand
@@ -416,7 +427,7 @@ struct bn_ivf {
 namespace bn {
 namespace api {
 int block_prepare(bn_flat* f);
-constexpr uint32_t BLOCK_VERIFY_ONLY = 1u << 31;  // internal block_plan_create flag
+constexpr uint32_t BLOCK_VERIFY_ONLY = 1u << 31, BLOCK_COMPACT = 1u << 30;  // internal block_plan_create flags
 int block_plan_create(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k, uint32_t flags, BlockPlan** out);
 void block_plan_config(const BlockPlan* b, uint32_t cfg[6], float tuned_ms[2]);
 int block_plan_status(BlockPlan* b, uint32_t* flags);
@@ -430,7 +441,7 @@ int block_query_launch(BlockPlan& b, uint32_t nq, const uint64_t* v_enc, const u
                        const int8_t* t_sign, const uint32_t* t_nnz, const uint8_t* seed, cudaStream_t s, bool want_mv);
 int block_query_finish(BlockPlan& b, uint32_t nq, uint32_t* ids, int64_t* scores, uint32_t* n_hits, int32_t* failed);
 uint64_t block_plan_bytes(const BlockPlan* b);
-uint64_t block_plan_estimate(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k);
+uint64_t block_plan_estimate(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k, bool compact = false);
 // Byte-planar corpus copies of block scoring (once per handle; caller holds
 // e.mu); offsets (nullable): the IVF list boundaries.
 int block_prepare_engine(Engine& e, const std::vector<uint64_t>* offsets);

@@ -51,14 +51,14 @@ struct IvPair {
     uint32_t pad;
 };
 
-// Up to IV_CHUNK_ROWS rows of one pair (ids; u . r partial sums per chunk).
+// Up to IvfBlockJob::chunk_rows rows of one pair (ids; u . r partial sums per chunk).
 struct IvChunk {
     uint64_t r0;    // first r-space entry
     uint64_t row0;  // first corpus row
     uint32_t ublk;  // first 128-row block of the list's U image
     uint32_t rows;
 };
-constexpr uint32_t IV_CHUNK_ROWS = 512;
+constexpr uint32_t IV_CHUNK_ROWS = 512, IV_CHUNK_ROWS_COMPACT = 2048;  // compact: a quarter of the tables and sums
 
 // u . r work of one CTA: chunk c of a list (its U blocks from ublk0 on) for
 // up to UR_SLAB of the list's pairs (list-major positions lp0 ...).
@@ -133,14 +133,15 @@ __device__ __forceinline__ void mac128(uint64_t& lo, uint64_t& hi, uint64_t a, u
 // Warp w owns trials w, w + 8, ... for the whole chunk; lane l takes rows 4l ..
 // 4l + 3 of each block, reads one 32-bit word from each of the 8 byte rows of
 // trial t, transposes them into the four u_t values and multiplies them with
-// every pair's r.  4 blocks x 4 rows = 16 products (< 2^122 each) per lane,
-// trial and pair are summed in 128 bits.  Latency bound: chunks of 2048 rows,
+// every pair's r.  4 blocks x 4 rows = 16 products (64 where the chunks are compact;
+// < 2^122 each) per lane, trial and pair are summed in 128 bits.  Latency bound: chunks of 2048 rows,
 // with r read from memory once per trial, left a batch of 512 pairs on 175 CTAs
 // (115 us) and one of 4,096 at 230 us.
 __global__ void __launch_bounds__(UR_WARPS * 32)
 ur_lists_kernel(const IvUrTask* __restrict__ tasks, const IvPair* __restrict__ pairs, const uint32_t* __restrict__ lmi,
                 const uint8_t* __restrict__ ub, uint32_t n_rows, uint32_t t_base, uint32_t t_cnt,
-                uint32_t trials_total, const uint64_t* __restrict__ r, uint64_t* __restrict__ ur_part) {
+                uint32_t trials_total, uint32_t chunk_rows, const uint64_t* __restrict__ r,
+                uint64_t* __restrict__ ur_part) {
     extern __shared__ uint4 u_img[];  // one U block: 8 t_cnt rows x 128 bytes
     // r of a block per pair: rows 4l, 4l + 1 of lane l, then its rows 4l + 2, 4l + 3
     __shared__ ulonglong2 r_s[UR_SLAB][2][TC_ROWS / 4];
@@ -150,7 +151,7 @@ ur_lists_kernel(const IvUrTask* __restrict__ tasks, const IvPair* __restrict__ p
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x < tk.npairs) {
         const IvPair pr = pairs[lmi[tk.lp0 + threadIdx.x]];
-        rbase_s[threadIdx.x] = pr.out0 + (uint64_t)tk.c * IV_CHUNK_ROWS;
+        rbase_s[threadIdx.x] = pr.out0 + (uint64_t)tk.c * chunk_rows;
         out_s[threadIdx.x] = pr.ch0 + tk.c;
     }
     uint64_t lo[UR_PER_WARP][UR_SLAB], hi[UR_PER_WARP][UR_SLAB];
@@ -333,6 +334,7 @@ struct IvfBlockJob {
     bool verify_only = false;
     uint32_t P = 0, U = 0, NB = 0, NP = 0, NCH = 0, n_pl = 0, n_s8 = 0, NZ = 0;
     uint32_t max_n = 0;   // most pairs of one list
+    uint32_t chunk_rows = IV_CHUNK_ROWS;
     uint32_t NP_big = 0;  // panels [0, NP_big) belong to lists longer than TC_SMALL_PANEL_ROWS
     uint32_t NUR = 0;     // u . r tasks (list chunk x pair slab)
     uint64_t R = 0, max_q_rows = 0;
@@ -395,7 +397,7 @@ uint32_t pick_w_tile(const std::vector<IvGroup>& groups, uint32_t B) {
 // + distinct lists); the per-block / per-panel / per-chunk tables are written
 // by ivf_block_pack and the GEMM item tables on the device.
 int ivf_block_plan(const bn_ivf& v, IvfBlockJob& j, uint32_t B, const uint32_t* probe_off, const uint32_t* probes,
-                   uint32_t trials, uint32_t k, bool verify_only, int sms) {
+                   uint32_t trials, uint32_t k, bool verify_only, int sms, bool compact) {
     const Corpus& c = v.e.c;
     if (k > BN_TOPK_MAX) return fail(BN_EINVAL, "k = %u exceeds BN_TOPK_MAX = %d", k, BN_TOPK_MAX);
     if (trials > BN_MAX_TRIALS) return fail(BN_EINVAL, "trials = %u exceeds %d", trials, BN_MAX_TRIALS);
@@ -406,6 +408,7 @@ int ivf_block_plan(const bn_ivf& v, IvfBlockJob& j, uint32_t B, const uint32_t* 
     j.trials = trials;
     j.k = k;
     j.verify_only = verify_only;
+    j.chunk_rows = compact ? IV_CHUNK_ROWS_COMPACT : IV_CHUNK_ROWS;
     // pairs, q-major; empty lists skipped (ivf.rs:787-789)
     j.pairs.clear();
     j.pairs.reserve(probe_off[B]);
@@ -458,7 +461,7 @@ int ivf_block_plan(const bn_ivf& v, IvfBlockJob& j, uint32_t B, const uint32_t* 
         IvGroup& g = j.groups.back();
         pr.u = (uint32_t)j.groups.size() - 1;
         pr.ch0 = nch;
-        pr.nch = (g.m + IV_CHUNK_ROWS - 1) / IV_CHUNK_ROWS;
+        pr.nch = (g.m + j.chunk_rows - 1) / j.chunk_rows;
         nch += pr.nch;
         ++g.n;
     }
@@ -483,7 +486,7 @@ int ivf_block_plan(const bn_ivf& v, IvfBlockJob& j, uint32_t B, const uint32_t* 
     j.NUR = 0;
     for (uint32_t u = 0; u < j.U; ++u) {
         j.NZ += (j.groups[u].m > TC_PANEL_ROWS) ? 1u : 0u;
-        j.NUR += ((j.groups[u].m + IV_CHUNK_ROWS - 1) / IV_CHUNK_ROWS) * ((j.groups[u].n + UR_SLAB - 1) / UR_SLAB);
+        j.NUR += ((j.groups[u].m + j.chunk_rows - 1) / j.chunk_rows) * ((j.groups[u].n + UR_SLAB - 1) / UR_SLAB);
     }
     // grouped GEMM item counts (the tables themselves are expanded on the device)
     j.n_pl = j.n_s8 = 0;
@@ -608,6 +611,7 @@ int ivf_block_pack(Engine& e, IvfBlockJob& j, DevMem& ws, PinnedMem& host, const
     uint32_t* lmi = reinterpret_cast<uint32_t*>(h + j.o_lmi);
     uint64_t* base = reinterpret_cast<uint64_t*>(h + j.o_base);
     IvChunk* ch = reinterpret_cast<IvChunk*>(h + j.o_chunks);
+    const uint32_t cr = j.chunk_rows;
     for (uint32_t lp = 0, nc = 0; lp < j.P; ++lp) {
         const uint32_t i = j.order[lp];
         const IvPair& pr = j.pairs[i];
@@ -615,9 +619,9 @@ int ivf_block_pack(Engine& e, IvfBlockJob& j, DevMem& ws, PinnedMem& host, const
         lmq[lp] = pr.q;
         lmi[lp] = i;
         base[lp] = pr.out0 - gr.row0;  // out[base + corpus row] (mod 2^64)
-        for (uint32_t c0 = 0; c0 < gr.m; c0 += IV_CHUNK_ROWS)
+        for (uint32_t c0 = 0; c0 < gr.m; c0 += cr)
             ch[nc++] = IvChunk{pr.out0 + c0, (uint64_t)gr.row0 + c0, j.block0[pr.u] + c0 / TC_ROWS,
-                               std::min<uint32_t>(IV_CHUNK_ROWS, gr.m - c0)};
+                               std::min<uint32_t>(cr, gr.m - c0)};
     }
     // Protocol 2 layout: one verify segment per distinct list (128-row U
     // blocks, 4096-row z panels); z of a single-panel list is its z_part,
@@ -625,10 +629,9 @@ int ivf_block_pack(Engine& e, IvfBlockJob& j, DevMem& ws, PinnedMem& host, const
     IvUrTask* ut = reinterpret_cast<IvUrTask*>(h + j.o_urtasks);
     for (uint32_t u = 0, nt = 0; u < j.U; ++u) {
         const IvGroup& gr = j.groups[u];
-        for (uint32_t c = 0; c * IV_CHUNK_ROWS < gr.m; ++c)
+        for (uint32_t c = 0; c * cr < gr.m; ++c)
             for (uint32_t p0 = 0; p0 < gr.n; p0 += UR_SLAB)
-                ut[nt++] = IvUrTask{j.block0[u] + c * (IV_CHUNK_ROWS / TC_ROWS),
-                                    std::min<uint32_t>(IV_CHUNK_ROWS, gr.m - c * IV_CHUNK_ROWS), gr.lp0 + p0,
+                ut[nt++] = IvUrTask{j.block0[u] + c * (cr / TC_ROWS), std::min<uint32_t>(cr, gr.m - c * cr), gr.lp0 + p0,
                                     std::min<uint32_t>(UR_SLAB, gr.n - p0), c};
     }
     VerifySeg* vs = reinterpret_cast<VerifySeg*>(h + j.o_vsegs);
@@ -764,7 +767,7 @@ int ivf_block_launch(Engine& e, IvfBlockJob& j, DevMem& ws, PinnedMem& host, cud
             if (last_chunk) mark(7);
             ur_lists_kernel<<<j.NUR, UR_WARPS * 32, 8 * tc * TC_ROWS, s>>>(
                 reinterpret_cast<const IvUrTask*>(d + j.o_urtasks), dpairs, U32(j.o_lmi), U8(j.o_ub), j.n_rows, t0, tc,
-                j.trials, U64(j.o_r), U64(j.o_urpart));
+                j.trials, j.chunk_rows, U64(j.o_r), U64(j.o_urpart));
         }
         mark(8);
         if (j.NZ)
@@ -862,6 +865,8 @@ int bn_ivf_query_block(bn_ivf* v, uint32_t B, uint32_t nprobe, const uint32_t* p
     const std::vector<uint32_t> off = fixed_probe_off(B, nprobe);
     IvfBlockJob j;
     TRY(ivf_block_plan(*v, j, B, off.data(), probes, trials, k, false, e.ctx->num_sms));
+    if (!e.ws.fits(e.ctx, j.total))
+        TRY(ivf_block_plan(*v, j, B, off.data(), probes, trials, k, false, e.ctx->num_sms, true));
     TRY(ivf_block_pack(e, j, e.ws, e.host, v_enc, g, t_idx, t_sign, t_nnz, block_seed));
     v->prof_host_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
     v->prof_have = false;
@@ -926,6 +931,8 @@ int bn_ivf_verify_block(bn_ivf* v, uint32_t B, uint32_t nprobe, const uint32_t* 
     const std::vector<uint32_t> off = fixed_probe_off(B, nprobe);
     IvfBlockJob j;
     TRY(ivf_block_plan(*v, j, B, off.data(), probes, trials, 0, true, e.ctx->num_sms));
+    if (!e.ws.fits(e.ctx, j.total))
+        TRY(ivf_block_plan(*v, j, B, off.data(), probes, trials, 0, true, e.ctx->num_sms, true));
     if (r_len != j.R)
         return fail(BN_EINVAL, "r holds %llu entries; the probed lists hold %llu rows", (unsigned long long)r_len,
                     (unsigned long long)j.R);

@@ -86,6 +86,7 @@ struct Slot {
     // the count): planned while sizing the batch, reused by its launch
     uint64_t ivj_ticket0 = 0;
     size_t ivj_count = 0;
+    bool compact = false;  // the batch to launch runs in the compact form (Sizes), for mem_budget's sake
     ~Slot() {
         if (ivj) ivf_block_job_free(ivj);
     }
@@ -172,40 +173,40 @@ bool ivf_block(const bn_server* s, size_t count) {
 
 // Host plan of an IVF block over requests [first, first + count).
 template <class It>
-int ivf_block_plan_reqs(bn_server* s, It first, size_t count, IvfBlockJob& j) {
+int ivf_block_plan_reqs(bn_server* s, It first, size_t count, bool compact, IvfBlockJob& j) {
     std::vector<uint32_t> off(count + 1, 0), probes;
     for (size_t b = 0; b < count; ++b) {
         probes.insert(probes.end(), first[b].probes.begin(), first[b].probes.end());
         off[b + 1] = (uint32_t)probes.size();
     }
     return ivf_block_plan(*s->ivf, j, (uint32_t)count, off.data(), probes.data(), s->cfg.trials, s->cfg.k, false,
-                          s->ivf->e.ctx->num_sms);
+                          s->ivf->e.ctx->num_sms, compact);
 }
 
 // Device workspace of a batch made of the first `count` requests of q (a
 // block plan's workspace when the batch runs as a block).  An IVF block's
 // host plan is made in `me`'s job and kept for the launch.
-uint64_t batch_bytes(bn_server* s, int kind, const std::deque<Request>& q, size_t count, Slot* me) {
+uint64_t batch_bytes(bn_server* s, int kind, const std::deque<Request>& q, size_t count, bool compact, Slot* me) {
     if (kind == BN_SERVER_FLAT)
         if (const uint32_t bucket = block_bucket(s, count))
-            return block_plan_estimate(s->flat, bucket, s->cfg.trials, s->cfg.k);
+            return block_plan_estimate(s->flat, bucket, s->cfg.trials, s->cfg.k, compact);
     if (kind == BN_SERVER_IVF && ivf_block(s, count)) {
         if (me) {
             if (!me->ivj) me->ivj = ivf_block_job_new();
             me->ivj_count = 0;
-            if (ivf_block_plan_reqs(s, q.begin(), count, *me->ivj) == BN_OK) {
+            if (ivf_block_plan_reqs(s, q.begin(), count, compact, *me->ivj) == BN_OK) {
                 me->ivj_ticket0 = q.front().ticket;
                 me->ivj_count = count;
                 return ivf_block_job_bytes(me->ivj);
             }
         } else {
             std::unique_ptr<IvfBlockJob, void (*)(IvfBlockJob*)> j(ivf_block_job_new(), ivf_block_job_free);
-            if (ivf_block_plan_reqs(s, q.begin(), count, *j) == BN_OK) return ivf_block_job_bytes(j.get());
+            if (ivf_block_plan_reqs(s, q.begin(), count, compact, *j) == BN_OK) return ivf_block_job_bytes(j.get());
         }
     }
     HostMeta hm;
     batch_meta(s, kind, q.begin(), q.begin() + count, hm);
-    const Sizes z = sizes_for(engine_of(s, kind), hm, (uint32_t)count, s->cfg.trials, s->cfg.k);
+    const Sizes z = sizes_for(engine_of(s, kind), hm, (uint32_t)count, s->cfg.trials, s->cfg.k, compact);
     return make_layout(z, false).total;
 }
 
@@ -319,7 +320,9 @@ int launch(bn_server* s, Slot& sl, int kind, std::vector<Request>&& reqs) {
         if (!sl.ivj) sl.ivj = ivf_block_job_new();
         Engine& e = s->ivf->e;
         if (!(sl.ivj_count == B && sl.ivj_ticket0 == sl.reqs.front().ticket))  // not planned while sizing
-            rc = ivf_block_plan_reqs(s, sl.reqs.begin(), B, *sl.ivj);
+            rc = ivf_block_plan_reqs(s, sl.reqs.begin(), B, sl.compact, *sl.ivj);
+        if (rc == BN_OK && !sl.ws.fits(e.ctx, ivf_block_job_bytes(sl.ivj)))
+            rc = ivf_block_plan_reqs(s, sl.reqs.begin(), B, true, *sl.ivj);
         sl.ivj_count = 0;
         if (rc == BN_OK)
             rc = ivf_block_pack(e, *sl.ivj, sl.ws, sl.host, v.data(), g.data(), ti.empty() ? nullptr : ti.data(),
@@ -341,7 +344,7 @@ int launch(bn_server* s, Slot& sl, int kind, std::vector<Request>&& reqs) {
         if (pi < 0) pi = pool_find(s, bucket, false);
         if (pi < 0) {
             BlockPlan* bp = nullptr;
-            rc = block_plan_create(s->flat, bucket, s->cfg.trials, s->cfg.k, 0, &bp);
+            rc = block_plan_create(s->flat, bucket, s->cfg.trials, s->cfg.k, sl.compact ? BLOCK_COMPACT : 0, &bp);
             if (rc == BN_OK) {
                 s->plans.push_back(PooledPlan{bp, bucket, false});
                 pi = (int)s->plans.size() - 1;
@@ -365,6 +368,7 @@ int launch(bn_server* s, Slot& sl, int kind, std::vector<Request>&& reqs) {
         sl.job.B = B;
         sl.job.trials = s->cfg.trials;
         sl.job.k = s->cfg.k;
+        sl.job.compact = sl.compact;
         Engine& e = engine_of(s, kind);
         rc = job_prepare(e, sl.job, sl.ws, sl.host, v.data(), g.data(), ti.empty() ? nullptr : ti.data(),
                          ts.empty() ? nullptr : ts.data(), tn.data(), seeds.data());
@@ -434,16 +438,23 @@ std::vector<Request> take_batch(bn_server* s, Slot& me, int& kind_out, bool& rej
     // workspace; a per-query or IVF batch grows this slot's workspace.
     const uint64_t others = held_bytes(s) - me.ws.bytes;
     const uint64_t budget = s->cfg.mem_budget;
-    auto need = [&](size_t cnt) -> uint64_t {
+    auto need = [&](size_t cnt, bool compact) -> uint64_t {
         const uint32_t bucket = kind == BN_SERVER_FLAT ? block_bucket(s, cnt) : 0;
         if (bucket) {
             if (pool_find(s, bucket, false) >= 0) return me.ws.bytes;  // an idle plan of this size or larger
-            return me.ws.bytes + batch_bytes(s, kind, q, cnt, &me);
+            return me.ws.bytes + batch_bytes(s, kind, q, cnt, compact, &me);
         }
-        return DevMem::grown(me.ws.bytes, batch_bytes(s, kind, q, cnt, &me));  // reserve_grow's size
+        return DevMem::grown(me.ws.bytes, batch_bytes(s, kind, q, cnt, compact, &me));  // reserve_grow's size
+    };
+    auto over = [&](size_t cnt) {  // in both forms
+        me.compact = false;
+        if (others + need(cnt, false) <= budget) return false;
+        me.compact = true;
+        return others + need(cnt, true) > budget;
     };
     size_t count = std::min<size_t>(q.size(), s->cfg.max_batch);
-    while (count > 0 && budget && others + need(count) > budget) count = count > 8 ? count / 2 : count - 1;
+    me.compact = false;
+    while (count > 0 && budget && over(count)) count = count > 8 ? count / 2 : count - 1;
     if (count == 0) {
         bool any_busy = false;
         for (auto& sl : s->slots) any_busy |= sl->busy;
@@ -452,7 +463,8 @@ std::vector<Request> take_batch(bn_server* s, Slot& me, int& kind_out, bool& rej
             for (auto& sl : s->slots) sl->ws.release();
             for (PooledPlan& pp : s->plans) block_plan_free(pp.bp);
             s->plans.clear();
-            if (batch_bytes(s, kind, q, 1, nullptr) + held_bytes(s) > budget) {
+            me.compact = batch_bytes(s, kind, q, 1, false, nullptr) + held_bytes(s) > budget;
+            if (me.compact && batch_bytes(s, kind, q, 1, true, nullptr) + held_bytes(s) > budget) {
                 reject_front = true;  // this request alone exceeds the budget
                 reject_kind = kind;
             } else {

@@ -1236,7 +1236,7 @@ void launch_tc_finish(const uint64_t* d_z_part, const uint64_t* d_ur_part, const
         const uint32_t ns = nseg - s0 < per_launch ? nseg - s0 : per_launch;
         const dim3 grid(trials, split > 1 ? FIN_CHUNKS + 1 : 2, ns * split);
         launch_after(tc_finish_kernel, grid, 128, 0, s, d_z_part, d_ur_part, d_seg_panel0 + s0, d_seg_block0 + s0, d_v_enc,
-                     d_vsegs + s0, trials, split, d_chunks + (uint64_t)s0 * trials * (FIN_CHUNKS + 1) * split, d_done + s0,
+                     d_vsegs + s0, trials, split, d_chunks + tc_finish_words(s0, trials), d_done + s0,
                      d_ur + (uint64_t)s0 * trials, d_zv + (uint64_t)s0 * trials, d_failed + s0);
     }
 }

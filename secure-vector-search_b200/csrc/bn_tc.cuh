@@ -169,8 +169,9 @@ void launch_tc_rreduce(const VerifySeg* d_vsegs, const TcBlock* d_blocks, uint32
 // decides it and leaves its ticket zero).
 constexpr uint32_t FIN_SPLIT = 16;
 inline uint32_t tc_finish_split(uint32_t nseg) { return nseg <= 4 ? FIN_SPLIT : 1u; }
-inline uint64_t tc_finish_words(uint32_t nseg, uint32_t trials) {
-    return (uint64_t)nseg * trials * (N / 128 + 1) * tc_finish_split(nseg);
+inline uint64_t tc_finish_words(uint32_t nseg, uint32_t trials) {  // shares: 8 column chunks and u . r, or one of each
+    const uint32_t split = tc_finish_split(nseg);
+    return (uint64_t)nseg * trials * (split > 1 ? (N / 128 + 1) * split : 2);
 }
 void launch_tc_finish(const uint64_t* d_z_part, const uint64_t* d_ur_part, const uint32_t* d_seg_panel0,
                       const uint32_t* d_seg_block0, const uint64_t* d_v_enc, const VerifySeg* d_vsegs, uint32_t nseg,
