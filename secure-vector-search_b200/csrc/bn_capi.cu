@@ -518,7 +518,8 @@ int make_tc_maps(const Sizes& z, const uint8_t* d_u, const uint8_t* d_w, TcMaps&
 int enqueue_pipeline(bn_ctx* ctx, const Corpus& c, const Sizes& z, const Meta& m, const Inputs& in, const Scratch& sc,
                      const Outputs& out, cudaStream_t s, cudaEvent_t prof0, cudaEvent_t prof1) {
     const bool tensor = z.trials && z.engine == BN_ENGINE_TENSOR;
-    launch_query_prep(c.L.at<uint64_t>(), c.n1, in.v, z.B, z.k ? sc.x : nullptr, tensor ? sc.wimg : nullptr, sc.err,
+    const bool decode = z.k || out.mv;  // k = 0 with the decoded residues wanted: ranked, and the hits dropped
+    launch_query_prep(c.L.at<uint64_t>(), c.n1, in.v, z.B, decode ? sc.x : nullptr, tensor ? sc.wimg : nullptr, sc.err,
                       sc.zero_words, s);
     if (z.trials && ctx->debug_draw_hit) launch_or_flag(sc.flags, DRAW_HIT_P, s);
     if (!tensor) launch_query_limbs(in.v, z.B, sc.limbs, s);
@@ -561,12 +562,10 @@ int enqueue_pipeline(bn_ctx* ctx, const Corpus& c, const Sizes& z, const Meta& m
             CU(cudaMemsetAsync(out.vfailed, 0xff, std::max<uint64_t>(m.nvseg, 1) * 4, s));
         }
     }
-    if (z.k) {
-        launch_decode_topk(sc.r, decode_corpus(c), m.segs, m.seg_unit, m.dq, z.B, in.v, in.g, sc.x, in.t, in.t_nnz, z.k,
-                           z.ctas, z.split, sc.topk, out.mv, out.ids, out.scores, out.n, s);
-    } else {
-        CU(cudaMemsetAsync(out.n, 0, (uint64_t)z.B * 4, s));
-    }
+    if (decode)
+        launch_decode_topk(sc.r, decode_corpus(c), m.segs, m.seg_unit, m.dq, z.B, in.v, in.g, sc.x, in.t, in.t_nnz,
+                           std::max<uint32_t>(z.k, 1), z.ctas, z.split, sc.topk, out.mv, out.ids, out.scores, out.n, s);
+    if (!z.k) CU(cudaMemsetAsync(out.n, 0, (uint64_t)z.B * 4, s));
     CU(cudaGetLastError());
     return BN_OK;
 }

@@ -143,3 +143,25 @@ def test_large_k(ctx, m, k):
     # beside the lists: r (8 m) and the query's own arrays (below 64 KB)
     assert grown <= 12 * k * lists + 16 * m + (64 << 10), (grown, lists)
     f.close()
+
+
+@pytest.mark.parametrize("trials", [0, 3])
+def test_decoded_residues_without_hits(ctx, trials):
+    """k = 0 with the decoded residues asked for: those, and no hits."""
+    from bn_b200 import capi as c
+
+    m = 700
+    M = int8_matrix(m, 768, 40)
+    L = O.generate_subspace(bytes([9]) * 32)
+    cl = O.encrypt_cluster(M.reshape(-1), m, L, O.derive_h_seed(2, 0))
+    f = c.Flat.build(ctx, cl.m_enc, cl.a_l, cl.h_mat, m)
+    f.attach_client(L, M.reshape(-1), cl.s_mat.rowptr, cl.s_mat.idx, cl.s_mat.sign)
+    for turn in range(2):  # the second run would find the first one's in its workspace
+        encs = [O.encode_query(int8_matrix(1, 768, 41 + 3 * turn + b)[0], L, O.derive_h_seed(42, b)) for b in range(3)]
+        hits, failed, _, mv = f.query(np.stack([e.v_enc for e in encs]), np.stack([e.g for e in encs]),
+                                      [(e.t_idx, e.t_sign) for e in encs], [bytes([b]) * 32 for b in range(3)], trials, 0,
+                                      want_mv=True)
+        for b, enc in enumerate(encs):
+            assert len(hits[b][0]) == 0 and failed[b] == -1
+            assert np.array_equal(mv[b], O.decode_scores(O.matvec(cl.m_enc, m, N, enc.v_enc), cl, L, enc))
+    f.close()
