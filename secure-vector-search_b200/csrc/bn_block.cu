@@ -387,6 +387,7 @@ int block_plan_create(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k, uint3
     if (!f->m) return fail(BN_EINVAL, "empty corpus");
     const bool verify_only = (flags & BLOCK_VERIFY_ONLY) != 0;  // Protocol 2 over claimed r: no planar corpus needed
     std::lock_guard<std::mutex> g(f->e.mu);
+    CU(cudaSetDevice(f->e.ctx->device));
     if (!verify_only) TRY(block_prepare_locked(f->e, nullptr));
     Corpus& c = f->e.c;
     auto* b = new BlockPlan();

@@ -694,6 +694,7 @@ int job_prepare(Engine& e, QueryJob& j, DevMem& ws, PinnedMem& host, const uint6
     TRY(validate_residues(v_enc, (uint64_t)B * N, "v_enc"));
     TRY(validate_residues(g, (uint64_t)B * c.n1, "g"));
 
+    CU(cudaSetDevice(e.ctx->device));  // the tensor maps need a context too, which a new thread does not have
     TRY(lay_out(e, j, ws));
     const RunLayout& o = j.o;
     TRY(host.reserve(o.out_end));
@@ -808,6 +809,7 @@ int run_verify(Engine& e, uint64_t row0, uint64_t rows, const uint64_t* r, const
     finish_meta(hm);
     Sizes z{1, e.c.n1, trials, 0, 1, rows, 0, 1, hm.blocks.size(), hm.panels.size(),
             plan_freivalds(rows, 1, e.ctx->num_sms), e.ctx->engine};
+    CU(cudaSetDevice(e.ctx->device));
     RunLayout o = make_layout(z, false);
     if (!e.ws.fits(e.ctx, o.total)) {  // the compact form (Sizes)
         make_panels(hm, 1, true);
@@ -823,7 +825,6 @@ int run_verify(Engine& e, uint64_t row0, uint64_t rows, const uint64_t* r, const
     memcpy(h + o.v, v_enc, N * 8);
     memcpy(h + o.seeds, seed, 32);
     pack_meta(h, o, hm);
-    CU(cudaSetDevice(e.ctx->device));
     CU(cudaMemcpyAsync(d, h, o.in_end, cudaMemcpyHostToDevice, e.stream));
     TRY(stage_h2d(e.ctx, d + o.r, r, rows * 8, e.stream));
     const Meta m = meta_at(d, o, hm, &maps);
@@ -874,6 +875,7 @@ int run_scan(Engine& e, uint64_t row0, uint64_t rows, const uint64_t* v_encs, ui
     const uint64_t o_v = L.take<uint64_t>((uint64_t)B * N), o_s = L.take<ScanSeg>(B), o_b = L.take<uint64_t>(B + 1), in_end = L.off;
     const uint64_t o_l = L.take<QLimb>((uint64_t)B * N), o_r = L.take<uint64_t>((uint64_t)B * rows);
     const uint64_t o_e = L.take<uint32_t>(1);
+    CU(cudaSetDevice(e.ctx->device));
     TRY(e.ws.reserve(e.ctx, L.off));
     TRY(e.host.reserve(std::max<uint64_t>(in_end, 4)));
     char* h = e.host.at<char>();
@@ -881,7 +883,6 @@ int run_scan(Engine& e, uint64_t row0, uint64_t rows, const uint64_t* v_encs, ui
     memcpy(h + o_s, hm.segs.data(), B * sizeof(ScanSeg));
     memcpy(h + o_b, hm.seg_blk.data(), (B + 1) * 8ull);
     char* d = e.ws.at<char>();
-    CU(cudaSetDevice(e.ctx->device));
     CU(cudaMemcpyAsync(d, h, in_end, cudaMemcpyHostToDevice, e.stream));
     CU(cudaMemsetAsync(d + o_e, 0, 4, e.stream));
     launch_query_limbs(reinterpret_cast<uint64_t*>(d + o_v), B, reinterpret_cast<QLimb*>(d + o_l), e.stream);
@@ -903,13 +904,13 @@ int run_dense_terms(Engine& e, uint64_t row0, uint64_t rows, const uint64_t* g, 
     if (!rows) return BN_OK;
     Layout L;
     const uint64_t o_g = L.take<uint64_t>(e.c.n1), o_x = L.take<uint64_t>(e.c.n1), in_end = L.off, o_o = L.take<uint64_t>(rows);
+    CU(cudaSetDevice(e.ctx->device));
     TRY(e.ws.reserve(e.ctx, L.off));
     TRY(e.host.reserve(in_end));
     char* h = e.host.at<char>();
     memcpy(h + o_g, g, e.c.n1 * 8ull);
     memcpy(h + o_x, lt, e.c.n1 * 8ull);
     char* d = e.ws.at<char>();
-    CU(cudaSetDevice(e.ctx->device));
     CU(cudaMemcpyAsync(d, h, in_end, cudaMemcpyHostToDevice, e.stream));
     // column-major arrays: the list's rows are a contiguous slice of each column
     launch_dense_terms(e.c.al_cm.at<uint64_t>() + row0, e.c.h_cm.at<uint64_t>() + row0, rows, e.c.n1,
@@ -1210,6 +1211,7 @@ int bn_flat_plan(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k, bn_plan** 
     if (trials > MAX_TRIALS) return fail(BN_EINVAL, "trials = %u exceeds %u", trials, MAX_TRIALS);
     if (k && !f->e.c.client) return fail(BN_EUNSUPPORTED, "this handle has no client state");
     std::lock_guard<std::mutex> gd(f->e.mu);
+    CU(cudaSetDevice(f->e.ctx->device));
     auto* p = new bn_plan();
     p->h = f;
     flat_meta(f->m, B, p->hm);
@@ -1532,6 +1534,7 @@ int bn_ivf_decode_dense_terms(bn_ivf* v, uint32_t ci, const uint64_t* g, const u
     // it a compact copy of this list's AL / H columns.
     Engine& e = v->e;
     const uint32_t n1 = e.c.n1;
+    CU(cudaSetDevice(e.ctx->device));
     DevMem al, hh;
     TRY(al.alloc(e.ctx, m * n1 * 8));
     TRY(hh.alloc(e.ctx, m * n1 * 8));

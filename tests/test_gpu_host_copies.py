@@ -72,3 +72,46 @@ def test_pinned_arrays_are_free_on_return(ctx):
         r[:] = want
     ivf.close()
     flat.close()
+
+
+def test_first_calls_of_a_new_thread(ctx):
+    """A thread that has made no CUDA call yet, over handles that need no new memory."""
+    import threading
+
+    from bn_b200 import capi as c
+    from bnutil import int8_matrix
+
+    m, B = 2000, 2
+    L = O.generate_subspace(bytes([3]) * 32)
+    x = int8_matrix(m, 768, 48)
+    f = c.Flat.build_keygen(ctx, x.reshape(-1), m, L, bytes([4]) * 32)
+    off = np.array([0, 900, m], np.uint64)
+    v = c.Ivf.build_keygen(ctx, off, np.arange(m, dtype=np.uint32), x.reshape(-1), L, 5)
+    v.block_prepare()
+    encs = [O.encode_query(int8_matrix(1, 768, 49 + b)[0], L, O.derive_h_seed(50, b)) for b in range(B)]
+    q = (np.stack([e.v_enc for e in encs]), np.stack([e.g for e in encs]), [(e.t_idx, e.t_sign) for e in encs])
+    seeds = [bytes([b]) * 32 for b in range(B)]
+    probes = np.array([[0, 1], [1, 0]], np.uint32)
+    r = f.compute_products_batch(q[0])
+    calls = {
+        "query": lambda: f.query(*q, seeds, 3, 5)[:2],
+        "verify": lambda: f.verify(r[0], q[0][0], seeds[0], 3),
+        "products": lambda: f.compute_products(q[0][0]),
+        "dense": lambda: f.decode_dense_terms(q[1][0], q[1][1]),
+        "list dense": lambda: v.decode_dense_terms(1, q[1][0], q[1][1]),
+        "block": lambda: f.query_block(*q, seeds[0], 3, 5)[:2],
+        "verify_block": lambda: f.verify_block(r, q[0], seeds[0], 3),
+        "ivf": lambda: v.query(probes, *q, seeds, 3, 5),
+        "ivf_block": lambda: v.query_block(probes, *q, seeds[0], 3, 5),
+    }
+    got = {}
+    flat = lambda y: [z for w in y for z in flat(w)] if isinstance(y, (list, tuple)) else [y]  # noqa: E731
+    for name, call in calls.items():
+        want = call()
+        t = threading.Thread(target=lambda: got.update({name: call()}))
+        t.start()
+        t.join()
+        assert name in got, name  # the call raised
+        assert all(np.array_equal(a, b) for a, b in zip(flat(got[name]), flat(want))), name
+    f.close()
+    v.close()
