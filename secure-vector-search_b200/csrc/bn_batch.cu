@@ -478,8 +478,8 @@ __device__ __forceinline__ uint64_t blk_off(uint64_t pr, uint32_t c, uint32_t ks
 // Byte planes of rows of src: row i's byte a lands in row (prow[i] or i) * 8 + a,
 // row-major with dst_ld (ks = 0) or K-blocked with ks K-steps per tile.
 __global__ void planar_rows_kernel(const uint64_t* __restrict__ src, uint64_t rows, uint32_t k, uint64_t src_ld,
-                                   int negate, uint8_t* __restrict__ dst, uint64_t dst_ld, uint32_t col0,
-                                   const uint32_t* __restrict__ prow, uint32_t ks) {
+                                   uint8_t* __restrict__ dst, uint64_t dst_ld, const uint32_t* __restrict__ prow,
+                                   uint32_t ks) {
     const uint32_t chunks = k / 16;
     const uint64_t total = rows * chunks;
     for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x) {
@@ -488,17 +488,14 @@ __global__ void planar_rows_kernel(const uint64_t* __restrict__ src, uint64_t ro
         uint64_t x[16];
         const uint64_t* s = src + i * src_ld + jc * 16;
 #pragma unroll
-        for (int t = 0; t < 16; ++t) {
-            const uint64_t y = s[t];
-            x[t] = negate ? (y == 0 ? 0 : P - y) : y;
-        }
+        for (int t = 0; t < 16; ++t) x[t] = s[t];
         const uint64_t pi = prow ? prow[i] : i;
 #pragma unroll
         for (int a = 0; a < 8; ++a) {
             uint32_t w[4] = {0, 0, 0, 0};
 #pragma unroll
             for (int t = 0; t < 16; ++t) w[t >> 2] |= (uint32_t)((x[t] >> (8 * a)) & 0xffu) << (8 * (t & 3));
-            uint8_t* d = ks ? dst + blk_off(pi * 8 + a, col0 + jc * 16, ks) : dst + (pi * 8 + a) * dst_ld + col0 + jc * 16;
+            uint8_t* d = ks ? dst + blk_off(pi * 8 + a, jc * 16, ks) : dst + (pi * 8 + a) * dst_ld + jc * 16;
             *reinterpret_cast<uint4*>(d) = make_uint4(w[0], w[1], w[2], w[3]);
         }
     }
@@ -746,11 +743,11 @@ void launch_bgemm(const CUtensorMap& tmap_a, const CUtensorMap& tmap_w, const Bg
                                                 p, stages, stage_bytes, d_err);
 }
 
-void launch_planar_rows(const uint64_t* d_src, uint64_t rows, uint32_t k, uint64_t src_ld, int negate, uint8_t* d_dst,
-                        uint64_t dst_ld, uint32_t col0, cudaStream_t s, const uint32_t* d_prow, uint32_t ks) {
+void launch_planar_rows(const uint64_t* d_src, uint64_t rows, uint32_t k, uint64_t src_ld, uint8_t* d_dst,
+                        uint64_t dst_ld, cudaStream_t s, const uint32_t* d_prow, uint32_t ks) {
     if (!rows) return;
-    planar_rows_kernel<<<grid_for(rows * (k / 16), 256, 148 * 16), 256, 0, s>>>(d_src, rows, k, src_ld, negate, d_dst,
-                                                                              dst_ld, col0, d_prow, ks);
+    planar_rows_kernel<<<grid_for(rows * (k / 16), 256, 148 * 16), 256, 0, s>>>(d_src, rows, k, src_ld, d_dst, dst_ld,
+                                                                              d_prow, ks);
 }
 
 void launch_planar_cm(const uint64_t* d_src_cm, uint64_t rows, uint32_t k, uint8_t* d_dst, uint64_t dst_ld,

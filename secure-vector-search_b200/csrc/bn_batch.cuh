@@ -92,15 +92,13 @@ uint32_t bgemm_max_stages(const BgParams& p);
 uint32_t bgemm_stage_bytes(uint32_t w_tile, bool a_resident, uint32_t ksub = 1);
 uint32_t bgemm_smem_bytes(const BgParams& p, uint32_t stages);
 
-// Byte planes of a row-major u64 matrix: byte a of (negate ? p - src :
-// src)[i * src_ld + j], j < k (k % 16 == 0), goes to plane row r = pi * 8 + a
-// (pi = d_prow[i], or i when d_prow is null), column col0 + j: row-major at
-// dst[r * dst_ld + col0 + j] (ks = 0), or K-blocked (ks > 0: tiles of 128
-// plane rows stored as ks runs of 128 rows x 128 bytes, the layout of the
+// Byte planes of a row-major u64 matrix: byte a of src[i * src_ld + j], j < k
+// (k % 16 == 0), goes to plane row r = pi * 8 + a (pi = d_prow[i], or i when d_prow
+// is null): row-major at dst[r * dst_ld + j] (ks = 0), or K-blocked (ks > 0: tiles of
+// 128 plane rows stored as ks runs of 128 rows x 128 bytes, the layout of the
 // corpus-side A operands, whose every (tile, K-step) TMA box is contiguous).
-void launch_planar_rows(const uint64_t* d_src, uint64_t rows, uint32_t k, uint64_t src_ld, int negate, uint8_t* d_dst,
-                        uint64_t dst_ld, uint32_t col0, cudaStream_t s, const uint32_t* d_prow = nullptr,
-                        uint32_t ks = 0);
+void launch_planar_rows(const uint64_t* d_src, uint64_t rows, uint32_t k, uint64_t src_ld, uint8_t* d_dst,
+                        uint64_t dst_ld, cudaStream_t s, const uint32_t* d_prow = nullptr, uint32_t ks = 0);
 // Same from a column-major source: element (i, j) at src_cm[j * rows + i].
 void launch_planar_cm(const uint64_t* d_src_cm, uint64_t rows, uint32_t k, uint8_t* d_dst, uint64_t dst_ld,
                       uint32_t col0, cudaStream_t s, const uint32_t* d_prow = nullptr, uint32_t ks = 0);

@@ -95,10 +95,10 @@ int block_prepare_locked(Engine& e, const std::vector<uint64_t>* offsets) {
     if (c.block_ready) return BN_OK;
     if (!c.client) return fail(BN_EUNSUPPORTED, "block scoring needs the client state (attach_client was not called)");
     if (!c.rows) return fail(BN_EINVAL, "empty corpus");
-    if (c.n1 % 16) return fail(BN_EINVAL, "n1 = %u is not a multiple of 16", c.n1);
+    if (c.n1 % 64) return fail(BN_EINVAL, "n1 = %u is not a multiple of 64", c.n1);  // [AL | H] rows: whole K steps, no pad
     CU(cudaSetDevice(e.ctx->device));
     const uint64_t rows = c.rows;
-    c.k_alh = (uint32_t)align_up(2ull * c.n1, 128);
+    c.k_alh = 2 * c.n1;
     // padded rows: list l's rows at list_p16[l] + i (16-row tiles of the
     // planes) and list_p128[l] + i (128-row tiles of [M | S])
     const std::vector<uint64_t> whole{0, rows};
@@ -145,11 +145,11 @@ int block_prepare_locked(Engine& e, const std::vector<uint64_t>* offsets) {
         pr128 = d_p128.at<uint32_t>();
     }
     CU(cudaMemsetAsync(bad.p, 0, 4, s));
-    // pad rows (and pad columns of [AL | H]) stay zero
+    // pad rows stay zero
     CU(cudaMemsetAsync(c.mp8.p, 0, c.mp8.bytes, s));
     CU(cudaMemsetAsync(c.alh8.p, 0, c.alh8.bytes, s));
     CU(cudaMemsetAsync(c.ms8.p, 0, c.ms8.bytes, s));
-    launch_planar_rows(c.m_enc.at<uint64_t>(), rows, N, N, 0, c.mp8.at<uint8_t>(), 0, 0, s, pr16, N / BG_KSTEP);
+    launch_planar_rows(c.m_enc.at<uint64_t>(), rows, N, N, c.mp8.at<uint8_t>(), 0, s, pr16, N / BG_KSTEP);
     launch_planar_cm(c.al_cm.at<uint64_t>(), rows, c.n1, c.alh8.at<uint8_t>(), 0, 0, s, pr16, c.k_alh / BG_KSTEP);
     launch_planar_cm(c.h_cm.at<uint64_t>(), rows, c.n1, c.alh8.at<uint8_t>(), 0, c.n1, s, pr16, c.k_alh / BG_KSTEP);
     launch_ms8(c.mp_cm.at<uint64_t>(), c.s_ell.at<uint16_t>(), c.s_off.at<uint32_t>(), c.s_w.at<uint16_t>(), rows,
@@ -314,7 +314,7 @@ int autotune(BlockPlan& b, cudaStream_t s) {
 }  // namespace
 
 // Offsets of every buffer of a block plan's workspace; returns its size.
-uint64_t block_layout(BlockPlan& b, uint32_t n1, uint32_t k_alh, bool verify_only) {
+uint64_t block_layout(BlockPlan& b, uint32_t n1, bool verify_only) {
     const uint32_t B = b.B, k = b.k, trials = b.trials;
     const uint32_t ks = std::max<uint32_t>(k, 1);
     const uint32_t tt = std::max<uint32_t>(trials, 1);
@@ -326,7 +326,7 @@ uint64_t block_layout(BlockPlan& b, uint32_t n1, uint32_t k_alh, bool verify_onl
     b.o_panels = L.take<TcPanel>(b.npanels);
     const uint64_t qb = verify_only ? 0 : B;  // per-query operand buffers of the scoring GEMMs
     b.o_vp = L.take<uint8_t>(8ull * qb * N);
-    b.o_gx = L.take<uint8_t>(8ull * qb * k_alh);
+    b.o_gx = L.take<uint8_t>(8ull * qb * 2 * n1);
     b.o_tv = L.take<uint8_t>(8ull * qb * 2 * N);
     b.o_x = L.take<uint64_t>(qb * n1);
     b.o_r = L.take<uint64_t>((uint64_t)B * b.nld);    // r = M_enc v
@@ -376,7 +376,7 @@ static uint64_t block_sizes(BlockPlan& b, const Corpus& c, int sms, bool verify_
     b.panel_rows = compact ? TC_PANEL_ROWS : tc_panel_rows(b.nblocks, 1);
     b.npanels = (uint32_t)((c.rows + b.panel_rows - 1) / b.panel_rows);
     b.topk_ctas = (int)std::max<uint64_t>(1, std::min<uint64_t>((c.rows + 511) / 512, (uint64_t)sms * 4 / b.B));
-    return block_layout(b, c.n1, (uint32_t)align_up(2ull * c.n1, 128), verify_only);
+    return block_layout(b, c.n1, verify_only);
 }
 
 int block_plan_create(bn_flat* f, uint32_t B, uint32_t trials, uint32_t k, uint32_t flags, BlockPlan** out) {
@@ -700,7 +700,7 @@ int block_verify_host(BlockPlan& b, const uint64_t* r, const uint64_t* v_enc, co
         CU(cudaMemcpyAsync(dr + (uint64_t)q * b.nld, r + (uint64_t)q * c.rows, c.rows * 8, cudaMemcpyHostToDevice, s));
     CU(cudaMemcpyAsync(d + b.o_in_v, v_enc, (uint64_t)B * N * 8, cudaMemcpyHostToDevice, s));
     CU(cudaMemcpyAsync(d + b.o_in_seed, seed, 32, cudaMemcpyHostToDevice, s));
-    launch_planar_rows(dr, B, (uint32_t)b.nld, b.nld, 0, reinterpret_cast<uint8_t*>(d + b.o_rp), b.npad, 0, s);
+    launch_planar_rows(dr, B, (uint32_t)b.nld, b.nld, reinterpret_cast<uint8_t*>(d + b.o_rp), b.npad, s);
     enqueue_verify(b, reinterpret_cast<uint64_t*>(d + b.o_in_v), reinterpret_cast<uint8_t*>(d + b.o_in_seed),
                    reinterpret_cast<int32_t*>(d + b.o_fail), s);
     CU(cudaGetLastError());

@@ -99,14 +99,14 @@ int encrypt_dense(bn_ctx* ctx, const uint64_t* d_mq, uint64_t rows, uint32_t n1,
     CU(cudaMemsetAsync(err, 0, 4, s));
     if (kh != n1) CU(cudaMemsetAsync(d + o_lp, 0, o_mp - o_lp, s));  // the pad columns of both
     launch_transpose_add(d_L, n1, N, nullptr, lt, N, s);  // L is [N][n1]: lt[k][j] = L[j][k]
-    launch_planar_rows(lt, n1, N, N, 0, u8(o_ltp), N, 0, s);
-    launch_planar_rows(d_L, N, n1, n1, 0, u8(o_lp), kh, 0, s);
+    launch_planar_rows(lt, n1, N, N, u8(o_ltp), N, s);
+    launch_planar_rows(d_L, N, n1, n1, u8(o_lp), kh, s);
     for (uint64_t r0 = 0; r0 < rows; r0 += chunk) {
         const uint32_t cr = (uint32_t)std::min(chunk, rows - r0);
-        launch_planar_rows(d_H + r0 * n1, cr, n1, n1, 0, u8(o_hp), 0, 0, s, nullptr, kh / BG_KSTEP);
+        launch_planar_rows(d_H + r0 * n1, cr, n1, n1, u8(o_hp), 0, s, nullptr, kh / BG_KSTEP);
         TRY(planar_product(d + o_hp, cr, d + o_lp, N, kh, oe, err, sms, s));
         launch_transpose_add(oe, cr, N, d_mq + r0 * N, d_enc + r0 * N, N, s);
-        launch_planar_rows(d_mq + r0 * N, cr, N, N, 0, u8(o_mp), 0, 0, s, nullptr, N / BG_KSTEP);
+        launch_planar_rows(d_mq + r0 * N, cr, N, N, u8(o_mp), 0, s, nullptr, N / BG_KSTEP);
         TRY(planar_product(d + o_mp, cr, d + o_ltp, n1, N, oa, err, sms, s));
         launch_transpose_add(oa, cr, n1, nullptr, d_al + r0 * n1, n1, s);
     }

@@ -208,7 +208,7 @@ struct Corpus {
     // Byte-planar operands of block scoring (built on first use, see
     // bn_block.cu), K-blocked for the GEMMs' A operand: m_enc planes
     // (rows16 * 8 plane rows x 1024 bytes), [AL | H] planes (rows16 * 8 x
-    // k_alh), [M | S] as signed bytes (rows128 x 2048), corr[rows].  Each
+    // k_alh = 2 n1), [M | S] as signed bytes (rows128 x 2048), corr[rows].  Each
     // list starts on a tile boundary: list c's rows sit at padded rows
     // list_p16[c] (16-row plane tiles) and list_p128[c] (128-row tiles).
     bool block_ready = false;
