@@ -162,7 +162,7 @@ bgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     const uint32_t a_ksteps = p.k_bytes / BG_KSTEP;
     // at most two 32-column chunks per item: half the epilogue warps take the
     // items of one TMEM buffer, half those of the other, so two items are
-    // recombined at a time (8 queries: see the figures at BG_EPI_WARPS)
+    // recombined at a time
     const bool narrow = p.w_tile <= 64;
     auto a_x = [&](uint32_t k) -> int { return p.a_blocked ? 0 : (int)k; };
     auto a_row = [&](const ItemIdx& ix, uint32_t k) -> int {

@@ -1,7 +1,7 @@
 // bn_tc.cu -- Protocol 2 (crypto.rs:1013-1046) on the 5th-generation tensor
 // cores: z_t = u_t^T M_enc for up to 20 trials per pass as an exact u8 GEMM
 // (tcgen05.mma kind::i8, s32 accumulators in TMEM), fed by TMA, drained by
-// four epilogue warps that recombine the byte limbs modulo p = 2^61 - 1.
+// eight epilogue warps that recombine the byte limbs modulo p = 2^61 - 1.
 //
 // Roles per CTA (one CTA per SM, persistent over panels of tc_panel_rows rows):
 //   warp 0  TMA producer: per 128-row stage, S boxes of 128 rows x 128 bytes
@@ -9,7 +9,7 @@
 //   warp 1  MMA issuer: per stage S x 4 tcgen05.mma (M=128, N=8T, K=32),
 //           tcgen05.commit frees the stage; after the panel's last stage a
 //           commit hands the TMEM accumulators to the epilogue
-//   warps 2-5 epilogue: tcgen05.ld, limb recombination, z partials to HBM
+//   warps 2-9 epilogue: tcgen05.ld, limb recombination, z partials to HBM
 // Every mbarrier wait is bounded; on timeout the CTA flags *err and winds
 // down (waits for its own copies and MMAs, frees TMEM) instead of hanging.
 #include <cudaTypedefs.h>
@@ -139,14 +139,6 @@ constexpr int TC_THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 constexpr uint32_t STRIP_BYTES = TC_ROWS * 128;  // one 128x128 M box
 constexpr int TC_EPI_WARPS = 8;                // TMEM drain warps: 2 per lane quarter
 
-// Drains one work item's accumulators into z partials.  TMEM holds, per strip
-// s < sg (columns s * n_rows ...), lanes = the strip's 128 byte columns (j, a)
-// (element j = lane / 8, byte a = lane % 8) and columns (t, b) (trial t, byte
-// b of u_t).  Warp (lane quarter q, half) reads every other 64-column chunk:
-// each lane folds its 8 trials' byte products to (lo + hi 2^32) 2^(8a) mod p,
-// then a butterfly over the 8 lanes of one element leaves lane a with trial
-// c0/8 + a's sum; 16-column remainders use a plain 3-level reduction.
-// z_out[t * N + j] receives z_t[j] for t < t_cnt.
 // (lo + hi 2^32) 2^w mod p, folded below 2^61 + 8 (so 8 of them sum below
 // 2^64): lo, hi < 2^56 (byte sums of s32 accumulators), 0 <= w < 61.
 __device__ __forceinline__ uint64_t fold_part(uint64_t lo, uint64_t hi, uint32_t w) {
@@ -624,14 +616,14 @@ tc_freivalds_small_kernel(const __grid_constant__ CUtensorMap tmap_m, const __gr
 // One pass over m_enc yields both products, all on the tensor cores.  Each
 // stage's S strips (128 rows x 128 bytes of m_enc each) feed two MMAs:
 //   z: D[c][(t,b)] += Mb^T Ub as in tc_freivalds_kernel (strip read
-//      MN-major), accumulated over the 4096-row panel and drained by the
-//      eight epilogue warps at the end of each work item;
+//      MN-major), accumulated over the panel (at most 8192 rows: 8192 * 255^2 <
+//      2^31) and drained by the eight epilogue warps at the end of each work item;
 //   r: E[i][s] = sum_{j,a} Mb[i][8j+a] W[s][8j+a], the same strip read
 //      K-major against the query's diagonal byte image W[s][8j+a] = byte
 //      (s - a) of v_j (16 rows per strip: s = a + b < 15), so that
 //      sum_s 2^(8s) E[i][s] = sum_j M[i][j] v_j over the group's elements.
-//      E is per stage (new rows every stage): two 16-column TMEM buffers at
-//      column 480 alternate, and four drain warps turn each into r partials
+//      E is per stage (new rows every stage): two 16-column TMEM buffers (from
+//      column 480 on) alternate, and four drain warps turn each into r partials
 //      r_part[group][r index] while the next stage accumulates.
 // Several queries over the same rows (TcShare) take the pass together: their
 // draws are the U tile's rows (slot, t, b), their images the r MMA's columns
@@ -639,7 +631,8 @@ tc_freivalds_small_kernel(const __grid_constant__ CUtensorMap tmap_m, const __gr
 // Bytes of m_enc bound the pass, so four queries at 3 trials cost what one does.
 // The z and r MMAs are issued by two warps (1 and FU_R_WARP), so neither
 // instruction stream waits for the other; a stage is free once the z issuer
-// has committed and a drain warp has seen the stage's r MMAs complete.  TMEM: z in columns [0, 3 n_rows) (n_rows <= 160), E behind.
+// has committed and a drain warp has seen the stage's r MMAs complete.  TMEM: z in
+// columns [0, 3 n_rows) (n_rows <= 160), E behind.
 constexpr int FU_S = 3;
 constexpr int FU_DRAIN_WARPS = 4;
 constexpr int FU_R_WARP = 2 + TC_EPI_WARPS + FU_DRAIN_WARPS;           // issues the r MMAs
