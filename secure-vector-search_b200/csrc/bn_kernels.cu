@@ -667,16 +667,38 @@ __device__ __forceinline__ void topk_offer(TopkBuf& b, bool valid, int64_t s, ui
 // folded lazily: every term is < 2^61, three terms fit below 2^63.
 __device__ __forceinline__ uint64_t signed_term(uint64_t x, bool neg) { return neg ? P - x : x; }
 
-// The columns [k_begin, k_end) (multiples of 32) of AL g + H x for the 32 rows of
-// block blk, row l's sum to lane l, from alh_b, where the 2 n1 columns of a block
-// are contiguous.  A 16-byte load takes two rows of two columns per warp (lanes
-// 0-15 rows 2l, 2l + 1 of column k, lanes 16-31 of column k + 1), so a column's
-// limbs, lim[2k], lim[2k + 1] (of g_k for k < n1, of x_(k-n1) for k >= n1), are
-// read from shared memory once for 32 rows of two columns: the decode is bound by
-// the shared-memory pipe as much as by HBM, and one row per lane read them twice
-// as often.  Every column adds lo*b + hi*c < 2^53 + 2^50 (hi < 2^29: residues are
-// < 2^61) to an accumulator, so the 2 n1 <= 1024 columns stay below 2^64 with no
-// fold.
+// AL_i . g + H_i . x for corpus row gr from the 32-row-blocked alh_b: the 2 n1 columns
+// of the row's block are contiguous, so a warp's batch of 32 column loads is one 8 KB
+// run.  lim[2k], lim[2k + 1] hold the limbs of g_k (k < n1) and of x_(k-n1) (k >= n1).
+// Every column adds lo*b + hi*c < 2^53 + 2^50 (hi < 2^29: residues are < 2^61) to an
+// accumulator, so the 2 n1 <= 1024 columns stay below 2^64 with no fold.  (In the form
+// of dense_terms_block the whole-unit decode of 64 queries over 50,000 rows took 1936 us
+// against 1815, one query over 100,000 rows 338 for the call against 328.)
+__device__ __forceinline__ uint64_t dense_terms_row(const uint64_t* __restrict__ alh_b, uint32_t n1, uint64_t gr,
+                                                    const uint4* __restrict__ lim) {
+    const uint64_t* p = alh_b + (gr >> 5) * (2ull * n1) * 32 + (gr & 31);
+    uint64_t a0 = 0, a1 = 0, a2 = 0;
+    for (uint32_t k0 = 0; k0 < 2 * n1; k0 += 32) {  // 2 n1 is a multiple of 32 (n1 >= 64)
+        uint64_t xs[32];
+#pragma unroll
+        for (int kk = 0; kk < 32; ++kk) xs[kk] = __ldg(p + (uint64_t)(k0 + kk) * 32);
+#pragma unroll
+        for (int kk = 0; kk < 32; ++kk) {
+            const uint4 l0 = lim[2 * (k0 + kk)], l1 = lim[2 * (k0 + kk) + 1];  // {b0,b1,b2,c0}, {c1,c2,-,-}
+            const uint32_t xl = (uint32_t)xs[kk], xh = (uint32_t)(xs[kk] >> 32);
+            a0 = mac(mac(a0, xl, l0.x), xh, l0.w);
+            a1 = mac(mac(a1, xl, l0.y), xh, l1.x);
+            a2 = mac(mac(a2, xl, l0.z), xh, l1.y);
+        }
+    }
+    return combine3(a0, a1, a2);
+}
+
+// The same for the columns [k_begin, k_end) (multiples of 32) of the 32 rows of block
+// blk, row l's share to lane l: the split decode, where a warp has a quarter of the
+// columns and no other unit's loads to hide behind.  A 16-byte load takes two rows of
+// two columns per warp (lanes 0-15 rows 2l, 2l + 1 of column k, lanes 16-31 of column
+// k + 1), so a column's limbs are read from shared memory half as often.
 __device__ __forceinline__ uint64_t dense_terms_block(const uint64_t* __restrict__ alh_b, uint32_t n1, uint64_t blk,
                                                       const uint4* __restrict__ lim, uint32_t k_begin, uint32_t k_end,
                                                       uint32_t lane) {
@@ -1104,8 +1126,8 @@ decode_topk_kernel(const uint64_t* __restrict__ r, DecodeCorpus dc, const ScanSe
                     m_t = mt >= 0 ? (uint64_t)mt : P - (uint64_t)(-(int64_t)mt);
                 }
                 const uint64_t s_v = s_times_v_part<1>(dc, blk, vt, 0, lane);
-                const uint64_t dense = dense_terms_block(dc.alh_b, n1, blk, dyn_limbs, 0, 2 * n1, lane);
                 if (valid) {
+                    const uint64_t dense = dense_terms_row(dc.alh_b, n1, gr, dyn_limbs);
                     if (!dc.m8_cm) m_t = m_times_t_cm(dc.mp_cm, dc.rows, gr, tl, 0, tn);
                     const uint64_t mv = sub_mod(sub_mod(rv, add_mod(dense, m_t)), s_v);
                     if (mv_out) mv_out[ridx] = mv;
