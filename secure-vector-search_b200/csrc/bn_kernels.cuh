@@ -35,12 +35,12 @@ namespace bn {
 // resident while the kernel before it in the stream still runs, does what does not
 // depend on it (set-up, inputs that were complete before the run's first kernel,
 // which is launched plainly) and waits for its results in after_wait; every
-// kernel of such a chain waits, so each is complete before the next passes its own
-// wait.  Launched plainly, both calls do nothing.  after_go lets the next kernel of
-// the chain start its own set-up.  What the kernels before it wrote is read after
-// the wait through L2 (__ldcg or TMA): no load of it may be taken for an invariant
-// one and moved up.  One query over 5,000 rows (six kernels): 119 -> 105 us,
-// 100,000 rows 345 -> 337 us.
+// kernel of such a chain waits or is launched plainly, so each is complete before the
+// next passes its own wait.  Launched plainly, both calls do nothing.  after_go lets
+// the next kernel start its own set-up.  What the kernels before it wrote is read after
+// the wait through L2 (__ldcg or TMA): no load of it may be taken for an invariant one
+// and moved up.  One query over 5,000 rows (six kernels): 119 -> 105 us, 100,000 rows
+// 345 -> 337 us.
 __device__ __forceinline__ void after_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void after_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... P, class... A>
