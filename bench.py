@@ -43,7 +43,7 @@ P = (1 << 61) - 1
 # dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of the
 # kernel on a 262,144-row corpus, divided by its rows (the traffic grows in
 # proportion to the rows, so it is scaled to the bench's N).
-FUSED_DRAM_BYTES_PER_ROW = 8670
+FUSED_DRAM_BYTES_PER_ROW = 8896
 METRIC = "BN F_p scan queries/s (flat N=1M, d=768, Freivalds k=20 fused, decode + top-10)"
 
 
@@ -501,7 +501,7 @@ def run_gpu(args, rank: int, world: int, local_rank: int):
                                                "frac": bytes_scan / scan_s / 1e9 / peak}},
         "e2e": {"value": whole_job_rate(args.steps, world, e2e_s), "unit": "queries/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h},
-        "gpu_launches": 9 * args.steps,  # limbs, ugen, query image, fused, rreduce, finish, decide, L^T v, decode + top-k
+        "gpu_launches": 6 * args.steps,  # preparation, draws, fused pass, partial sums, verdict sums, decode + top-k
         "clocks": dict(clk.summary(), window="the K timed steps (sampled every 25 ms)"),
         "sustained": {"queries": args.sustained, "qps": whole_job_rate(args.sustained, world, sus_ms / 1e3)
                       if args.sustained else None, "ms_per_query": sus_ms / max(args.sustained, 1),

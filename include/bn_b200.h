@@ -445,7 +445,8 @@ int bn_debug_set_wait_limit(bn_ctx* ctx, uint64_t cycles);
  * same ChaCha20 stream positions as bn_host_regenerate_h_s, which they equal
  * bit for bit; S is parsed in parallel (the column / sign draw structure
  * scanned as a two-state machine).  S must fit in s_cap entries (*nnz gets
- * the count either way; BN_EINVAL when it does not fit).  BN_EDRAW when an H
+ * the count either way; BN_EINVAL when it does not fit, or when there are entries and
+ * s_idx or s_sign is null).  BN_EDRAW when an H
  * draw equalled p (the reference redraws there; odds 2^-61 per draw): use the
  * host keygen for that seed. */
 int bn_keygen_h_s(bn_ctx* ctx, const uint8_t h_seed[32], uint64_t m, uint32_t n1, uint64_t* H, uint64_t* s_rowptr,
